@@ -177,21 +177,12 @@ constexpr int kFanWidths[] = {24, 40, 56, 72};
 constexpr int kPU = CBCT_PAIR_COLS;
 constexpr int kPV = CBCT_PAIR_ROWS;
 constexpr int kPairThreads = kPU * kPV / 2;
-// Row-quad forward projector: kQU columns x kQV rows per CTA, four adjacent
-// rows of a column per thread.
-#ifndef CBCT_QUAD_ROWS
-#define CBCT_QUAD_ROWS 32
-#endif
-constexpr int kQU = 16;
-constexpr int kQV = CBCT_QUAD_ROWS;
-constexpr int kQuadThreads = kQU * kQV / 4;
-
-// Forward-projector blocks per view: the largest of the slab, pair, quad and fan
-// tilings (one FP64 partial sum per block).
+// Forward-projector blocks per view: the largest of the slab, pair, quad (8 x 16
+// tiles at the finest) and fan tilings (one FP64 partial sum per block).
 inline size_t forward_tiles(int W, int H) {
   const size_t slab = (size_t)((W + kTU - 1) / kTU) * ((H + kTV - 1) / kTV);
   const size_t pair = (size_t)((W + kPU - 1) / kPU) * ((H + kPV - 1) / kPV);
-  const size_t quad = (size_t)((W + kQU - 1) / kQU) * ((H + kQV - 1) / kQV);
+  const size_t quad = (size_t)((W + 7) / 8) * ((H + 15) / 16);
   const size_t fan = (size_t)((W + kFU - 1) / kFU) * ((H + kFV - 1) / kFV);
   return std::max(std::max(slab, pair), std::max(quad, fan));
 }
@@ -219,6 +210,7 @@ struct cbct_plan {
   cbct::SlabBox pair16{};   // row-pair kernel box for 16-bit storage
   cbct::SlabBox quad{};     // row-quad kernel box for fp32 storage
   cbct::SlabBox quad16{};   // row-quad kernel box for 16-bit storage
+  int quad_shape = 0;       // its tile shape (QuadShape)
   cbct::SlabBox fan{};      // fan kernel box for fp32 storage
   cbct::SlabBox fan16{};    // fan kernel box for 16-bit storage
   int fan_lz = 0;           // line length (planes) of the fan kernel, odd

@@ -16,11 +16,11 @@
 //    memory rows and the box is never padded along its slab axis.  Samples are
 //    taken in ray order, so each ray's sum has the reference's summation
 //    order.  Pairs of lerps run as packed FP32 (FFMA2).
-//  * fwd_pair_kernel / fwd_quad_kernel: the same slabs, but one thread marches
-//    two or four vertically adjacent rays of a detector column that share
-//    their in-plane sample positions, interpolating them in e and d once.  A
-//    plan takes the quad kernel where adjacent rows stay under 0.66 z texel
-//    apart, the pair kernel under 0.99, else the slab kernel.
+//  * fwd_pair_kernel: the same slabs, but one thread marches two vertically
+//    adjacent rays of a detector column that share their in-plane sample
+//    positions, interpolating them in e and d once.
+//  * fwd_quad_kernel (forward_quad.cuh): four such rays per thread; the kernel of
+//    launches that fill the GPU (quad_choose has the rule).
 //  * fwd_fan_kernel (opt-in): the in-plane sharing across a whole column,
 //    through shared-memory lines.
 //  * fwd_gather_kernel: the same arithmetic with bounds-checked global loads,
@@ -31,8 +31,7 @@
 #include <cstring>
 #include <type_traits>
 
-#include "device_common.cuh"
-#include "forward_device.cuh"
+#include "forward_host.h"
 
 namespace cbct {
 
@@ -637,414 +636,6 @@ __global__ void __launch_bounds__(kPairThreads, pair_min_blocks<V>())
   fwd_pair_body<V, BX, CHECK>(&map_v, &map_t, vol, views, gc, BZ, nsl_max, o, flags, launch_tile(), smem_raw, sh);
 }
 
-// ------------------------------------------------------------------ row quads
-// The row-pair argument for four adjacent rows of a column: when all four rays
-// leave through the side faces (one clip) and, sorted by z, each lies less
-// than two texels above the lowest at both ends of the ray (the second-lowest
-// less than one), their planes are among the lowest ray's fz .. fz + 3.  One thread marches the quad: one e/d
-// position, four planes interpolated in e and d (16 shared loads for four
-// samples), each ray's own z lerp on its two planes.  Values are the slab
-// kernel's for every ray, so results are bitwise equal.  Quads that do not
-// qualify run as two pairs (or single rays) exactly as the row-pair kernel.
-
-// Rows of a quad box: the slab's kTS + 1 rows and no padding.  The two quads
-// of a warp read planes two or three apart; with a plane stride of BX * 9
-// words (8 mod 32 banks for BX = 8 mod 16) those fall 16 or 24 banks apart,
-// where the padded stride (16 mod 32) puts planes two apart on the same banks.
-#ifndef CBCT_QUAD_BOXY
-#define CBCT_QUAD_BOXY 9
-#endif
-constexpr int kQuadBoxY = CBCT_QUAD_BOXY;
-static_assert(kQuadBoxY >= kTS + 1, "a quad box holds the slab's rows and the next one");
-
-// One sample of a quad (rays sorted by z; z0/dz hold their z start and step).
-template <class V, int BX, bool CHECK>
-__device__ __forceinline__ float4 quad_eval(const V* __restrict__ s, float k, float2 c0, float2 dc, float4 z0,
-                                            float4 dz, float cmo, unsigned maxidx, int& bad) {
-  constexpr int BXY = BX * kQuadBoxY;
-  const float2 pq = __ffma2_rn(make_float2(k, k), dc, c0);
-  const float fe = floor_small(pq.x), fd = floor_small(pq.y);
-  const float2 aed = __fadd2_rn(pq, make_float2(-fe, -fd));
-  const float c0z = fmaf(k, dz.x, z0.x), c1z = fmaf(k, dz.y, z0.y);
-  const float c2z = fmaf(k, dz.z, z0.z), c3z = fmaf(k, dz.w, z0.w);
-  const float f0 = floor_small(c0z), f1 = floor_small(c1z), f2 = floor_small(c2z), f3 = floor_small(c3z);
-  const float s1 = f1 - f0, s2 = f2 - f0, s3 = f3 - f0;   // 0, 1 or 2
-  const int idx0 = int_of_biased(fmaf(f0, float(BXY), fmaf(fd, float(BX), fe)) + cmo);
-  if (CHECK) {
-    const float smax = fmaxf(s1, fmaxf(s2, s3)), smin = fminf(s1, fminf(s2, s3));
-    bad |= ((unsigned)idx0 > maxidx) | (smax >= 1.f && (unsigned)idx0 + 2u * BXY > maxidx) | (smax > 2.f) |
-           (smin < 0.f) | (s1 > 1.f);
-  }
-  // planes fz, fz + 1 from q; fz + 2, fz + 3 from q2 (in the box whenever a ray
-  // needs them; clamped otherwise)
-  const V* q = s + min((unsigned)idx0, maxidx);
-  const V* q2 = s + min((unsigned)idx0 + 2u * BXY, maxidx);
-  const float2 te = make_float2(aed.x, aed.x);
-  const float2 e0 = lerp2(make_float2(sm_f(q[0]), sm_f(q[BX])), make_float2(sm_f(q[1]), sm_f(q[BX + 1])), te);
-  const float2 e1 = lerp2(make_float2(sm_f(q[BXY]), sm_f(q[BXY + BX])),
-                          make_float2(sm_f(q[BXY + 1]), sm_f(q[BXY + BX + 1])), te);
-  const float2 e2 = lerp2(make_float2(sm_f(q2[0]), sm_f(q2[BX])), make_float2(sm_f(q2[1]), sm_f(q2[BX + 1])), te);
-  const float2 e3 = lerp2(make_float2(sm_f(q2[BXY]), sm_f(q2[BXY + BX])),
-                          make_float2(sm_f(q2[BXY + 1]), sm_f(q2[BXY + BX + 1])), te);
-  const float2 td = make_float2(aed.y, aed.y);
-  const float2 d01 = lerp2(make_float2(e0.x, e1.x), make_float2(e0.y, e1.y), td);   // planes fz, fz + 1
-  const float2 d23 = lerp2(make_float2(e2.x, e3.x), make_float2(e2.y, e3.y), td);   // planes fz + 2, fz + 3
-  // Each ray lerps between two consecutive planes of the four: base value and
-  // difference picked by its plane offset (the same subtraction hi - lo for
-  // every ray that uses the pair, so the result is unchanged).
-  const float g0 = d01.y - d01.x, g1 = d23.x - d01.y, g2 = d23.y - d23.x;
-  auto ray = [&](float sk, float cz, float fz) {
-    const float lo = sk < 0.5f ? d01.x : (sk < 1.5f ? d01.y : d23.x);
-    const float gd = sk < 0.5f ? g0 : (sk < 1.5f ? g1 : g2);
-    return fmaf(cz - fz, gd, lo);
-  };
-  // the second-lowest ray is under one texel above the lowest: planes fz, fz + 1 or fz + 1, fz + 2
-  const float lo1 = s1 < 0.5f ? d01.x : d01.y, g1s = s1 < 0.5f ? g0 : g1;
-  return make_float4(fmaf(c0z - f0, g0, d01.x), fmaf(c1z - f1, g1s, lo1), ray(s2, c2z, f2), ray(s3, c3z, f3));
-}
-
-// The quad's samples inside one slab, each ray's values added in ray order.
-#ifndef CBCT_QUAD_UNROLL
-#define CBCT_QUAD_UNROLL 1
-#endif
-
-template <class V, int BX, int SGN, bool CHECK>
-__device__ __forceinline__ void quad_samples(const V* __restrict__ s, float& kf, float Nf, float ce0, float cd0,
-                                             float dce, float dcd, float idcd, float4 z0, float4 dz, float lo,
-                                             float hi, float cmo, unsigned maxidx, float4& acc, int& bad) {
-  const float2 c0 = make_float2(ce0, cd0), dc = make_float2(dce, dcd);
-  auto out_at = [&](float k) {
-    const float x = fmaf(k, dcd, cd0);
-    return SGN > 0 ? (x >= hi) : (x < lo);
-  };
-  float ke = ceilf(((SGN > 0 ? hi : lo) - cd0) * idcd);
-  ke = fminf(fmaxf(ke, kf), Nf);
-  while (ke > kf && out_at(ke - 1.f)) ke -= 1.f;
-  while (ke < Nf && !out_at(ke)) ke += 1.f;
-  float k = kf;
-#if CBCT_QUAD_UNROLL > 1
-  // Two quad-samples evaluated before they are added (in ray order).
-  for (; k + 1.f < ke; k += 2.f) {
-    const float4 v0 = quad_eval<V, BX, CHECK>(s, k, c0, dc, z0, dz, cmo, maxidx, bad);
-    const float4 v1 = quad_eval<V, BX, CHECK>(s, k + 1.f, c0, dc, z0, dz, cmo, maxidx, bad);
-    acc.x += v0.x;
-    acc.y += v0.y;
-    acc.z += v0.z;
-    acc.w += v0.w;
-    acc.x += v1.x;
-    acc.y += v1.y;
-    acc.z += v1.z;
-    acc.w += v1.w;
-  }
-#endif
-  for (; k < ke; k += 1.f) {
-    const float4 v = quad_eval<V, BX, CHECK>(s, k, c0, dc, z0, dz, cmo, maxidx, bad);
-    acc.x += v.x;
-    acc.y += v.y;
-    acc.z += v.z;
-    acc.w += v.w;
-  }
-  kf = ke;
-}
-
-// Two rays of one column (rows a, b) outside a quad: a pair when they qualify,
-// else each on its own.  Frame coordinates: (ce0, cd0, dce, dcd, idcd) per ray.
-struct RayFrame {
-  float ce0, cd0, dce, dcd, idcd, c0z, dcz;
-};
-
-__device__ __forceinline__ RayFrame ray_frame(const Ray& r, int dom) {
-  RayFrame f;
-  f.ce0 = dom ? r.c0x : r.c0y;
-  f.dce = dom ? r.dcx : r.dcy;
-  f.cd0 = dom ? r.c0y : r.c0x;
-  f.dcd = dom ? r.dcy : r.dcx;
-  f.idcd = 1.f / f.dcd;
-  f.c0z = r.c0z;
-  f.dcz = r.dcz;
-  return f;
-}
-
-// Pair test of the row-pair kernel: 1 = pair with a lower, -1 = pair with b
-// lower, 0 = no pair.
-__device__ __forceinline__ int pair_kind(const Ray& ra, const Ray& rb, bool hit_a, bool hit_b, float Nf) {
-  if (!(hit_a && hit_b && ra.a1 == rb.a1 && ra.a2 == rb.a2)) return 0;
-  const float d0 = rb.c0z - ra.c0z;
-  const float d1 = fmaf(Nf - 1.f, rb.dcz, rb.c0z) - fmaf(Nf - 1.f, ra.dcz, ra.c0z);
-  if (d0 >= 2e-3f && d0 <= 0.998f && d1 >= 2e-3f && d1 <= 0.998f) return 1;
-  if (d0 <= -2e-3f && d0 >= -0.998f && d1 <= -2e-3f && d1 >= -0.998f) return -1;
-  return 0;
-}
-
-template <class V, int BX, int SGN, bool CHECK>
-__device__ __forceinline__ void half_samples(const V* __restrict__ s, int kind, bool hit_a, bool hit_b,
-                                             const RayFrame& fa, const RayFrame& fb, float& kfa, float& kfb,
-                                             float Nf, float lo, float hi, float cmo, unsigned maxidx,
-                                             unsigned maxidx3, float& acca, float& accb, int& bad) {
-  if (kind != 0) {
-    const bool al = kind > 0;
-    float accl = al ? acca : accb, accu = al ? accb : acca;
-    constexpr int QY = kQuadBoxY;
-    pair_samples<V, BX, SGN, CHECK, QY>(s, kfa, Nf, fa.ce0, fa.cd0, fa.dce, fa.dcd, fa.idcd, al ? fa.c0z : fb.c0z,
-                                        al ? fa.dcz : fb.dcz, al ? fb.c0z : fa.c0z, al ? fb.dcz : fa.dcz, lo, hi,
-                                        cmo, maxidx, maxidx3, accl, accu, bad);
-    acca = al ? accl : accu;
-    accb = al ? accu : accl;
-    return;
-  }
-  constexpr int QY = kQuadBoxY;
-  if (hit_a)
-    slab_samples<V, BX, SGN, CHECK, QY>(s, kfa, Nf, fa.ce0, fa.cd0, fa.c0z, fa.dce, fa.dcd, fa.idcd, fa.dcz, lo, hi,
-                                        cmo, maxidx, acca, bad);
-  if (hit_b)
-    slab_samples<V, BX, SGN, CHECK, QY>(s, kfb, Nf, fb.ce0, fb.cd0, fb.c0z, fb.dce, fb.dcd, fb.idcd, fb.dcz, lo, hi,
-                                        cmo, maxidx, accb, bad);
-}
-
-// CTAs per SM the register budget is sized for: four 128-thread CTAs (124
-// registers, no spills), as many as the fp32 boxes of 16x32 tiles leave room
-// for; the half-size 16-bit boxes leave room for five (96 registers).
-#ifndef CBCT_QUAD_MINB16
-#define CBCT_QUAD_MINB16 5
-#endif
-template <class V>
-constexpr int quad_min_blocks() {
-#ifdef CBCT_QUAD_MINB
-  return CBCT_QUAD_MINB;
-#else
-  return kQuadThreads >= 256 ? 2 : kQuadThreads >= 128 ? (sizeof(V) == 4 ? 4 : CBCT_QUAD_MINB16) : 6;
-#endif
-}
-
-// One CTA of the row-quad kernel (see fwd_slab_body).
-template <class V, int BX, bool CHECK>
-__device__ __forceinline__ void fwd_quad_body(const CUtensorMap* map_v, const CUtensorMap* map_t,
-                                              const V* __restrict__ vol, const ViewParams* __restrict__ views,
-                                              const GridConst& gc, int BZ, int nsl_max, const FwdOut& o,
-                                              int* flags, const TileId& tile, unsigned char* smem_raw,
-                                              PairShared& sh) {
-  constexpr int BXY = BX * kQuadBoxY;
-  const ViewParams vp = views[tile.z];
-  const int dom = vp.dom;
-  const CUtensorMap* map = dom ? map_v : map_t;
-  const int tid = threadIdx.x;
-  const int p = tile.z;
-  const int u0 = tile.x * kQU, v0 = tile.y * kQV;
-  const int u = u0 + (tid % kQU), vq = v0 + 4 * (tid / kQU);
-  const int uc = min(u, gc.W - 1);
-  const float Nf = float(gc.N);
-  Ray r[4];
-  bool act[4], hit[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    act[i] = (u < gc.W) && (vq + i < gc.H);
-    r[i] = make_ray(vp, gc, uc, min(vq + i, gc.H - 1));
-    hit[i] = act[i] && (r[i].a2 > r[i].a1);
-  }
-  RayFrame f[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) f[i] = ray_frame(r[i], dom);
-  // Quad test: one clip; sorted by z (rows run one way), every ray within
-  // [0.002, 1.998] texels above the lowest at both ends, the second-lowest
-  // within [0.002, 0.998].
-  bool quad = hit[0] && hit[1] && hit[2] && hit[3];
-#pragma unroll
-  for (int i = 1; i < 4; ++i) quad = quad && r[i].a1 == r[0].a1 && r[i].a2 == r[0].a2;
-  const bool up = r[1].c0z > r[0].c0z;   // z grows with the row
-  if (quad) {
-    const int lo_i = up ? 0 : 3;
-    const float zs = r[lo_i].c0z, ze = fmaf(Nf - 1.f, r[lo_i].dcz, r[lo_i].c0z);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (i == lo_i) continue;
-      const float d0 = r[i].c0z - zs, d1 = fmaf(Nf - 1.f, r[i].dcz, r[i].c0z) - ze;
-      const float dmax = (up ? i == 1 : i == 2) ? 0.998f : 1.998f;
-      quad = quad && d0 >= 2e-3f && d0 <= dmax && d1 >= 2e-3f && d1 <= dmax;
-    }
-  }
-  // Sorted z parameters of the quad (lowest first).
-  const float4 qz0 = up ? make_float4(f[0].c0z, f[1].c0z, f[2].c0z, f[3].c0z)
-                        : make_float4(f[3].c0z, f[2].c0z, f[1].c0z, f[0].c0z);
-  const float4 qdz = up ? make_float4(f[0].dcz, f[1].dcz, f[2].dcz, f[3].dcz)
-                        : make_float4(f[3].dcz, f[2].dcz, f[1].dcz, f[0].dcz);
-  const int kind01 = quad ? 0 : pair_kind(r[0], r[1], hit[0], hit[1], Nf);
-  const int kind23 = quad ? 0 : pair_kind(r[2], r[3], hit[2], hit[3], Nf);
-  const float ke_ = dom ? gc.kx : gc.ky, be = dom ? gc.bx : gc.by;
-  const float kd = dom ? gc.ky : gc.kx, bd = dom ? gc.by : gc.bx;
-  const float Se = dom ? vp.Sx : vp.Sy, Sd = dom ? vp.Sy : vp.Sx;
-
-  if (tid == 0) {
-    sh.mlo = INT_MAX;
-    sh.mhi = INT_MIN;
-    sh.abort_flag = 0;
-    for (int st = 0; st < kPairStages; ++st) mbar_init(&sh.bars[st], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  {
-    int mn = INT_MAX, mx = INT_MIN;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (!hit[i]) continue;
-      const int m0 = (max(int(floorf(f[i].cd0)), kSlabBase) - kSlabBase) / kTS;
-      const int m1 = (max(int(floorf(fmaf(Nf - 1.f, f[i].dcd, f[i].cd0))), kSlabBase) - kSlabBase) / kTS;
-      mn = min(mn, min(m0, m1));
-      mx = max(mx, max(m0, m1));
-    }
-    if (mn <= mx) {
-      atomicMin(&sh.mlo, mn);
-      atomicMax(&sh.mhi, mx);
-    }
-  }
-  __syncthreads();
-  const int mlo = sh.mlo, mhi = sh.mhi;
-  int nslab = (mhi >= mlo) ? (mhi - mlo + 1) : 0;
-  if (nslab > nsl_max) {
-    if (tid == 0) atomicAdd(&flags[0], 1);
-    nslab = 0;
-  }
-  const uint32_t box_bytes = uint32_t(BX * kQuadBoxY * BZ * sizeof(V));
-  const uint32_t stage_stride = (box_bytes + 127u) & ~127u;
-  int* const emin = reinterpret_cast<int*>(smem_raw + kPairStages * stage_stride);
-  int* const emax = emin + nsl_max;
-  int* const zmin = emax + nsl_max;
-  int* const zmax = zmin + nsl_max;
-  for (int i = tid; i < nslab; i += blockDim.x) {
-    emin[i] = INT_MAX; emax[i] = INT_MIN;
-    zmin[i] = INT_MAX; zmax[i] = INT_MIN;
-  }
-  __syncthreads();
-  const int ue = min(u0 + kQU, gc.W) - 1, ve = min(v0 + kQV, gc.H) - 1;
-  const int ne = dom ? gc.nx : gc.ny;
-  for (int qq = tid; qq < nslab * 8; qq += blockDim.x) {
-    const int i = qq >> 3, c = qq & 7;
-    const int m = mlo + i;
-    const float plane = float(kSlabBase + m * kTS + ((c & 4) ? kTS : 0));
-    const int ucc = (c & 1) ? ue : u0, vcc = (c & 2) ? ve : v0;
-    const float dx = fmaf(float(ucc), vp.Eux, vp.D0x);
-    const float dy = fmaf(float(ucc), vp.Euy, vp.D0y);
-    const float dzz = fmaf(float(vcc), vp.Evz, vp.D0z);
-    const float de = dom ? dx : dy, dd = dom ? dy : dx;
-    const float t = ((plane - bd) / kd - Sd) / dd;
-    const float ce = fmaf(fmaf(t, de, Se), ke_, be);
-    const float cz = fmaf(t * dzz, gc.kz, gc.bz);
-    const int fe = min(max(int(floorf(fminf(fmaxf(ce, -1.0e5f), 1.0e5f))), -1), ne - 1);
-    const int fz = min(max(int(floorf(fminf(fmaxf(cz, -1.0e5f), 1.0e5f))), -1), gc.nz - 1);
-    atomicMin(&emin[i], fe);
-    atomicMax(&emax[i], fe);
-    atomicMin(&zmin[i], fz);
-    atomicMax(&zmax[i], fz);
-  }
-  __syncthreads();
-
-  const unsigned maxidx = unsigned(BXY * (BZ - 1) - BX - 2);   // two-plane loads stay in the box
-  const unsigned maxidx3 = unsigned(BXY * BZ - BX - 2);        // the pair's third plane
-  auto origin = [&](int i, int& oe, int& od, int& oz, int& m) {
-    m = (vp.dsgn > 0) ? mlo + i : mhi - i;
-    const int ii = m - mlo;
-    oe = (emin[ii] - 1) & ~(int(16 / sizeof(V)) - 1);   // 16-byte aligned x start
-    od = kSlabBase + m * kTS;
-    oz = zmin[ii] - 1;
-  };
-  auto issue = [&](int i) {
-    int oe, od, oz, m;
-    origin(i, oe, od, oz, m);
-    uint64_t* bar = &sh.bars[i % kPairStages];
-    mbar_arrive_expect_tx(bar, box_bytes);
-    tma_load_3d(smem_raw + (i % kPairStages) * stage_stride, map, oe, od, oz, bar);
-  };
-  if (tid == 0) {
-    for (int i = 0; i < min(kPairStages, nslab); ++i) issue(i);
-  }
-
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);   // quad: sorted by z; else per row
-  float kf[4] = {0.f, 0.f, 0.f, 0.f};            // quad / pairs: kf[0], kf[2] lead
-  int bad = 0;
-  int done = 0;
-  for (int i = 0; i < nslab; ++i) {
-    const int slot = i % kPairStages;
-    const bool ok = mbar_wait_bounded(&sh.bars[slot], (i / kPairStages) & 1, gc.wait_limit);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) { atomicAdd(&flags[1], 1); sh.abort_flag = 1; }
-      break;
-    }
-    done = i + 1;
-    int oe, od, oz, m;
-    origin(i, oe, od, oz, m);
-    if (CHECK && tid == 0) {
-      const int ii = m - mlo;
-      if (emax[ii] + 2 - oe >= BX || zmax[ii] + 2 - oz >= BZ) atomicAdd(&flags[0], 1);
-    }
-    const V* sm = reinterpret_cast<const V*>(smem_raw + slot * stage_stride);
-    const float lo = float(od), hi = lo + float(kTS);
-    const float cmo = kRoundC - float(oe + od * BX + oz * BXY);
-    if (quad) {
-      if (vp.dsgn > 0)
-        quad_samples<V, BX, 1, CHECK>(sm, kf[0], Nf, f[0].ce0, f[0].cd0, f[0].dce, f[0].dcd, f[0].idcd, qz0, qdz, lo,
-                                      hi, cmo, maxidx, acc, bad);
-      else
-        quad_samples<V, BX, -1, CHECK>(sm, kf[0], Nf, f[0].ce0, f[0].cd0, f[0].dce, f[0].dcd, f[0].idcd, qz0, qdz,
-                                       lo, hi, cmo, maxidx, acc, bad);
-    } else if (vp.dsgn > 0) {
-      half_samples<V, BX, 1, CHECK>(sm, kind01, hit[0], hit[1], f[0], f[1], kf[0], kf[1], Nf, lo, hi, cmo, maxidx,
-                                    maxidx3, acc.x, acc.y, bad);
-      half_samples<V, BX, 1, CHECK>(sm, kind23, hit[2], hit[3], f[2], f[3], kf[2], kf[3], Nf, lo, hi, cmo, maxidx,
-                                    maxidx3, acc.z, acc.w, bad);
-    } else {
-      half_samples<V, BX, -1, CHECK>(sm, kind01, hit[0], hit[1], f[0], f[1], kf[0], kf[1], Nf, lo, hi, cmo, maxidx,
-                                     maxidx3, acc.x, acc.y, bad);
-      half_samples<V, BX, -1, CHECK>(sm, kind23, hit[2], hit[3], f[2], f[3], kf[2], kf[3], Nf, lo, hi, cmo, maxidx,
-                                     maxidx3, acc.z, acc.w, bad);
-    }
-    __syncthreads();
-    if (tid == 0 && i + kPairStages < nslab) {
-      fence_proxy_async();
-      issue(i + kPairStages);
-    }
-  }
-  if (sh.abort_flag && tid == 0) {
-    for (int i = done; i < min(done + kPairStages, nslab); ++i)
-      if (!mbar_wait_bounded(&sh.bars[i % kPairStages], (i / kPairStages) & 1, kWaitLimit)) sh.abort_flag = 2;
-  }
-  if (CHECK) {
-    // every sample of a hit ray must be consumed
-    if (quad) {
-      if (kf[0] != Nf) bad = 1;
-    } else {
-      if (kind01 != 0 ? kf[0] != Nf : ((hit[0] && kf[0] != Nf) || (hit[1] && kf[1] != Nf))) bad = 1;
-      if (kind23 != 0 ? kf[2] != Nf : ((hit[2] && kf[2] != Nf) || (hit[3] && kf[3] != Nf))) bad = 1;
-    }
-    if (bad) atomicAdd(&flags[0], 1);
-  }
-  // Per-row sums (the quad's are sorted by z).
-  float sum[4];
-  if (quad && !up) {
-    sum[0] = acc.w; sum[1] = acc.z; sum[2] = acc.y; sum[3] = acc.x;
-  } else {
-    sum[0] = acc.x; sum[1] = acc.y; sum[2] = acc.z; sum[3] = acc.w;
-  }
-  double sq = 0.0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float val = grown_rays(vol, vp, gc, u, vq + i, act[i] && !hit[i]);
-    if (hit[i]) val = sum[i] * r[i].delta;
-    if (act[i]) sq += fwd_store(o, gc, vp, p, u, vq + i, val);
-  }
-  fwd_block_partial(o, sq, sh.red, tid, tile.bid);
-}
-
-template <class V, int BX, bool CHECK>
-__global__ void __launch_bounds__(kQuadThreads, quad_min_blocks<V>())
-    fwd_quad_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_t,
-                    const V* __restrict__ vol, const ViewParams* __restrict__ views, GridConst gc, int BZ,
-                    int nsl_max, FwdOut o, int* flags) {
-  extern __shared__ __align__(128) unsigned char smem_dyn[];
-  unsigned char* smem_raw =
-      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
-  __shared__ PairShared sh;
-  fwd_quad_body<V, BX, CHECK>(&map_v, &map_t, vol, views, gc, BZ, nsl_max, o, flags, launch_tile(), smem_raw, sh);
-}
-
 // ------------------------------------------------------------------ fan
 // The rays of one detector column lie in one vertical plane (the detector's
 // v axis is the world z axis).  A ray that enters and leaves the volume
@@ -1344,28 +935,16 @@ CUtensorMapDataType tma_dtype(cbct_dtype dt) {
 // until the list is empty and run the one-scan kernel's body on them, so every
 // ray gets the arithmetic of its own launch.  A scan's items are numbered in
 // its one-scan launch order (x fastest), which is also its partial-sum slot.
-enum { kVarSlab1 = 0, kVarSlab2 = 1, kVarPair = 2, kVarQuad = 3 };
-
-struct alignas(128) FwdScanRec {
-  CUtensorMap map_v, map_t;    // volume and x/y-transposed volume, the plan's box
-  const void* vol;
-  const ViewParams* views;     // the subset's views
-  int* flags;
-  GridConst gc;
-  FwdOut o;
-  int BZ, nsl_max;
-  int tx, ty;                  // ray tiles per view (x, y)
-  int base;                    // work-list index of the scan's first tile
-};
+enum { kVarSlab1 = 0, kVarSlab2 = 1, kVarPair = 2, kVars = 3 };
 
 template <int VAR>
-constexpr int var_threads() { return VAR == kVarPair ? kPairThreads : VAR == kVarQuad ? kQuadThreads : 256; }
+constexpr int var_threads() { return VAR == kVarPair ? kPairThreads : 256; }
 template <int VAR, class V>
 constexpr int var_min_blocks() {
 #ifdef CBCT_MULTI_PAIR_MINB
   if (VAR == kVarPair) return CBCT_MULTI_PAIR_MINB;
 #endif
-  return VAR == kVarPair ? pair_min_blocks<V>() : VAR == kVarQuad ? quad_min_blocks<V>() : slab_min_blocks<V>();
+  return VAR == kVarPair ? pair_min_blocks<V>() : slab_min_blocks<V>();
 }
 
 template <int VAR, class V, int BX>
@@ -1406,11 +985,8 @@ __global__ void __launch_bounds__(var_threads<VAR>(), var_min_blocks<VAR, V>())
       fwd_slab_body<V, BX, false, 1>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.o, R.flags, tile, smem_raw, sh);
     else if constexpr (VAR == kVarSlab2)
       fwd_slab_body<V, BX, false, 2>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.o, R.flags, tile, smem_raw, sh);
-    else if constexpr (VAR == kVarPair)
-      fwd_pair_body<V, BX, false>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.nsl_max, R.o, R.flags, tile,
-                                  smem_raw, sh);
     else
-      fwd_quad_body<V, BX, false>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.nsl_max, R.o, R.flags, tile,
+      fwd_pair_body<V, BX, false>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.nsl_max, R.o, R.flags, tile,
                                   smem_raw, sh);
     __syncthreads();
     // A wait that gave up is counted in the scan's flag word and its loads
@@ -1424,7 +1000,9 @@ __global__ void __launch_bounds__(var_threads<VAR>(), var_min_blocks<VAR, V>())
   }
 }
 
-CUtensorMap make_map(cbct_dtype dt, const void* vol, int n0, int n1, int n2, const SlabBox& b) {
+}  // namespace
+
+CUtensorMap make_volume_map(cbct_dtype dt, const void* vol, int n0, int n1, int n2, const SlabBox& b) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
   const size_t es = dtype_size(dt);
@@ -1439,6 +1017,8 @@ CUtensorMap make_map(cbct_dtype dt, const void* vol, int n0, int n1, int n2, con
     throw Error(CBCT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)res));
   return m;
 }
+
+namespace {
 
 // Dynamic shared memory of a slab or fan launch: kNStage TMA stages of the
 // box (128-byte aligned) + the fan kernel's lines + alignment slack.
@@ -1478,8 +1058,8 @@ template <class V, int BX>
 void launch_slab(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, dim3 grid, int first,
                  cudaStream_t st, cbct_dtype dt) {
   const SlabBox& b = box_for<V>(p);
-  const CUtensorMap mv = make_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = make_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
+  const CUtensorMap mv = make_volume_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
+  const CUtensorMap mt = make_volume_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
                                   volT ? p->g.nx : p->g.ny, p->g.nz, b);
   size_t smem = 0;
   const bool two = slab_stages<V>(b, smem) == 2;
@@ -1498,8 +1078,8 @@ template <class V, int BX>
 void launch_pair(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
                  cbct_dtype dt) {
   const SlabBox& b = pair_box_for<V>(p);
-  const CUtensorMap mv = make_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = make_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
+  const CUtensorMap mv = make_volume_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
+  const CUtensorMap mt = make_volume_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
                                   volT ? p->g.nx : p->g.ny, p->g.nz, b);
   const int nsl = slabs_max(p->g);
   const size_t smem = pair_smem(b, sizeof(V), nsl);
@@ -1517,39 +1097,14 @@ void launch_pair(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int
 }
 
 template <class V>
-const SlabBox& quad_box_for(const cbct_plan* p) { return sizeof(V) == 4 ? p->quad : p->quad16; }
-
-template <class V, int BX>
-void launch_quad(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
-                 cbct_dtype dt) {
-  const SlabBox& b = quad_box_for<V>(p);
-  const CUtensorMap mv = make_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = make_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
-                                  volT ? p->g.nx : p->g.ny, p->g.nz, b);
-  const int nsl = slabs_max(p->g);
-  const size_t smem = pair_smem(b, sizeof(V), nsl);
-  const dim3 grid((p->g.width + kQU - 1) / kQU, (p->g.height + kQV - 1) / kQV, cnt);
-  if (p->debug_checks) {
-    auto k = fwd_quad_kernel<V, BX, true>;
-    ensure_smem_attr((const void*)k, smem);
-    k<<<grid, kQuadThreads, smem, st>>>(mv, mt, vol, p->d_views + first, p->gc, b.bz, nsl, o, p->d_flags);
-  } else {
-    auto k = fwd_quad_kernel<V, BX, false>;
-    ensure_smem_attr((const void*)k, smem);
-    k<<<grid, kQuadThreads, smem, st>>>(mv, mt, vol, p->d_views + first, p->gc, b.bz, nsl, o, p->d_flags);
-  }
-  check_launch("fwd_quad_kernel");
-}
-
-template <class V>
 const SlabBox& fan_box_for(const cbct_plan* p) { return sizeof(V) == 4 ? p->fan : p->fan16; }
 
 template <class V, int BX>
 void launch_fan(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
                 cbct_dtype dt) {
   const SlabBox& b = fan_box_for<V>(p);
-  const CUtensorMap mv = make_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = make_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
+  const CUtensorMap mv = make_volume_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
+  const CUtensorMap mt = make_volume_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
                                   volT ? p->g.nx : p->g.ny, p->g.nz, b);
   const int nsl = slabs_max(p->g);
   const size_t smem = forward_smem(b, sizeof(V), p->fan_lz, nsl);
@@ -1586,14 +1141,7 @@ void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaS
     volT = t;
   }
   if (p->fwd_variant == 4) {
-    switch (quad_box_for<V>(p).bx) {
-      case 40: launch_quad<V, 40>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 56: launch_quad<V, 56>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 72: launch_quad<V, 72>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 104: launch_quad<V, 104>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 136: launch_quad<V, 136>(p, vol, volT, o, first, cnt, st, dt); break;
-      default: throw Error(CBCT_ERR_INTERNAL, "unsupported quad box width");
-    }
+    quad_launch(p, dt, vol, volT, o, first, cnt, st);
     return;
   }
   if (p->fwd_variant == 3) {
@@ -1636,12 +1184,6 @@ void prepare_width(size_t smem) {
 }
 
 template <class V, int BX>
-void prepare_quad_width(size_t smem) {
-  ensure_smem_attr((const void*)fwd_quad_kernel<V, BX, false>, smem);
-  ensure_smem_attr((const void*)fwd_quad_kernel<V, BX, true>, smem);
-}
-
-template <class V, int BX>
 void prepare_pair_width(size_t smem) {
   ensure_smem_attr((const void*)fwd_pair_kernel<V, BX, false>, smem);
   ensure_smem_attr((const void*)fwd_pair_kernel<V, BX, true>, smem);
@@ -1655,18 +1197,6 @@ void prepare_fan_width(size_t smem) {
 
 template <class V>
 void prepare_typed(const cbct_plan* p) {
-  if (p->fwd_variant == 4) {
-    const SlabBox& b = quad_box_for<V>(p);
-    const size_t qs = pair_smem(b, sizeof(V), slabs_max(p->g));
-    switch (b.bx) {
-      case 40: prepare_quad_width<V, 40>(qs); break;
-      case 56: prepare_quad_width<V, 56>(qs); break;
-      case 72: prepare_quad_width<V, 72>(qs); break;
-      case 104: prepare_quad_width<V, 104>(qs); break;
-      case 136: prepare_quad_width<V, 136>(qs); break;
-      default: break;
-    }
-  }
   if (p->fwd_variant == 3) {
     const SlabBox& b = pair_box_for<V>(p);
     const size_t ps = pair_smem(b, sizeof(V), slabs_max(p->g));
@@ -1690,6 +1220,7 @@ void prepare_typed(const cbct_plan* p) {
       default: break;
     }
   }
+  if (p->fwd_variant != 1) return;
   const SlabBox& b = box_for<V>(p);
   const size_t smem = forward_smem(b, sizeof(V), 0);
   switch (b.bx) {
@@ -1708,7 +1239,7 @@ void prepare_typed(const cbct_plan* p) {
 // (corner-ray bounding box in the view's frame, computed in FP64): e extent
 // and z extent in elements, including margins.  False when some view cannot
 // use slabs (a ray not dominated by its view's slab axis, or too many slabs).
-static bool slab_extents(const cbct_plan* p, int TU, int TV, int& ext_e, int& ext_z) {
+bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& ext_z) {
   const cbct_geometry& g = p->g;
   const double kx = g.nx / (double)g.lx, ky = g.ny / (double)g.ly, kz = g.nz / (double)g.lz;
   const double bx = g.nx / 2.0 - 0.5, by = g.ny / 2.0 - 0.5, bz = g.nz / 2.0 - 0.5;
@@ -1727,13 +1258,15 @@ static bool slab_extents(const cbct_plan* p, int TU, int TV, int& ext_e, int& ex
       const int Nd = dom ? g.ny : g.nx;
       const double ke = dom ? kx : ky, be = dom ? bx : by, kd = dom ? ky : kx, bd = dom ? by : bx;
       const double Se = dom ? vp.Sx : vp.Sy, Sd = dom ? vp.Sy : vp.Sx;
-      const int nsl = (Nd + 1 - kSlabBase + kTS - 1) / kTS + 1;
-      if (nsl > kMaxSlabs) { a.ok = 0; break; }
+      const int nsl = (Nd + 1 - kSlabBase + TS - 1) / TS + 1;
+      if (nsl * TS > kMaxSlabs * kTS) { a.ok = 0; break; }
       for (int tv = 0; tv < tiles_v; ++tv) {
         const int v0 = tv * TV, ve = std::min(v0 + TV, g.height) - 1;
         dz0[tv] = vp.D0z + v0 * (double)vp.Evz;
         dz1[tv] = vp.D0z + ve * (double)vp.Evz;
       }
+      const double dzabs = std::max(std::fabs(dz0[0]), std::fabs(dz1[tiles_v - 1]));
+      const double dzspan = (TV - 1) * (double)vp.Evz;
       for (int tu = 0; tu < tiles_u && a.ok; ++tu) {
         const int uc[2] = {tu * TU, std::min(tu * TU + TU, g.width) - 1};
         double de[2], dd[2];
@@ -1748,7 +1281,7 @@ static bool slab_extents(const cbct_plan* p, int TU, int TV, int& ext_e, int& ex
         for (int m = 0; m < nsl; ++m) {
           double emn = 1e30, emx = -1e30, tmn = 1e30, tmx = -1e30;
           for (int c = 0; c < 4; ++c) {
-            const double plane = kSlabBase + m * kTS + ((c & 2) ? kTS : 0);
+            const double plane = kSlabBase + m * TS + ((c & 2) ? TS : 0);
             const double t = ((plane - bd) / kd - Sd) / dd[c & 1];
             const double ce = (Se + t * de[c & 1]) * ke + be;
             emn = std::min(emn, ce); emx = std::max(emx, ce);
@@ -1757,11 +1290,18 @@ static bool slab_extents(const cbct_plan* p, int TU, int TV, int& ext_e, int& ex
           // elements from floor(min)-1 to floor(max)+1 inclusive, +2 margin; the
           // kernels clamp footprints to the volume, whose extent bounds the box
           const int Ne = dom ? g.nx : g.ny;
+          // a slab where the tile's rays are beside the volume holds no samples
+          if (emx < -1.0 || emn > Ne) continue;
           a.e = std::max(a.e, std::min((int)(std::floor(emx) - std::floor(emn)) + 3 + 2, Ne + 4));
+          // A tile row inside the volume spans at most this in z: skip the rows
+          // where none can exceed the extent found so far.
+          const double dmax = std::min(dzabs, (g.nz + 1.0 - bz) / (kz * std::max(tmn, 1e-9)));
+          if (tmn > 0 && std::ceil(kz * ((tmx - tmn) * dmax + tmx * dzspan)) + 3 + 2 <= a.z) continue;
           for (int tv = 0; tv < tiles_v; ++tv) {
             const double z00 = tmn * dz0[tv], z01 = tmn * dz1[tv], z10 = tmx * dz0[tv], z11 = tmx * dz1[tv];
             const double zmn = std::min(std::min(z00, z01), std::min(z10, z11)) * kz + bz;
             const double zmx = std::max(std::max(z00, z01), std::max(z10, z11)) * kz + bz;
+            if (zmx < -1.0 || zmn > g.nz) continue;
             const int ez = (int)(std::floor(zmx) - std::floor(zmn)) + 3 + 2;
             a.z = std::max(a.z, std::min(ez, g.nz + 4));
           }
@@ -1796,10 +1336,11 @@ static double row_dz_max(const cbct_plan* p) {
 }
 
 // Chooses the forward variant and its TMA boxes from the plan geometry: the
-// row-pair kernel where adjacent detector rows are less than one z texel
-// apart over the whole volume (so pairs share their planes) and its boxes fit,
-// else the per-ray slab kernel where its boxes fit, else the gather kernel.
-// CBCT_OPT_FORWARD_KERNEL forces slab (1), gather (2), fan (3) or pairs (4).
+// row-quad kernel by quad_choose's rule, else the row-pair kernel where adjacent
+// detector rows are less than one z texel apart over the whole volume (so pairs
+// share their planes) and its boxes fit, else the per-ray slab kernel where its
+// boxes fit, else the gather kernel.  CBCT_OPT_FORWARD_KERNEL forces slab (1),
+// gather (2), fan (3), pairs (4) or quads (5).
 void forward_choose_variant(cbct_plan* p) {
   p->fwd_variant = 0;
   p->slab = SlabBox{0, 0, 0, 0};
@@ -1819,8 +1360,13 @@ void forward_choose_variant(cbct_plan* p) {
       if (w >= ext + slack) return w;
     return 0;
   };
+  const double row_dz = row_dz_max(p);
+  if ((p->fwd_pref == 0 || p->fwd_pref == 5) && quad_choose(p, row_dz, p->fwd_pref == 5)) {
+    p->fwd_variant = 4;
+    return;
+  }
   int e, z;
-  if (slab_extents(p, kTU, kTV, e, z)) {
+  if (slab_extents(p, kTU, kTV, kTS, e, z)) {
     const int w32 = width(kBoxWidths, e, 3), w16 = width(kBoxWidths, e, 7);
     const int boxz = std::max(z, 2);
     const SlabBox b32{w32, kBoxY, boxz, 1}, b16{w16, kBoxY, boxz, 1};
@@ -1832,9 +1378,8 @@ void forward_choose_variant(cbct_plan* p) {
       p->fwd_variant = 1;
     }
   }
-  const double row_dz = row_dz_max(p);
   if ((p->fwd_pref == 4 || (p->fwd_pref == 0 && p->fwd_variant == 1 && row_dz < 0.99)) &&
-      slab_extents(p, kPU, kPV, e, z)) {
+      slab_extents(p, kPU, kPV, kTS, e, z)) {
     const int w32 = width(kBoxWidths, e, 3), w16 = width(kBoxWidths, e, 7);
     const int boxz = std::max(z, 3);
     const SlabBox b32{w32, kPairBoxY, boxz, 1}, b16{w16, kPairBoxY, boxz, 1};
@@ -1846,22 +1391,7 @@ void forward_choose_variant(cbct_plan* p) {
       p->fwd_variant = 3;
     }
   }
-  // Row quads where four adjacent rows stay within two z texels (3 row steps
-  // under 0.66 texel each, margin included).
-  if ((p->fwd_pref == 5 || (p->fwd_pref == 0 && p->fwd_variant == 3 && row_dz < 0.66)) &&
-      slab_extents(p, kQU, kQV, e, z)) {
-    const int w32 = width(kBoxWidths, e, 3), w16 = width(kBoxWidths, e, 7);
-    const int boxz = std::max(z, 4);
-    const SlabBox b32{w32, kQuadBoxY, boxz, 1}, b16{w16, kQuadBoxY, boxz, 1};
-    const int nsl = slabs_max(p->g);
-    if (w32 && w16 && boxz <= 256 && pair_smem(b32, 4, nsl) <= (size_t)kSmemBudget &&
-        pair_smem(b16, 2, nsl) <= (size_t)kSmemBudget) {
-      p->quad = b32;
-      p->quad16 = b16;
-      p->fwd_variant = 4;
-    }
-  }
-  if (p->fwd_pref == 3 && slab_extents(p, kFU, kFV, e, z)) {
+  if (p->fwd_pref == 3 && slab_extents(p, kFU, kFV, kTS, e, z)) {
     const int w32 = width(kFanWidths, e, 3), w16 = width(kFanWidths, e, 7);
     const int boxz = std::max(z, 2);
     const int lz = (boxz + 1) | 1;  // odd: consecutive lines start in different banks
@@ -1882,6 +1412,7 @@ void forward_prepare(cbct_plan* p) {
   prepare_typed<float>(p);
   prepare_typed<__half>(p);
   prepare_typed<__nv_bfloat16>(p);
+  if (p->fwd_variant == 4) quad_prepare(p);
   bool any_x = false;
   for (size_t s = 0; s < p->subset_has_xdom.size(); ++s) any_x = any_x || p->subset_has_xdom[s];
   if (any_x && !p->d_volT)
@@ -1917,7 +1448,8 @@ void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, floa
   // One partial sum per block of the kernel that will run.
   const bool fan = use_slab && p->fwd_variant == 2, pair = use_slab && p->fwd_variant == 3;
   const bool quad = use_slab && p->fwd_variant == 4;
-  const int TU = fan ? kFU : pair ? kPU : quad ? kQU : kTU, TV = fan ? kFV : pair ? kPV : quad ? kQV : kTV;
+  int TU = fan ? kFU : pair ? kPU : kTU, TV = fan ? kFV : pair ? kPV : kTV;
+  if (quad) quad_tile(p->quad_shape, TU, TV);
   const size_t nblocks = (size_t)((p->g.width + TU - 1) / TU) * ((p->g.height + TV - 1) / TV) * cnt;
   if (norm2_out) {
     if (nblocks > p->n_partials) throw Error(CBCT_ERR_INTERNAL, "partials buffer too small");
@@ -1934,60 +1466,51 @@ void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, floa
 
 namespace {
 
-template <int VAR, int BX>
-void add_fwd_group(WorkArena& A, const std::vector<FwdScanRec>& recs, int total, size_t smem) {
-  auto k = fwd_multi_kernel<VAR, float, BX>;
+// Work-list launch of kernel k over the records of one group.
+void add_fwd_group(WorkArena& A, FwdMultiKernel k, int threads, const std::vector<FwdScanRec>& recs, int total,
+                   size_t smem) {
   ensure_smem_attr((const void*)k, smem);
   const size_t off = A.add(recs.data(), recs.size() * sizeof(FwdScanRec));
   const int ci = A.n_counters++;
-  const int threads = var_threads<VAR>();
   const int grid = std::min(total, resident_grid((const void*)k, threads, smem));
   const int n = (int)recs.size();
   A.ops.push_back([&A, k, off, ci, grid, threads, n, total, smem](cudaStream_t st) {
     k<<<grid, threads, smem, st>>>(reinterpret_cast<const FwdScanRec*>(A.dev + off), n, total, A.counter(ci));
-    check_launch("fwd_multi_kernel");
+    check_launch("forward work-list kernel");
   });
 }
 
 template <int VAR>
-const void* fwd_multi_ptr_v(int c) {
-  switch (kBoxWidths[c]) {
-    case 40: return (const void*)fwd_multi_kernel<VAR, float, 40>;
-    case 56: return (const void*)fwd_multi_kernel<VAR, float, 56>;
-    case 72: return (const void*)fwd_multi_kernel<VAR, float, 72>;
-    case 104: return (const void*)fwd_multi_kernel<VAR, float, 104>;
-    case 136: return (const void*)fwd_multi_kernel<VAR, float, 136>;
+FwdMultiKernel fwd_multi_ptr_v(int bx) {
+  switch (bx) {
+    case 40: return fwd_multi_kernel<VAR, float, 40>;
+    case 56: return fwd_multi_kernel<VAR, float, 56>;
+    case 72: return fwd_multi_kernel<VAR, float, 72>;
+    case 104: return fwd_multi_kernel<VAR, float, 104>;
+    case 136: return fwd_multi_kernel<VAR, float, 136>;
     default: throw Error(CBCT_ERR_INTERNAL, "unsupported forward box width");
   }
 }
 
-const void* fwd_multi_ptr(int var, int c) {
-  return var == kVarSlab1 ? fwd_multi_ptr_v<kVarSlab1>(c) : var == kVarSlab2 ? fwd_multi_ptr_v<kVarSlab2>(c)
-         : var == kVarPair ? fwd_multi_ptr_v<kVarPair>(c) : fwd_multi_ptr_v<kVarQuad>(c);
+FwdMultiKernel fwd_multi_ptr(int var, int bx) {
+  return var == kVarSlab1   ? fwd_multi_ptr_v<kVarSlab1>(bx)
+         : var == kVarSlab2 ? fwd_multi_ptr_v<kVarSlab2>(bx)
+                            : fwd_multi_ptr_v<kVarPair>(bx);
 }
 
-int var_threads_of(int var) {
-  return var == kVarPair ? var_threads<kVarPair>() : var == kVarQuad ? var_threads<kVarQuad>() : 256;
-}
-
-template <int VAR>
-void add_fwd_group_w(WorkArena& A, int c, const std::vector<FwdScanRec>& g, int total, size_t smem) {
-  switch (kBoxWidths[c]) {
-    case 40: add_fwd_group<VAR, 40>(A, g, total, smem); break;
-    case 56: add_fwd_group<VAR, 56>(A, g, total, smem); break;
-    case 72: add_fwd_group<VAR, 72>(A, g, total, smem); break;
-    case 104: add_fwd_group<VAR, 104>(A, g, total, smem); break;
-    case 136: add_fwd_group<VAR, 136>(A, g, total, smem); break;
-    default: throw Error(CBCT_ERR_INTERNAL, "unsupported forward box width");
-  }
-}
+// The scans of one kernel (kind, shape and box width).
+struct FwdGroup {
+  FwdMultiKernel k;
+  int threads;
+  std::vector<FwdScanRec> recs;
+  int total = 0;
+  size_t smem = 0;
+};
 
 }  // namespace
 
 void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
-  std::vector<FwdScanRec> groups[4][5];
-  int totals[4][5] = {};
-  size_t smem[4][5] = {};
+  std::vector<FwdGroup> groups;
   // Transposes of the volumes the next launches read, one launch for all.
   std::vector<TransposeRec> tr;
   int tr_total = 0;
@@ -2002,16 +1525,13 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
     tr.clear();
     tr_total = 0;
   };
-  auto flush = [&](int v, int c) {
-    if (groups[v][c].empty()) return;
+  auto flush = [&](FwdGroup& g) {
+    if (g.recs.empty()) return;
     flush_transposes();
-    if (v == kVarSlab1) add_fwd_group_w<kVarSlab1>(A, c, groups[v][c], totals[v][c], smem[v][c]);
-    else if (v == kVarSlab2) add_fwd_group_w<kVarSlab2>(A, c, groups[v][c], totals[v][c], smem[v][c]);
-    else if (v == kVarPair) add_fwd_group_w<kVarPair>(A, c, groups[v][c], totals[v][c], smem[v][c]);
-    else add_fwd_group_w<kVarQuad>(A, c, groups[v][c], totals[v][c], smem[v][c]);
-    groups[v][c].clear();
-    totals[v][c] = 0;
-    smem[v][c] = 0;
+    add_fwd_group(A, g.k, g.threads, g.recs, g.total, g.smem);
+    g.recs.clear();
+    g.total = 0;
+    g.smem = 0;
   };
   std::vector<std::function<void(cudaStream_t)>> after;
   for (const MultiFwdJob& j : jobs) {
@@ -2031,32 +1551,36 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
       one_scan(j);
       continue;
     }
-    const int nsl = slabs_max(p->g);
-    int var, TU, TV;
+    int nsl = slabs_max(p->g), TU, TV, threads;
     SlabBox b;
     size_t sm = 0;
+    FwdMultiKernel kernel;
     if (fv == 4) {
-      b = p->quad; var = kVarQuad; TU = kQU; TV = kQV; sm = pair_smem(b, 4, nsl);
+      const QuadMulti q = quad_multi(p);
+      b = p->quad; kernel = q.kernel; nsl = q.nsl; sm = q.smem; threads = q.threads;
+      quad_tile(p->quad_shape, TU, TV);
     } else if (fv == 3) {
-      b = p->pair; var = kVarPair; TU = kPU; TV = kPV; sm = pair_smem(b, 4, nsl);
+      b = p->pair; TU = kPU; TV = kPV; sm = pair_smem(b, 4, nsl); threads = kPairThreads;
+      kernel = fwd_multi_ptr(kVarPair, b.bx);
     } else {
-      b = p->slab; TU = kTU; TV = kTV;
-      var = slab_stages<float>(b, sm) == 2 ? kVarSlab2 : kVarSlab1;
+      b = p->slab; TU = kTU; TV = kTV; threads = 256;
+      kernel = fwd_multi_ptr(slab_stages<float>(b, sm) == 2 ? kVarSlab2 : kVarSlab1, b.bx);
     }
-    int w = -1;
-    for (int c = 0; c < 5; ++c)
-      if (kBoxWidths[c] == b.bx) w = c;
-    if (w < 0) throw Error(CBCT_ERR_INTERNAL, "unsupported forward box width");
     const int tx = (p->g.width + TU - 1) / TU, ty = (p->g.height + TV - 1) / TV;
     const int nblocks = tx * ty * cnt;
-    {
-      const void* kfn = fwd_multi_ptr(var, w);
-      ensure_smem_attr(kfn, sm);
-      if (nblocks >= kMultiFillWaves * resident_grid(kfn, var_threads_of(var), sm)) {
-        one_scan(j);
-        continue;
-      }
+    ensure_smem_attr((const void*)kernel, sm);
+    if (nblocks >= kMultiFillWaves * resident_grid((const void*)kernel, threads, sm)) {
+      one_scan(j);
+      continue;
     }
+    auto gi = std::find_if(groups.begin(), groups.end(), [&](const FwdGroup& g) { return g.k == kernel; });
+    if (gi == groups.end()) {
+      FwdGroup ng;
+      ng.k = kernel;
+      ng.threads = threads;
+      gi = groups.insert(groups.end(), std::move(ng));
+    }
+    FwdGroup& g = *gi;
     const float* volT = nullptr;
     if (p->subset_has_xdom[s]) {
       float* t = static_cast<float*>(p->d_volT);
@@ -2079,8 +1603,8 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
     o.wproj = p->d_pweights ? p->d_pweights + (size_t)p->g.width * p->g.height * first : nullptr;
     FwdScanRec r;
     std::memset(&r, 0, sizeof(r));
-    r.map_v = make_map(CBCT_F32, j.vol, p->g.nx, p->g.ny, p->g.nz, b);
-    r.map_t = make_map(CBCT_F32, volT ? (const void*)volT : (const void*)j.vol, volT ? p->g.ny : p->g.nx,
+    r.map_v = make_volume_map(CBCT_F32, j.vol, p->g.nx, p->g.ny, p->g.nz, b);
+    r.map_t = make_volume_map(CBCT_F32, volT ? (const void*)volT : (const void*)j.vol, volT ? p->g.ny : p->g.nx,
                        volT ? p->g.nx : p->g.ny, p->g.nz, b);
     r.vol = j.vol;
     r.views = p->d_views + first;
@@ -2098,14 +1622,13 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
       after.push_back([part, nblocks, out](cudaStream_t st) { finalize_partials(part, nblocks, out, st); });
     }
     r.o = o;
-    if ((int)groups[var][w].size() == kMultiMaxRecs) flush(var, w);
-    r.base = totals[var][w];
-    totals[var][w] += nblocks;
-    smem[var][w] = std::max(smem[var][w], sm);
-    groups[var][w].push_back(r);
+    if ((int)g.recs.size() == kMultiMaxRecs) flush(g);
+    r.base = g.total;
+    g.total += nblocks;
+    g.smem = std::max(g.smem, sm);
+    g.recs.push_back(r);
   }
-  for (int v = 0; v < 4; ++v)
-    for (int c = 0; c < 5; ++c) flush(v, c);
+  for (FwdGroup& g : groups) flush(g);
   flush_transposes();
   for (auto& f : after) A.ops.push_back(std::move(f));
 }

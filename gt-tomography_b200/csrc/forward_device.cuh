@@ -9,8 +9,6 @@
 
 namespace cbct {
 
-namespace {
-
 enum { kModeStore = 0, kModeResidual = 1, kModeRecip = 2 };
 
 struct FwdOut {
@@ -26,6 +24,14 @@ struct FwdOut {
   const float* wproj;    // projection weights of the subset (CBSubsetWeightOperator; nullable)
 };
 
+// Tile of one CTA: detector tile (x, y) of view z of the call, and its index
+// among the call's tiles in launch order (its partial-sum slot).
+struct TileId {
+  int x, y, z;
+  size_t bid;
+};
+
+namespace {
 
 // Sample range of a ray restricted to the box grown by half a voxel: samples
 // outside it touch only border texels and add exactly 0.  Returns false when
@@ -131,13 +137,6 @@ __device__ __forceinline__ double fwd_store(const FwdOut& o, const GridConst& gc
 __device__ __forceinline__ size_t launch_block_id() {
   return ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
 }
-
-// Tile of one CTA: detector tile (x, y) of view z of the call, and its index
-// among the call's tiles in launch order (its partial-sum slot).
-struct TileId {
-  int x, y, z;
-  size_t bid;
-};
 
 __device__ __forceinline__ TileId launch_tile() {
   return TileId{int(blockIdx.x), int(blockIdx.y), int(blockIdx.z), launch_block_id()};

@@ -1,0 +1,46 @@
+// forward_host.h -- host-side declarations shared by the forward projector's
+// translation units.
+#pragma once
+
+#include "forward_device.cuh"
+
+namespace cbct {
+
+// A scan's entry in a work-list launch over many scans: the arguments of its
+// one-scan launch and where its tiles start in the list.
+struct alignas(128) FwdScanRec {
+  CUtensorMap map_v, map_t;    // volume and x/y-transposed volume, the plan's box
+  const void* vol;
+  const ViewParams* views;     // the subset's views
+  int* flags;
+  GridConst gc;
+  FwdOut o;
+  int BZ, nsl_max;
+  int tx, ty;                  // ray tiles per view (x, y)
+  int base;                    // work-list index of the scan's first tile
+};
+
+// Tensor map of a volume (n0, n1, n2) with box b.
+CUtensorMap make_volume_map(cbct_dtype dt, const void* vol, int n0, int n1, int n2, const SlabBox& b);
+
+// Largest footprint of a slab of TS voxels over every view and tile of a TU x TV
+// tiling, margins included; false when some view cannot use slabs.
+bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& ext_z);
+
+// Row-quad projector (forward_quad.cu).
+enum QuadShape { kQuadWide = 0, kQuadWarp = 1, kQuadThin = 2, kQuadShapes = 3 };
+void quad_tile(int shape, int& TU, int& TV);
+bool quad_choose(cbct_plan* p, double row_dz, bool forced);
+void quad_prepare(const cbct_plan* p);
+void quad_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volT, const FwdOut& o, int first, int cnt,
+                 cudaStream_t st);
+
+using FwdMultiKernel = void (*)(const FwdScanRec*, int, int, int*);
+struct QuadMulti {
+  FwdMultiKernel kernel;       // work-list kernel of the plan's shape and box width
+  int nsl, threads;
+  size_t smem;
+};
+QuadMulti quad_multi(const cbct_plan* p);
+
+}  // namespace cbct

@@ -155,14 +155,14 @@ CBCT_API cbct_status cbct_plan_autotune(cbct_plan* plan, float* times_ms_out, vo
 #define CBCT_OPT_DEBUG_CHECKS 1
 #define CBCT_OPT_FORCE_GATHER 2
 /* CBCT_OPT_FORWARD_KERNEL: 0 = automatic (the row-quad kernel where adjacent
- * detector rows stay within 0.66 z texel of each other, else the row-pair
- * kernel where they stay within one texel, else the per-ray slab kernel, each
- * where its boxes fit, else gather), 1 = slab, 2 = gather, 3 = the column-fan
- * kernel (e/d interpolation shared by the rays of a detector column; slower on
- * B200 at the sizes measured so far), 4 = the row-pair kernel (one thread
- * marches two vertically adjacent rays of a column and shares their in-plane
- * interpolation), 5 = the row-quad kernel (four rows per thread).  Slab, fan,
- * row-pair and row-quad results are bitwise equal. */
+ * detector rows stay within 0.66 z texel of each other, and up to 1.4 texels in
+ * launches with enough rays; else the row-pair kernel where rows stay within one
+ * texel, else the per-ray slab kernel, each where its boxes fit, else gather),
+ * 1 = slab, 2 = gather, 3 = the column-fan kernel (e/d interpolation shared by the
+ * rays of a detector column; slower on B200 at the sizes measured so far), 4 = the
+ * row-pair kernel (one thread marches two vertically adjacent rays of a column and
+ * shares their in-plane interpolation), 5 = the row-quad kernel (four rows per
+ * thread).  Slab, fan, row-pair and row-quad results are bitwise equal. */
 #define CBCT_OPT_FORWARD_KERNEL 3
 /* CBCT_OPT_WAIT_LIMIT: polls (>= 0) a TMA-staged projector kernel spends
  * waiting for its next shared-memory stage before it gives up (default

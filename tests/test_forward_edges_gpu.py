@@ -6,9 +6,13 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# World coordinates near the source distance (1000 mm) round to 6e-5 mm, 1e-5 of
-# a 6 mm voxel, against border weights of 0.25 on average: some 4e-5 relative.
+# Whole projections against the FP64 oracle: the FP32 path's bound.  A silhouette
+# ray alone is ill-conditioned in FP32 whatever kernel samples it (its coordinates
+# round at the source distance), so those rays are held to the gather kernel, which
+# samples every ray by itself at the same FP32 coordinates: the two sums of up to
+# 320 terms differ in order only, N 2^-24 = 2e-5 at most.
 TOL = 1e-4
+TOL_ORDER = 2e-5
 
 
 def _misses(W, H, pitch, L, angles, SAD=1000.0, SDD=1500.0):
@@ -29,7 +33,7 @@ def _misses(W, H, pitch, L, angles, SAD=1000.0, SDD=1500.0):
     return np.stack(out)
 
 
-@pytest.mark.parametrize("kernel", [0, 1, 2, 3, 4, 5])
+@pytest.mark.parametrize("kernel", [0, 1, 3, 4, 5])
 @pytest.mark.parametrize("n,vox", [((12, 8, 6), 6.0), ((40, 36, 3), 1.5)])
 def test_silhouette_rays(gtb, O, cuda, kernel, n, vox):
     import torch
@@ -43,12 +47,16 @@ def test_silhouette_rays(gtb, O, cuda, kernel, n, vox):
     ref = O.forward(og, vol.astype(np.float64), angles, offsets, spp=8.0)
     sel = _misses(W, H, pitch, L, angles) & (ref > 0)
     assert sel.sum() > 100
-    plan = gtb.Plan(cg, angles, offsets)
-    plan.set_option(gtb._lib.CBCT_OPT_FORWARD_KERNEL, kernel)
-    plan.set_option(gtb._lib.CBCT_OPT_DEBUG_CHECKS, 1)
-    out = torch.full(plan.proj_shape(), -1.0, dtype=torch.float32, device=cuda)
-    plan.forward(torch.from_numpy(vol).to(cuda), out)
-    assert plan.read_flags() == (0, 0)
-    got = out.cpu().numpy().astype(np.float64)
-    assert np.linalg.norm(got[sel] - ref[sel]) <= TOL * np.linalg.norm(ref[sel]), plan.forward_variant()
+    v = torch.from_numpy(vol).to(cuda)
+    outs = []
+    for k in (kernel, 2):
+        plan = gtb.Plan(cg, angles, offsets)
+        plan.set_option(gtb._lib.CBCT_OPT_FORWARD_KERNEL, k)
+        plan.set_option(gtb._lib.CBCT_OPT_DEBUG_CHECKS, 1)
+        out = torch.full(plan.proj_shape(), -1.0, dtype=torch.float32, device=cuda)
+        plan.forward(v, out)
+        assert plan.read_flags() == (0, 0)
+        outs.append(out.cpu().numpy().astype(np.float64))
+    got, gather = outs
+    assert np.linalg.norm(got[sel] - gather[sel]) <= TOL_ORDER * np.linalg.norm(gather[sel])
     assert np.linalg.norm(got - ref) <= TOL * np.linalg.norm(ref)
