@@ -218,11 +218,14 @@ struct cbct_plan {
   cbct::SlabBox slab16{};   // box for 16-bit storage (x starts aligned to 8)
   size_t slab_smem = 0;     // dynamic shared memory of the fp32 slab kernel (bytes)
   std::vector<int> subset_has_xdom;  // per subset (and all-views entry): any x-dominant view
-  void* d_volT = nullptr;   // x/y-transposed volume for x-dominant views (fp32 capacity)
+  void* d_volT = nullptr;   // x/y-transposed volume for x-dominant views (volT_bytes)
+  void* d_volP = nullptr;   // row-padded volume where nx is not a multiple of 4 (volP_bytes)
   int bp_variant = 0;       // 0 = global loads, 1 = TMA-staged detector boxes
   int bp_pref = 0;          // 0: TMA-staged where it fits, 1: global loads (autotuner)
   cbct::SlabBox bp_box{};   // detector box (bx = u width, by = v rows)
   int bp_max_views = 0;     // views per launch the TMA back-projector holds
+  float* d_bp_pad = nullptr;  // row-padded projections where W is not a multiple of 4 (bp_pad_bytes)
+  int bp_pad_views = 0;     // views it holds
 
   // scratch owned by the plan (allocated at creation or first use, reused)
   float* d_proj_scratch = nullptr;  // weighted copies of projections (mult_MH with offset weight)
@@ -292,6 +295,33 @@ T* plan_alloc_n(cbct_plan* p, size_t n) {
 // and device (no-op when already high enough, so it is safe to call before
 // launches that may be captured).
 void ensure_smem_attr(const void* func, size_t bytes);
+
+// Row pitch (elements) of a TMA-readable copy: rows of a multiple of 16 bytes.
+inline int tma_pitch(int n, size_t es) {
+  const int q = int(16 / es);
+  return (n + q - 1) / q * q;
+}
+// Bytes of the forward projector's volume copies: the transposed one (fp32, or a
+// 16-bit one with a row-padded 16-bit copy behind it) and the row-padded one of
+// fp32 volumes whose nx is not a multiple of 4 (0: none).
+inline size_t volT16_bytes(const cbct_geometry& g) {
+  return ((size_t)g.nx * tma_pitch(g.ny, 2) * g.nz * 2 + 255) & ~size_t(255);
+}
+inline size_t volT_bytes(const cbct_geometry& g) {
+  const size_t b32 = (size_t)g.nx * tma_pitch(g.ny, 4) * g.nz * 4;
+  const size_t b16 = volT16_bytes(g) + (g.nx % 8 && g.nx % 4 == 0 ? (size_t)tma_pitch(g.nx, 2) * g.ny * g.nz * 2 : 0);
+  return std::max(b32, b16);
+}
+inline size_t volP_bytes(const cbct_geometry& g) {
+  return g.nx % 4 ? (size_t)tma_pitch(g.nx, 4) * g.ny * g.nz * 4 : 0;
+}
+
+// Views of the back-projector's row-padded projections (at most the largest
+// subset's), and their bytes: only detectors whose rows TMA cannot read need them.
+constexpr int kBpPadViews = 128;
+inline size_t bp_pad_bytes(const cbct_geometry& g, int max_subset) {
+  return g.width % 4 ? (size_t)tma_pitch(g.width, 4) * g.height * std::min(max_subset, kBpPadViews) * 4 : 0;
+}
 
 // forward.cu
 void forward_prepare(cbct_plan* p);

@@ -59,29 +59,37 @@ __global__ void __launch_bounds__(256) fwd_gather_kernel(const V* __restrict__ v
 }
 
 // ------------------------------------------------------------------ transpose
-// volT[k][i][j] = vol[k][j][i]: the volume seen with x and y exchanged.
+// volT[k][i][j] = vol[k][j][i]: the volume seen with x and y exchanged, rows
+// pitchT elements apart.  With volP, also a copy of the volume whose rows are
+// pitchP apart (TMA needs rows of a multiple of 16 bytes).
 template <class V>
-__device__ __forceinline__ void transpose_tile(const V* __restrict__ in, V* __restrict__ out, int nx, int ny, int bx,
-                                               int by, int bz, V (&tile)[32][33]) {
-  const size_t plane = (size_t)nx * ny;
-  const V* src = in + bz * plane;
-  V* dst = out + bz * plane;
+__device__ __forceinline__ void transpose_tile(const V* __restrict__ in, V* __restrict__ volT, int pitchT,
+                                               V* __restrict__ volP, int pitchP, int nx, int ny, int bx, int by,
+                                               int bz, V (&tile)[32][33]) {
+  const V* src = in + bz * ((size_t)nx * ny);
   const int x0 = bx * 32, y0 = by * 32;
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
     const int x = x0 + threadIdx.x, y = y0 + j;
-    if (x < nx && y < ny) tile[j][threadIdx.x] = src[(size_t)y * nx + x];
+    if (x < nx && y < ny) {
+      const V v = src[(size_t)y * nx + x];
+      tile[j][threadIdx.x] = v;
+      if (volP) volP[((size_t)bz * ny + y) * pitchP + x] = v;
+    }
   }
+  if (!volT) return;
   __syncthreads();
+  V* dst = volT + bz * ((size_t)nx * pitchT);
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
     const int y = y0 + threadIdx.x, x = x0 + j;
-    if (x < nx && y < ny) dst[(size_t)x * ny + y] = tile[threadIdx.x][j];
+    if (x < nx && y < ny) dst[(size_t)x * pitchT + y] = tile[threadIdx.x][j];
   }
 }
 
 template <class V>
-__global__ void transpose_xy_kernel(const V* __restrict__ in, V* __restrict__ out, int nx, int ny) {
+__global__ void volume_copies_kernel(const V* __restrict__ in, V* __restrict__ volT, int pitchT,
+                                     V* __restrict__ volP, int pitchP, int nx, int ny) {
   __shared__ V tile[32][33];
-  transpose_tile<V>(in, out, nx, ny, blockIdx.x, blockIdx.y, blockIdx.z, tile);
+  transpose_tile<V>(in, volT, pitchT, volP, pitchP, nx, ny, blockIdx.x, blockIdx.y, blockIdx.z, tile);
 }
 
 // x/y transposes of many scans' volumes in one launch: one CTA per 32x32 tile
@@ -107,7 +115,7 @@ __global__ void transpose_multi_kernel(const TransposeRec* __restrict__ recs, in
   int l = t - R.base;
   const int bx = l % R.tx;
   l /= R.tx;
-  transpose_tile<float>(R.in, R.out, R.nx, R.ny, bx, l % R.ty, l / R.ty, tile);
+  transpose_tile<float>(R.in, R.out, R.ny, nullptr, 0, R.nx, R.ny, bx, l % R.ty, l / R.ty, tile);
 }
 
 // ------------------------------------------------------------------ slab/TMA
@@ -1007,7 +1015,8 @@ CUtensorMap make_volume_map(cbct_dtype dt, const void* vol, int n0, int n1, int 
   std::memset(&m, 0, sizeof(m));
   const size_t es = dtype_size(dt);
   cuuint64_t dims[3] = {(cuuint64_t)n0, (cuuint64_t)n1, (cuuint64_t)n2};
-  cuuint64_t strides[2] = {(cuuint64_t)n0 * es, (cuuint64_t)n0 * n1 * es};
+  const cuuint64_t pitch = (cuuint64_t)tma_pitch(n0, es) * es;
+  cuuint64_t strides[2] = {pitch, pitch * n1};
   cuuint32_t box[3] = {(cuuint32_t)b.bx, (cuuint32_t)b.by, (cuuint32_t)b.bz};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult res = tensor_map_encoder()(&m, tma_dtype(dt), 3, const_cast<void*>(vol), dims, strides, box, estr,
@@ -1055,12 +1064,11 @@ int slab_stages(const SlabBox& b, size_t& smem) {
 }
 
 template <class V, int BX>
-void launch_slab(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, dim3 grid, int first,
+void launch_slab(cbct_plan* p, const V* vol, const V* volP, const V* volT, const FwdOut& o, dim3 grid, int first,
                  cudaStream_t st, cbct_dtype dt) {
   const SlabBox& b = box_for<V>(p);
-  const CUtensorMap mv = make_volume_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = make_volume_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
-                                  volT ? p->g.nx : p->g.ny, p->g.nz, b);
+  const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
+  const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
   size_t smem = 0;
   const bool two = slab_stages<V>(b, smem) == 2;
   auto pick = [&](auto k2, auto k1) { return two ? k2 : k1; };
@@ -1075,12 +1083,11 @@ template <class V>
 const SlabBox& pair_box_for(const cbct_plan* p) { return sizeof(V) == 4 ? p->pair : p->pair16; }
 
 template <class V, int BX>
-void launch_pair(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
+void launch_pair(cbct_plan* p, const V* vol, const V* volP, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
                  cbct_dtype dt) {
   const SlabBox& b = pair_box_for<V>(p);
-  const CUtensorMap mv = make_volume_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = make_volume_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
-                                  volT ? p->g.nx : p->g.ny, p->g.nz, b);
+  const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
+  const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
   const int nsl = slabs_max(p->g);
   const size_t smem = pair_smem(b, sizeof(V), nsl);
   const dim3 grid((p->g.width + kPU - 1) / kPU, (p->g.height + kPV - 1) / kPV, cnt);
@@ -1100,12 +1107,11 @@ template <class V>
 const SlabBox& fan_box_for(const cbct_plan* p) { return sizeof(V) == 4 ? p->fan : p->fan16; }
 
 template <class V, int BX>
-void launch_fan(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
+void launch_fan(cbct_plan* p, const V* vol, const V* volP, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
                 cbct_dtype dt) {
   const SlabBox& b = fan_box_for<V>(p);
-  const CUtensorMap mv = make_volume_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = make_volume_map(dt, volT ? (const void*)volT : (const void*)vol, volT ? p->g.ny : p->g.nx,
-                                  volT ? p->g.nx : p->g.ny, p->g.nz, b);
+  const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
+  const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
   const int nsl = slabs_max(p->g);
   const size_t smem = forward_smem(b, sizeof(V), p->fan_lz, nsl);
   const dim3 grid((p->g.width + kFU - 1) / kFU, (p->g.height + kFV - 1) / kFV, cnt);
@@ -1121,6 +1127,22 @@ void launch_fan(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int 
   check_launch("fwd_fan_kernel");
 }
 
+// A volume TMA cannot read in place: rows or start off a 16-byte boundary.  The
+// TMA kernels then read a row-padded copy, made with the transposed one in one pass
+// (8 to 12 bytes per voxel, HBM-bound): 40 views of 301x211 from 150x141x93 voxels
+// take 0.97 ms, the gather kernel's bounds-checked global loads 2.36 ms.
+bool needs_padded_rows(const void* vol, int nx, size_t es) {
+  return (nx * es) % 16 != 0 || reinterpret_cast<uintptr_t>(vol) % 16 != 0;
+}
+
+// Plan buffer for a row-padded copy of a volume of element size es, or NULL.
+// 16-bit volumes keep theirs behind the transposed copy (d_volT has fp32 room).
+void* padded_rows(cbct_plan* p, size_t es) {
+  if (p->g.nx % 4 != 0) return p->d_volP;
+  if (es == 2 && p->g.nx % 8 != 0 && p->d_volT) return static_cast<char*>(p->d_volT) + volT16_bytes(p->g);
+  return nullptr;
+}
+
 template <class V>
 void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaStream_t st, cbct_dtype dt,
                   bool use_slab) {
@@ -1132,45 +1154,48 @@ void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaS
     check_launch("fwd_gather_kernel");
     return;
   }
-  const V* volT = nullptr;
-  if (p->subset_has_xdom[s]) {
-    V* t = static_cast<V*>(p->d_volT);
+  // Copies the TMA boxes come from: the x/y-transposed volume for x-dominant
+  // views, and a row-padded one where the caller's rows are not TMA-aligned.
+  const int pitchT = tma_pitch(p->g.ny, sizeof(V)), pitchP = tma_pitch(p->g.nx, sizeof(V));
+  V* const volT = p->subset_has_xdom[s] ? static_cast<V*>(p->d_volT) : nullptr;
+  V* const pad = needs_padded_rows(vol, p->g.nx, sizeof(V)) ? static_cast<V*>(padded_rows(p, sizeof(V))) : nullptr;
+  if (volT || pad) {
     dim3 tg((p->g.nx + 31) / 32, (p->g.ny + 31) / 32, p->g.nz);
-    transpose_xy_kernel<V><<<tg, dim3(32, 8), 0, st>>>(vol, t, p->g.nx, p->g.ny);
-    check_launch("transpose_xy_kernel");
-    volT = t;
+    volume_copies_kernel<V><<<tg, dim3(32, 8), 0, st>>>(vol, volT, pitchT, pad, pitchP, p->g.nx, p->g.ny);
+    check_launch("volume_copies_kernel");
   }
+  const V* const volP = pad ? pad : vol;
   if (p->fwd_variant == 4) {
-    quad_launch(p, dt, vol, volT, o, first, cnt, st);
+    quad_launch(p, dt, vol, volP, volT, o, first, cnt, st);
     return;
   }
   if (p->fwd_variant == 3) {
     switch (pair_box_for<V>(p).bx) {
-      case 40: launch_pair<V, 40>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 56: launch_pair<V, 56>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 72: launch_pair<V, 72>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 104: launch_pair<V, 104>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 136: launch_pair<V, 136>(p, vol, volT, o, first, cnt, st, dt); break;
+      case 40: launch_pair<V, 40>(p, vol, volP, volT, o, first, cnt, st, dt); break;
+      case 56: launch_pair<V, 56>(p, vol, volP, volT, o, first, cnt, st, dt); break;
+      case 72: launch_pair<V, 72>(p, vol, volP, volT, o, first, cnt, st, dt); break;
+      case 104: launch_pair<V, 104>(p, vol, volP, volT, o, first, cnt, st, dt); break;
+      case 136: launch_pair<V, 136>(p, vol, volP, volT, o, first, cnt, st, dt); break;
       default: throw Error(CBCT_ERR_INTERNAL, "unsupported pair box width");
     }
     return;
   }
   if (p->fwd_variant == 2) {
     switch (fan_box_for<V>(p).bx) {
-      case 24: launch_fan<V, 24>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 40: launch_fan<V, 40>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 56: launch_fan<V, 56>(p, vol, volT, o, first, cnt, st, dt); break;
-      case 72: launch_fan<V, 72>(p, vol, volT, o, first, cnt, st, dt); break;
+      case 24: launch_fan<V, 24>(p, vol, volP, volT, o, first, cnt, st, dt); break;
+      case 40: launch_fan<V, 40>(p, vol, volP, volT, o, first, cnt, st, dt); break;
+      case 56: launch_fan<V, 56>(p, vol, volP, volT, o, first, cnt, st, dt); break;
+      case 72: launch_fan<V, 72>(p, vol, volP, volT, o, first, cnt, st, dt); break;
       default: throw Error(CBCT_ERR_INTERNAL, "unsupported fan box width");
     }
     return;
   }
   switch (box_for<V>(p).bx) {
-    case 40: launch_slab<V, 40>(p, vol, volT, o, grid, first, st, dt); break;
-    case 56: launch_slab<V, 56>(p, vol, volT, o, grid, first, st, dt); break;
-    case 72: launch_slab<V, 72>(p, vol, volT, o, grid, first, st, dt); break;
-    case 104: launch_slab<V, 104>(p, vol, volT, o, grid, first, st, dt); break;
-    case 136: launch_slab<V, 136>(p, vol, volT, o, grid, first, st, dt); break;
+    case 40: launch_slab<V, 40>(p, vol, volP, volT, o, grid, first, st, dt); break;
+    case 56: launch_slab<V, 56>(p, vol, volP, volT, o, grid, first, st, dt); break;
+    case 72: launch_slab<V, 72>(p, vol, volP, volT, o, grid, first, st, dt); break;
+    case 104: launch_slab<V, 104>(p, vol, volP, volT, o, grid, first, st, dt); break;
+    case 136: launch_slab<V, 136>(p, vol, volP, volT, o, grid, first, st, dt); break;
     default: throw Error(CBCT_ERR_INTERNAL, "unsupported slab box width");
   }
 }
@@ -1415,8 +1440,8 @@ void forward_prepare(cbct_plan* p) {
   if (p->fwd_variant == 4) quad_prepare(p);
   bool any_x = false;
   for (size_t s = 0; s < p->subset_has_xdom.size(); ++s) any_x = any_x || p->subset_has_xdom[s];
-  if (any_x && !p->d_volT)
-    p->d_volT = plan_alloc_n<float>(p, (size_t)p->g.nx * p->g.ny * p->g.nz);
+  if (any_x && !p->d_volT) p->d_volT = plan_alloc(p, volT_bytes(p->g));
+  if (volP_bytes(p->g) && !p->d_volP) p->d_volP = plan_alloc(p, volP_bytes(p->g));
 }
 
 void forward_launch(cbct_plan* p, int s, cbct_dtype dt, const void* vol, float* out, const float* b,
@@ -1442,8 +1467,8 @@ void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, floa
   if (cnt == 0) return;
   o.wproj = p->d_pweights ? p->d_pweights + (size_t)p->g.width * p->g.height * p->first[s] : nullptr;
   const size_t es = dtype_size(dt);
-  const bool use_slab = p->fwd_variant >= 1 && ((size_t)p->g.nx * es) % 16 == 0 &&
-                        ((size_t)p->g.ny * es) % 16 == 0 && (reinterpret_cast<uintptr_t>(vol) % 16 == 0) &&
+  const bool use_slab = p->fwd_variant >= 1 &&
+                        (!needs_padded_rows(vol, p->g.nx, es) || padded_rows(p, es) != nullptr) &&
                         (!p->subset_has_xdom[s] || p->d_volT != nullptr);
   // One partial sum per block of the kernel that will run.
   const bool fan = use_slab && p->fwd_variant == 2, pair = use_slab && p->fwd_variant == 3;

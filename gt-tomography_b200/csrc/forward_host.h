@@ -32,8 +32,9 @@ enum QuadShape { kQuadWide = 0, kQuadWarp = 1, kQuadThin = 2, kQuadShapes = 3 };
 void quad_tile(int shape, int& TU, int& TV);
 bool quad_choose(cbct_plan* p, double row_dz, bool forced);
 void quad_prepare(const cbct_plan* p);
-void quad_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volT, const FwdOut& o, int first, int cnt,
-                 cudaStream_t st);
+// vol: the caller's volume; volP: the copy TMA reads it from (or vol itself).
+void quad_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volP, const void* volT, const FwdOut& o,
+                 int first, int cnt, cudaStream_t st);
 
 using FwdMultiKernel = void (*)(const FwdScanRec*, int, int, int*);
 struct QuadMulti {

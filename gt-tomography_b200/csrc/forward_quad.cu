@@ -82,10 +82,10 @@ void prepare_typed(const cbct_plan* p) {
 }
 
 template <class V>
-void launch_typed(cbct_plan* p, const V* vol, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
+void launch_typed(cbct_plan* p, const V* vol, const V* volP, const V* volT, const FwdOut& o, int first, int cnt, cudaStream_t st,
                   cbct_dtype dt) {
   const SlabBox& b = sizeof(V) == 4 ? p->quad : p->quad16;
-  const CUtensorMap mv = make_volume_map(dt, vol, p->g.nx, p->g.ny, p->g.nz, b);
+  const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
   const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
   const QuadDims& d = kDims[p->quad_shape];
   const int nsl = quad_slabs(p->g, d.TS);
@@ -199,19 +199,16 @@ void quad_prepare(const cbct_plan* p) {
   prepare_typed<__nv_bfloat16>(p);
 }
 
-void quad_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volT, const FwdOut& o, int first, int cnt,
-                 cudaStream_t st) {
-  switch (dt) {
-    case CBCT_F32:
-      launch_typed<float>(p, static_cast<const float*>(vol), static_cast<const float*>(volT), o, first, cnt, st, dt);
-      break;
-    case CBCT_F16:
-      launch_typed<__half>(p, static_cast<const __half*>(vol), static_cast<const __half*>(volT), o, first, cnt, st, dt);
-      break;
-    default:
-      launch_typed<__nv_bfloat16>(p, static_cast<const __nv_bfloat16*>(vol), static_cast<const __nv_bfloat16*>(volT), o,
-                                  first, cnt, st, dt);
-  }
+void quad_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volP, const void* volT, const FwdOut& o,
+                 int first, int cnt, cudaStream_t st) {
+  auto go = [&](auto v) {
+    using V = decltype(v);
+    launch_typed<V>(p, static_cast<const V*>(vol), static_cast<const V*>(volP), static_cast<const V*>(volT), o, first,
+                    cnt, st, dt);
+  };
+  if (dt == CBCT_F32) go(float{});
+  else if (dt == CBCT_F16) go(__half{});
+  else go(__nv_bfloat16{});
 }
 
 QuadMulti quad_multi(const cbct_plan* p) {

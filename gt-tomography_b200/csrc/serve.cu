@@ -80,6 +80,8 @@ size_t request_bytes(const cbct_request& r) {
   add(sizeof(int) * 4);
   add(pl * P * dtype_size(r.storage));  // projections
   add(nv * sizeof(float));              // volume
+  const int sub = r.kind == CBCT_REQ_FDK ? r.n_views : (r.n_views + r.n_subsets - 1) / r.n_subsets;
+  if (bp_pad_bytes(g, sub)) add(bp_pad_bytes(g, sub));  // row-padded projections of the back-projector
   if (r.kind == CBCT_REQ_FDK) {
     size_t L = 2;
     while (L < 2 * (size_t)g.width - 1) L <<= 1;
@@ -90,7 +92,8 @@ size_t request_bytes(const cbct_request& r) {
     add(sizeof(float) * g.width * P);
     if (r.storage != CBCT_F32) add(sizeof(float) * pl * P);  // FP32 filtered copy
   } else {
-    add(nv * sizeof(float));  // transposed volume of the forward projector (upper bound)
+    add(volT_bytes(g));       // volume copies of the forward projector (upper bound)
+    if (volP_bytes(g)) add(volP_bytes(g));
     add((2 * nv + pl * P) * sizeof(float));  // solver workspace (FP32 volume input)
   }
   return b + n * kAllocSlack;

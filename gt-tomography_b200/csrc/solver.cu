@@ -176,7 +176,7 @@ void osmom_update_launch(float* z, float* xold, const float* precon, const float
   check_launch("osmom_update_kernel");
 }
 
-static void recip_launch(float* x, size_t n, cudaStream_t st) {
+void recip_launch(float* x, size_t n, cudaStream_t st) {
   if (n == 0) return;
   recip_kernel<<<ew_blocks(n), 256, 0, st>>>(x, n);
   check_launch("recip_kernel");
