@@ -96,18 +96,11 @@ __device__ __forceinline__ void bp_store(const BpEpi& e, size_t idx, float g) {
   bp_finish<EPI>(e, idx, g, bp_load<EPI>(e, idx));
 }
 
-// 1: the view loop of the TMA back-projector passes one barrier per view (the
-// wait check rides on the barrier that frees the stage); 0 (shipped): two,
-// the wait checked before the stage is read (measured the same: 0.514 vs
-// 0.516 ms per C2 subset, 814.5 vs 815.0 GUPS for the solve).
-#ifndef CBCT_BP_ONE_BARRIER
-#define CBCT_BP_ONE_BARRIER 0
-#endif
-
-// Voxels of a thread's z-run whose epilogue operands are loaded together.
-#ifndef CBCT_BP_EPI_CHUNK
-#define CBCT_BP_EPI_CHUNK 4
-#endif
+// Voxels of a thread's z-run whose epilogue operands are loaded together.  Besides
+// the loads in flight, this sets the registers the compiler gives the kernel: at 8 the
+// view loop keeps its register pairs in place (96 registers for runs of 32; FDK of
+// 256^3 from 360 views of 512x384: 4.67 ms, at 4 with 72 registers 4.90).
+constexpr int kEpiChunk = 8;
 
 template <int EPI, bool FDK>
 __global__ void __launch_bounds__(kBX * kBY) bp_kernel(const float* __restrict__ proj,
@@ -185,16 +178,26 @@ __global__ void __launch_bounds__(kBX * kBY) bp_kernel(const float* __restrict__
 }
 
 // ------------------------------------------------------------------ TMA-staged
-// A CTA owns a kTX x kTY x kZT voxel block; each warp holds an 8 x 4 patch of
+// A CTA owns a kTX x kTY x ZT voxel block; each warp holds an 8 x 4 patch of
 // columns so that its lanes read a narrow range of detector words.  For each view the block's footprint
 // on the detector (the bounding box of its eight projected corners, a convex
 // image of a convex block) is staged into shared memory by a 3-D TMA load
 // whose out-of-detector texels arrive as zeros, so the bilinear taps need no
 // bounds checks.  Views are pipelined over two stages.
-#ifndef CBCT_BP_ZRUN
-#define CBCT_BP_ZRUN 16
-#endif
-constexpr int kZT = CBCT_BP_ZRUN;
+// What bounds it: shared-memory wavefronts (four loads per voxel and view) and the
+// FMA pipe together.  The loop has no index clamp (a run's ends are checked per
+// view), takes the byte address of a tap from one multiply-add on the bits of its
+// biased row, and packs pairs of voxels.  36 views of 512x384 into 256^3, the kernel
+// alone: 517 us with clamps, runs of 16 and boxes 56 wide; 447 us now (1.35e12
+// voxel-views/s).
+// Runs of 32 voxels along z halve the per-view geometry, barriers and staging per
+// voxel against runs of 16 (FDK of 256^3 from 360 views: 4.65 against 5.14 ms); runs
+// of 16 keep more CTAs where the volume is small.
+constexpr int kZRuns[] = {16, 32};
+// Least CTAs of a launch with long runs, four per SM: 20 views into 128^3 (512 CTAs)
+// take 45.1 us with them and 43.1 without, 25 views into 160x144x128 (720) 65.6
+// and 67.6, 20 views into 64^3 (64) 22.5 and 16.4.
+constexpr int kLongRunCtas = 592;
 constexpr int kTX = 16, kTY = 8;     // columns per CTA of the TMA back-projector
 
 struct BpView {
@@ -203,35 +206,36 @@ struct BpView {
 
 // Detector box widths (u, fp32 elements) the TMA back-projector is compiled
 // for; a plan takes the smallest that holds its footprints.  Rows of a box
-// sit BU floats apart, so BU mod 32 is the bank offset between the two rows a
-// bilinear tap reads.
-#ifdef CBCT_BP_WIDTHS_16
-constexpr int kBpWidths[] = {48, 80, 112, 144};      // row offset 16 banks
-#else
-constexpr int kBpWidths[] = {40, 56, 72, 104, 136};  // row offset 8 or 24 banks
-#endif
+// sit BU floats apart, so BU mod 32 is the bank offset between the rows that a
+// warp's 8 x 4 columns read: up to about 23 detector pixels in one to four rows
+// where pixels are finer than voxels.  16 banks apart (48) they collide least, 1.09
+// wavefronts per load at 1.9 pixels per voxel against 1.37 at 8 or 24 (40, 56); with
+// about one pixel per voxel (footprints up to kBpNarrow) no width conflicts.
+constexpr int kBpWidths[] = {40, 48, 56, 72, 104, 136};
+constexpr int kBpNarrow = 32;
 constexpr int kNBpWidths = int(sizeof(kBpWidths) / sizeof(int));
 
-// Calls f(std::integral_constant<int, W>) for the compiled width W == w;
-// false when w is not one of them.
+// Calls f(std::integral_constant<int, W>, std::integral_constant<int, Z>) for the
+// compiled width W == w and run Z == zrun; false when there is none.
 template <int I = 0, class F>
-bool with_bp_width(int w, F&& f) {
+bool with_bp(int w, int zrun, F&& f) {
   if constexpr (I < kNBpWidths) {
     if (w == kBpWidths[I]) {
-      f(std::integral_constant<int, kBpWidths[I]>{});
+      if (zrun == kZRuns[0]) f(std::integral_constant<int, kBpWidths[I]>{}, std::integral_constant<int, kZRuns[0]>{});
+      else f(std::integral_constant<int, kBpWidths[I]>{}, std::integral_constant<int, kZRuns[1]>{});
       return true;
     }
-    return with_bp_width<I + 1>(w, std::forward<F>(f));
+    return with_bp<I + 1>(w, zrun, std::forward<F>(f));
   } else {
     return false;
   }
 }
 
-// One CTA's work: the kTX x kTY x kZT voxel block (bi, bj, bk) over the views
+// One CTA's work: the kTX x kTY x ZT voxel block (bi, bj, bk) over the views
 // of the call.  Shared by the one-scan kernel (block = blockIdx) and the
 // work-list kernel over many scans (block = the item's); base_ptr is the
 // 128-byte aligned dynamic shared memory, bars/abort_flag the CTA's statics.
-template <int EPI, bool FDK, int BU>
+template <int EPI, bool FDK, int BU, int ZT>
 __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewParams* __restrict__ views,
                                             int n_views, const GridConst& gc, const BpEpi& e, int BV, int* flags,
                                             int bi, int bj, int bk, unsigned char* base_ptr, uint64_t* bars,
@@ -243,7 +247,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   int2* ext = org + n_views;                             // per view: (max u, max v) for checks
   const int tid = threadIdx.x;
   const int nthr = kTX * kTY;
-  const int i0 = bi * kTX, j0 = bj * kTY, k0 = bk * kZT;
+  const int i0 = bi * kTX, j0 = bj * kTY, k0 = bk * ZT;
 
   for (int q = tid; q < n_views; q += nthr) {
     const ViewParams& vp = views[q];
@@ -259,7 +263,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   }
   __syncthreads();
   // Footprints: 8 corners of the block (voxel centres) per view.
-  const int ie = min(i0 + kTX, gc.nx) - 1, je = min(j0 + kTY, gc.ny) - 1, ke = min(k0 + kZT, gc.nz) - 1;
+  const int ie = min(i0 + kTX, gc.nx) - 1, je = min(j0 + kTY, gc.ny) - 1, ke = k0 + ZT - 1;
   for (int q = tid; q < n_views * 8; q += nthr) {
     const int pv = q >> 3, c = q & 7;
     const BpView w = tv[pv];
@@ -301,20 +305,12 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   const float x = fmaf(float(min(i, gc.nx - 1)) + 0.5f, gc.vx, -gc.hx);
   const float y = fmaf(float(min(j, gc.ny - 1)) + 0.5f, gc.vy, -gc.hy);
   const float z0 = fmaf(float(k0) + 0.5f, gc.vz, -gc.hz);
-  const unsigned maxidx = unsigned(BU * (BV - 1) - 2);
-  float acc[kZT];
+  float2 acc[ZT / 2];
 #pragma unroll
-  for (int q = 0; q < kZT; ++q) acc[q] = 0.f;
+  for (int q = 0; q < ZT / 2; ++q) acc[q] = make_float2(0.f, 0.f);
   int done = 0;
   for (int pv = 0; pv < n_views; ++pv) {
     const bool ok = mbar_wait_bounded(&bars[pv & 1], (pv >> 1) & 1, gc.wait_limit);
-#if !CBCT_BP_ONE_BARRIER
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) { atomicAdd(&flags[1], 1); abort_flag = 1; }
-      break;
-    }
-    done = pv + 1;
-#endif
     const BpView w = tv[pv];
     const int2 o = org[pv];
     const float* sp = reinterpret_cast<const float*>(base_ptr + (pv & 1) * stage_stride);
@@ -330,27 +326,36 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
       const float U = 1.f - yr / gc.SAD;
       wt = 1.f / (U * U);
     }
-    // Floors and the box index on the FMA pipe (exact for |cv| < 2^22; the
-    // index is clamped into the box below whatever it is).
+    // Floors on the FMA pipe (exact for |cv| < 2^22).  The run's rows grow with q,
+    // so taps whose first and last row lie in the box need no clamp; the byte
+    // address comes out of one multiply-add on the biased row's bits.  A run outside
+    // its box lies beyond the detector (taps of 0); a footprint that did not fit its
+    // box was reported above.
     const float fu = floor_small(cu);
     const float au = cu - fu;
-    const float2 tu = make_float2(au, au);
-    const float fubc = fu + kRoundC;
+    const float2 tu = make_float2(au, au), ntu = make_float2(-au, -au);
+    const bool inside = fu >= 0.f && fu <= float(BU - 2) && cv >= 0.f &&
+                        fmaf(float(ZT - 1), dz, cv) <= float(BV - 1) - 0.01f;
+    if (inside) {
+      const uint32_t base = smem_u32(sp) + 4u * (unsigned)int(fu) - unsigned(kRoundBits) * (4u * BU);
+      const float2 wt2 = make_float2(wt, wt);
 #pragma unroll
-    for (int q = 0; q < kZT; ++q) {
-      const float fv = floor_small(cv);
-      const float av = cv - fv;
-      const int idx0 = int_of_biased(fmaf(fv, float(BU), fubc));
-      const unsigned idx = min((unsigned)idx0, maxidx);
-      const float* t = sp + idx;
-      const float2 r0 = make_float2(t[0], t[BU]);        // (u0,v0) (u0,v1)
-      const float2 r1 = make_float2(t[1], t[BU + 1]);    // (u1,v0) (u1,v1)
-      const float2 h = __ffma2_rn(tu, r1, __ffma2_rn(make_float2(-au, -au), r0, r0));
-      const float smp = fmaf(av, h.y - h.x, h.x);
-      acc[q] = FDK ? fmaf(wt, smp, acc[q]) : acc[q] + smp;
-      cv += dz;
+      for (int q = 0; q < ZT / 2; ++q) {   // two voxels, packed
+        const float2 c = make_float2(cv, cv + dz);
+        const float2 bv = __fadd2_rd(c, make_float2(kRoundC, kRoundC));
+        const float2 nf = __ffma2_rn(bv, make_float2(-1.f, -1.f), make_float2(kRoundC, kRoundC));   // -floor
+        const float2 av = __fadd2_rn(c, nf);
+        const uint32_t ta = __float_as_uint(bv.x) * (4u * BU) + base, tb = __float_as_uint(bv.y) * (4u * BU) + base;
+        const float2 p00 = make_float2(lds_f32<0>(ta), lds_f32<0>(tb)), p10 = make_float2(lds_f32<4>(ta), lds_f32<4>(tb));
+        const float2 p01 = make_float2(lds_f32<4 * BU>(ta), lds_f32<4 * BU>(tb));
+        const float2 p11 = make_float2(lds_f32<4 * BU + 4>(ta), lds_f32<4 * BU + 4>(tb));
+        const float2 lo = __ffma2_rn(tu, p10, __ffma2_rn(ntu, p00, p00));
+        const float2 hi = __ffma2_rn(tu, p11, __ffma2_rn(ntu, p01, p01));
+        const float2 smp = __ffma2_rn(av, __ffma2_rn(lo, make_float2(-1.f, -1.f), hi), lo);
+        acc[q] = FDK ? __ffma2_rn(wt2, smp, acc[q]) : __fadd2_rn(acc[q], smp);
+        cv = c.y + dz;
+      }
     }
-#if CBCT_BP_ONE_BARRIER
     // One barrier per view: every thread is done with the stage before it is
     // refilled, and a wait that gave up anywhere ends the loop (the taps read
     // after such a wait stay inside the box; the block's sums are discarded
@@ -360,9 +365,6 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
       break;
     }
     done = pv + 1;
-#else
-    __syncthreads();
-#endif
     if (tid == 0 && pv + 2 < n_views) {
       fence_proxy_async();
       issue(pv + 2);
@@ -375,22 +377,23 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   if (i >= gc.nx || j >= gc.ny) return;
   const size_t base = ((size_t)k0 * gc.ny + j) * gc.nx + i;
   const size_t sz = (size_t)gc.nx * gc.ny;
-  const int nq = min(kZT, gc.nz - k0);
-  constexpr int C = CBCT_BP_EPI_CHUNK;
-  static_assert(kZT % C == 0, "epilogue chunks tile the z-run");
+  const int nq = min(ZT, gc.nz - k0);
+  constexpr int C = kEpiChunk;
+  static_assert(ZT % C == 0, "epilogue chunks tile the z-run");
 #pragma unroll
-  for (int c0 = 0; c0 < kZT; c0 += C) {
+  for (int c0 = 0; c0 < ZT; c0 += C) {
     BpOps ops[C];
 #pragma unroll
     for (int q = 0; q < C; ++q)
       if (c0 + q < nq) ops[q] = bp_load<EPI>(e, base + (c0 + q) * sz);
 #pragma unroll
     for (int q = 0; q < C; ++q)
-      if (c0 + q < nq) bp_finish<EPI>(e, base + (c0 + q) * sz, acc[c0 + q], ops[q]);
+      if (c0 + q < nq)
+        bp_finish<EPI>(e, base + (c0 + q) * sz, (c0 + q) % 2 ? acc[(c0 + q) / 2].y : acc[(c0 + q) / 2].x, ops[q]);
   }
 }
 
-template <int EPI, bool FDK, int BU>
+template <int EPI, bool FDK, int BU, int ZT>
 __global__ void __launch_bounds__(kTX * kTY) bp_tma_kernel(const __grid_constant__ CUtensorMap map,
                                                            const ViewParams* __restrict__ views, int n_views,
                                                            GridConst gc, BpEpi e, int BV, int* flags) {
@@ -399,7 +402,7 @@ __global__ void __launch_bounds__(kTX * kTY) bp_tma_kernel(const __grid_constant
   __shared__ int abort_flag;
   unsigned char* base_ptr =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
-  bp_tma_body<EPI, FDK, BU>(&map, views, n_views, gc, e, BV, flags, blockIdx.x, blockIdx.y, blockIdx.z, base_ptr,
+  bp_tma_body<EPI, FDK, BU, ZT>(&map, views, n_views, gc, e, BV, flags, blockIdx.x, blockIdx.y, blockIdx.z, base_ptr,
                             bars, abort_flag);
 }
 
@@ -421,7 +424,7 @@ struct alignas(128) BpScanRec {
 // atomic counter until the list is empty; the item runs the one-scan kernel's
 // body, so every voxel gets the same arithmetic as in a launch of its own.
 // Items are numbered scan by scan, CTA-grid order (x fastest) inside a scan.
-template <int EPI, bool FDK, int BU>
+template <int EPI, bool FDK, int BU, int ZT>
 __global__ void __launch_bounds__(kTX * kTY) bp_tma_multi_kernel(const BpScanRec* __restrict__ recs, int n_recs,
                                                                  int total, int* __restrict__ counter) {
   extern __shared__ __align__(128) unsigned char smem_dyn[];
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(kTX * kTY) bp_tma_multi_kernel(const BpScanRec
       tensormap_acquire(&R.map);
       last = lo;
     }
-    bp_tma_body<EPI, FDK, BU>(&R.map, R.views, R.n_views, R.gc, R.e, R.BV, R.flags, bi, bj, bk, base_ptr, bars,
+    bp_tma_body<EPI, FDK, BU, ZT>(&R.map, R.views, R.n_views, R.gc, R.e, R.BV, R.flags, bi, bj, bk, base_ptr, bars,
                               abort_flag);
     __syncthreads();
     // A wait that gave up is counted in the scan's flag word and its loads
@@ -485,13 +488,13 @@ CUtensorMap make_bp_map(const cbct_plan* p, const float* proj, int cnt) {
   return m;
 }
 
-template <int EPI, bool FDK, int BU>
+template <int EPI, bool FDK, int BU, int ZT>
 void launch_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi& e, cudaStream_t st) {
   const CUtensorMap m = make_bp_map(p, proj, cnt);
   dim3 block(kTX * kTY);
-  dim3 grid((p->g.nx + kTX - 1) / kTX, (p->g.ny + kTY - 1) / kTY, (p->g.nz + kZT - 1) / kZT);
+  dim3 grid((p->g.nx + kTX - 1) / kTX, (p->g.ny + kTY - 1) / kTY, (p->g.nz + ZT - 1) / ZT);
   const size_t smem = bp_tma_smem(p, cnt);
-  auto k = bp_tma_kernel<EPI, FDK, BU>;
+  auto k = bp_tma_kernel<EPI, FDK, BU, ZT>;
   ensure_smem_attr((const void*)k, smem);
   k<<<grid, block, smem, st>>>(m, p->d_views + first, cnt, p->gc, e, p->bp_box.by, p->d_flags);
   check_launch("bp_tma_kernel");
@@ -524,24 +527,24 @@ bool try_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi
     check_launch("pad_rows_kernel");
     proj = p->d_bp_pad;
   }
-  return with_bp_width(p->bp_box.bx, [&](auto W) {
-    launch_bp_tma<EPI, FDK, decltype(W)::value>(p, first, cnt, proj, e, st);
+  return with_bp(p->bp_box.bx, p->bp_zrun, [&](auto W, auto Z) {
+    launch_bp_tma<EPI, FDK, decltype(W)::value, decltype(Z)::value>(p, first, cnt, proj, e, st);
   });
 }
 
-template <int EPI, bool FDK, int BU>
+template <int EPI, bool FDK, int BU, int ZT>
 void prepare_bp_width(size_t smem) {
-  ensure_smem_attr((const void*)bp_tma_kernel<EPI, FDK, BU>, smem);
+  ensure_smem_attr((const void*)bp_tma_kernel<EPI, FDK, BU, ZT>, smem);
 }
 
-template <int BU>
+template <int BU, int ZT>
 void prepare_bp_all(size_t smem) {
-  prepare_bp_width<kStore, false, BU>(smem);
-  prepare_bp_width<kStore, true, BU>(smem);
-  prepare_bp_width<kRecip, false, BU>(smem);
-  prepare_bp_width<kMom, false, BU>(smem);
-  prepare_bp_width<kSart, false, BU>(smem);
-  prepare_bp_width<kStep, false, BU>(smem);
+  prepare_bp_width<kStore, false, BU, ZT>(smem);
+  prepare_bp_width<kStore, true, BU, ZT>(smem);
+  prepare_bp_width<kRecip, false, BU, ZT>(smem);
+  prepare_bp_width<kMom, false, BU, ZT>(smem);
+  prepare_bp_width<kSart, false, BU, ZT>(smem);
+  prepare_bp_width<kStep, false, BU, ZT>(smem);
 }
 
 template <int EPI, bool FDK>
@@ -578,7 +581,7 @@ void launch_bp(cbct_plan* p, int s, const float* proj, const BpEpi& e, cudaStrea
 }  // namespace
 
 // Chooses the TMA-staged back-projector and its detector box: the largest
-// footprint of any kTX x kTY x kZT block in any view (FP64, corner projections),
+// footprint of any kTX x kTY x zrun block in any view (FP64, corner projections),
 // plus margins.
 void backproject_choose_variant(cbct_plan* p) {
   const cbct_geometry& g = p->g;
@@ -589,7 +592,14 @@ void backproject_choose_variant(cbct_plan* p) {
   const double vx = double(g.lx) / g.nx, vy = double(g.ly) / g.ny, vz = double(g.lz) / g.nz;
   const double ku = g.width / double(g.fov_u), kv = g.height / double(g.fov_v);
   const double bu = g.width / 2.0 - 0.5, bv = g.height / 2.0 - 0.5;
-  const int bxn = (g.nx + kTX - 1) / kTX, byn = (g.ny + kTY - 1) / kTY, bzn = (g.nz + kZT - 1) / kZT;
+  const int bxn = (g.nx + kTX - 1) / kTX, byn = (g.ny + kTY - 1) / kTY;
+  // Long runs where they leave kLongRunCtas CTAs and pad the volume's height by at
+  // most an eighth more than short ones.
+  auto layers = [&](int r) { return (g.nz + r - 1) / r; };
+  const bool tall = bxn * byn * layers(kZRuns[1]) >= kLongRunCtas &&
+                    layers(kZRuns[1]) * kZRuns[1] * 8 <= layers(kZRuns[0]) * kZRuns[0] * 9;
+  const int zrun = kZRuns[tall], bzn = layers(zrun);
+  p->bp_zrun = zrun;
   std::vector<std::pair<int, int>> acc(host_threads(), {0, 0});
   parallel_for(p->n_views, [&](int lo, int hi, int tid) {
     int& eu = acc[tid].first;
@@ -615,10 +625,10 @@ void backproject_choose_variant(cbct_plan* p) {
           eu = std::max(eu, (int)(std::floor(umx) - std::floor(umn)) + 3 + 2);
           // rows: z spans of every z block, at the nearest and farthest magnification;
           // no block spans more than this, so most columns need not look at them
-          const double bound = g.SDD * kv * ((imx - imn) * 0.5 * g.lz + imx * (kZT - 1) * vz);
+          const double bound = g.SDD * kv * ((imx - imn) * (0.5 * g.lz + zrun * vz) + imx * (zrun - 1) * vz);
           if (imn > 0 && std::ceil(bound) + 3 + 2 <= ev) continue;
           for (int bk = 0; bk < bzn; ++bk) {
-            const int k0 = bk * kZT, ke = std::min(k0 + kZT, g.nz) - 1;
+            const int k0 = bk * zrun, ke = k0 + zrun - 1;   // whole runs, also past the volume's top
             const double z0 = (k0 + 0.5) * vz - g.lz / 2.0, z1 = (ke + 0.5) * vz - g.lz / 2.0;
             double vmn = 1e30, vmx = -1e30;
             for (double inv : {imn, imx})
@@ -638,7 +648,7 @@ void backproject_choose_variant(cbct_plan* p) {
   }
   int w = 0;
   for (int c : kBpWidths)
-    if (c >= eu + 3) { w = c; break; }
+    if (c >= eu + 3 && (c != kBpWidths[0] || eu + 3 <= kBpNarrow)) { w = c; break; }
   if (w == 0 || ev > 256) return;
   p->bp_box = SlabBox{w, std::max(ev, 2), 1, 1};
   const int maxv = std::min(p->n_views, 1024);
@@ -650,7 +660,7 @@ void backproject_choose_variant(cbct_plan* p) {
 void backproject_prepare(cbct_plan* p) {
   if (p->bp_variant == 1) {
     const size_t sm = bp_tma_smem(p, p->bp_max_views);
-    with_bp_width(p->bp_box.bx, [&](auto W) { prepare_bp_all<decltype(W)::value>(sm); });
+    with_bp(p->bp_box.bx, p->bp_zrun, [&](auto W, auto Z) { prepare_bp_all<decltype(W)::value, decltype(Z)::value>(sm); });
     if (bp_pad_bytes(p->g, p->max_subset) && !p->d_bp_pad) {
       p->d_bp_pad = static_cast<float*>(plan_alloc(p, bp_pad_bytes(p->g, p->max_subset)));
       p->bp_pad_views = std::min(p->max_subset, kBpPadViews);
@@ -729,9 +739,9 @@ void backproject_step_launch(cbct_plan* p, int s, const float* proj, const float
 namespace {
 
 // Work-list launch of one box width: records at A.dev + off.
-template <int EPI, int BU>
+template <int EPI, int BU, int ZT>
 void add_bp_group(WorkArena& A, const std::vector<BpScanRec>& recs, int total, size_t smem) {
-  auto k = bp_tma_multi_kernel<EPI, false, BU>;
+  auto k = bp_tma_multi_kernel<EPI, false, BU, ZT>;
   ensure_smem_attr((const void*)k, smem);
   const size_t off = A.add(recs.data(), recs.size() * sizeof(BpScanRec));
   const int ci = A.n_counters++;
@@ -744,23 +754,27 @@ void add_bp_group(WorkArena& A, const std::vector<BpScanRec>& recs, int total, s
 }
 
 template <int EPI>
-const void* bp_multi_ptr(int c) {
+const void* bp_multi_ptr(int c, int z) {
   const void* k = nullptr;
-  with_bp_width(kBpWidths[c], [&](auto W) { k = (const void*)bp_tma_multi_kernel<EPI, false, decltype(W)::value>; });
+  with_bp(kBpWidths[c], kZRuns[z], [&](auto W, auto Z) {
+    k = (const void*)bp_tma_multi_kernel<EPI, false, decltype(W)::value, decltype(Z)::value>;
+  });
   return k;
 }
 
 template <int EPI>
 void backproject_multi_t(WorkArena& A, const std::vector<MultiBpJob>& jobs) {
-  std::vector<BpScanRec> groups[kNBpWidths];
-  int totals[kNBpWidths] = {};
-  size_t smem[kNBpWidths] = {};
-  auto flush = [&](int c) {
-    if (groups[c].empty()) return;
-    with_bp_width(kBpWidths[c], [&](auto W) { add_bp_group<EPI, decltype(W)::value>(A, groups[c], totals[c], smem[c]); });
-    groups[c].clear();
-    totals[c] = 0;
-    smem[c] = 0;
+  std::vector<BpScanRec> groups[2][kNBpWidths];
+  int totals[2][kNBpWidths] = {};
+  size_t smem[2][kNBpWidths] = {};
+  auto flush = [&](int z, int c) {
+    if (groups[z][c].empty()) return;
+    with_bp(kBpWidths[c], kZRuns[z], [&](auto W, auto Z) {
+      add_bp_group<EPI, decltype(W)::value, decltype(Z)::value>(A, groups[z][c], totals[z][c], smem[z][c]);
+    });
+    groups[z][c].clear();
+    totals[z][c] = 0;
+    smem[z][c] = 0;
   };
   for (const MultiBpJob& j : jobs) {
     cbct_plan* p = j.p;
@@ -778,10 +792,11 @@ void backproject_multi_t(WorkArena& A, const std::vector<MultiBpJob>& jobs) {
     for (int c = 0; c < kNBpWidths; ++c)
       if (kBpWidths[c] == p->bp_box.bx) w = c;
     const bool tma = p->bp_variant == 1 && cnt <= p->bp_max_views && !needs_padded_rows(p, j.proj) && w >= 0;
-    const int tx = (p->g.nx + kTX - 1) / kTX, ty = (p->g.ny + kTY - 1) / kTY, tz = (p->g.nz + kZT - 1) / kZT;
+    const int tx = (p->g.nx + kTX - 1) / kTX, ty = (p->g.ny + kTY - 1) / kTY, tz = (p->g.nz + p->bp_zrun - 1) / p->bp_zrun;
+    const int z = p->bp_zrun == kZRuns[1];
     bool own = !tma;
     if (tma) {
-      const void* kfn = bp_multi_ptr<EPI>(w);
+      const void* kfn = bp_multi_ptr<EPI>(w, z);
       const size_t sm = bp_tma_smem(p, cnt);
       ensure_smem_attr(kfn, sm);
       own = tx * ty * tz >= kMultiFillWaves * resident_grid(kfn, kTX * kTY, sm);
@@ -803,13 +818,14 @@ void backproject_multi_t(WorkArena& A, const std::vector<MultiBpJob>& jobs) {
     r.BV = p->bp_box.by;
     r.tx = tx;
     r.ty = ty;
-    if ((int)groups[w].size() == kMultiMaxRecs) flush(w);
-    r.base = totals[w];
-    totals[w] += r.tx * r.ty * tz;
-    smem[w] = std::max(smem[w], bp_tma_smem(p, cnt));
-    groups[w].push_back(r);
+    if ((int)groups[z][w].size() == kMultiMaxRecs) flush(z, w);
+    r.base = totals[z][w];
+    totals[z][w] += r.tx * r.ty * tz;
+    smem[z][w] = std::max(smem[z][w], bp_tma_smem(p, cnt));
+    groups[z][w].push_back(r);
   }
-  for (int c = 0; c < kNBpWidths; ++c) flush(c);
+  for (int z = 0; z < 2; ++z)
+    for (int c = 0; c < kNBpWidths; ++c) flush(z, c);
 }
 
 }  // namespace
