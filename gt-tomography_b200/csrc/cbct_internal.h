@@ -71,11 +71,12 @@ inline int host_threads() {
   return (int)std::min(32u, std::max(1u, hc));
 }
 
-// Runs f(begin, end, thread_index) over [0, n) split into contiguous chunks on
-// host_threads() threads (the calling thread takes the first chunk).
+// Runs f(begin, end, thread_index) over [0, n) split into contiguous chunks of at
+// least `grain` on up to host_threads() threads (the calling thread takes the first
+// chunk).  Starting a thread takes some 30 us: a small plan is done sooner without.
 template <class F>
-void parallel_for(int n, F&& f) {
-  const int T = std::max(1, std::min(host_threads(), n));
+void parallel_for(int n, F&& f, int grain = 1) {
+  const int T = std::max(1, std::min(host_threads(), n / std::max(grain, 1)));
   std::vector<std::thread> th;
   const int chunk = (n + T - 1) / T;
   for (int t = 1; t < T; ++t) {
@@ -143,9 +144,9 @@ struct SlabBox {
   int valid;
 };
 
-// Forward projector tiling (compile-time): CTA = TU x TV rays of one view,
-// slabs of TS voxels along the view's dominant in-plane axis, NSTAGE-deep
-// TMA pipeline.  The box holds TS+1 rows of the slab axis padded to kBoxY so
+// Forward projector tiling (compile-time): CTA = TU x TV rays of one view in the
+// gather kernel; slabs of TS voxels along the view's dominant in-plane axis, NSTAGE-deep
+// TMA pipeline in the fan kernel.  The box holds TS+1 rows of the slab axis padded to kBoxY so
 // that neighbouring rows and planes fall in different shared-memory banks.
 constexpr int kTU = 16;
 constexpr int kTV = 16;
@@ -158,7 +159,7 @@ constexpr int kNStage = CBCT_NSTAGE;
 constexpr int kSlabBase = -1;      // slab m covers texel rows [kSlabBase + m*kTS, +kTS)
 constexpr int kMaxSlabs = 260;
 constexpr int kSmemBudget = 200 * 1024;
-// Box widths (memory x) the slab kernel is compiled for; each is 8 mod 16.
+// Box widths (memory x) the row-pair kernel is compiled for; each is 8 mod 16.
 constexpr int kBoxWidths[] = {40, 56, 72, 104, 136};
 // Fan forward projector: kFU detector columns (one per warp) x kFV rows per
 // CTA; the column's samples are interpolated in e and d kFKC at a time.
@@ -177,14 +178,14 @@ constexpr int kFanWidths[] = {24, 40, 56, 72};
 constexpr int kPU = CBCT_PAIR_COLS;
 constexpr int kPV = CBCT_PAIR_ROWS;
 constexpr int kPairThreads = kPU * kPV / 2;
-// Forward-projector blocks per view: the largest of the slab, pair, quad (8 x 16
-// tiles at the finest) and fan tilings (one FP64 partial sum per block).
+// Forward-projector blocks per view: the largest of the gather, pair, slab and quad (8 x
+// 16 tiles at the finest) and fan tilings (one FP64 partial sum per block).
 inline size_t forward_tiles(int W, int H) {
-  const size_t slab = (size_t)((W + kTU - 1) / kTU) * ((H + kTV - 1) / kTV);
+  const size_t gather = (size_t)((W + kTU - 1) / kTU) * ((H + kTV - 1) / kTV);
   const size_t pair = (size_t)((W + kPU - 1) / kPU) * ((H + kPV - 1) / kPV);
   const size_t quad = (size_t)((W + 7) / 8) * ((H + 15) / 16);
   const size_t fan = (size_t)((W + kFU - 1) / kFU) * ((H + kFV - 1) / kFV);
-  return std::max(std::max(slab, pair), std::max(quad, fan));
+  return std::max(std::max(gather, pair), std::max(quad, fan));
 }
 
 
@@ -205,6 +206,7 @@ struct cbct_plan {
   // forward variant: 0 = gather (global loads), 1 = TMA slab, 2 = TMA fan, 3 = TMA row pairs,
   // 4 = TMA row quads
   int fwd_variant = 0;
+  double fwd_fill_rays = 0; // row-pair and row-quad launches of fewer rays run the slab kernel (launch_variant)
   int fwd_pref = 0;         // CBCT_OPT_FORWARD_KERNEL: 0 automatic, 1 slab, 2 gather, 3 fan, 4 pair, 5 quad
   cbct::SlabBox pair{};     // row-pair kernel box for fp32 storage
   cbct::SlabBox pair16{};   // row-pair kernel box for 16-bit storage
@@ -216,7 +218,6 @@ struct cbct_plan {
   int fan_lz = 0;           // line length (planes) of the fan kernel, odd
   cbct::SlabBox slab{};     // box in the view frame for fp32 storage (x starts aligned to 4)
   cbct::SlabBox slab16{};   // box for 16-bit storage (x starts aligned to 8)
-  size_t slab_smem = 0;     // dynamic shared memory of the fp32 slab kernel (bytes)
   std::vector<int> subset_has_xdom;  // per subset (and all-views entry): any x-dominant view
   void* d_volT = nullptr;   // x/y-transposed volume for x-dominant views (volT_bytes)
   void* d_volP = nullptr;   // row-padded volume where nx is not a multiple of 4 (volP_bytes)

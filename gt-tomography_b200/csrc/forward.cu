@@ -7,11 +7,11 @@
 // Interpolation here is FP32 in software (not 9-bit texture weights).
 //
 // Variants (all but the gather kernel give bitwise equal results):
-//  * fwd_slab_kernel: a CTA marches a 16x16 tile of rays of one view through
-//    the volume in slabs of kTS voxels along the view's dominant in-plane
-//    axis.  Each slab's footprint (the box around the tile's ray pyramid) is
-//    staged into shared memory by a 3-D TMA load; out-of-volume texels arrive
-//    as zeros (the border rule for free).  Views whose rays run mostly along x
+//  * fwd_slab_kernel (forward_slab.cuh): one thread per ray.  A warp marches a tile of
+//    rays of one view through the volume in slabs of a few voxels along the view's
+//    dominant in-plane axis.  Each slab's footprint (the box around the tile's ray
+//    pyramid) is staged into shared memory by a 3-D TMA load; out-of-volume texels
+//    arrive as zeros (the border rule for free).  Views whose rays run mostly along x
 //    read an x/y-transposed copy of the volume, so every slab is a range of
 //    memory rows and the box is never padded along its slab axis.  Samples are
 //    taken in ray order, so each ray's sum has the reference's summation
@@ -20,7 +20,7 @@
 //    adjacent rays of a detector column that share their in-plane sample
 //    positions, interpolating them in e and d once.
 //  * fwd_quad_kernel (forward_quad.cuh): four such rays per thread; the kernel of
-//    launches that fill the GPU (quad_choose has the rule).
+//    launches that fill the GPU (quad_choose and launch_variant have the rules).
 //  * fwd_fan_kernel (opt-in): the in-plane sharing across a whole column,
 //    through shared-memory lines.
 //  * fwd_gather_kernel: the same arithmetic with bounds-checked global loads,
@@ -29,7 +29,6 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
-#include <type_traits>
 
 #include "forward_host.h"
 
@@ -116,192 +115,6 @@ __global__ void transpose_multi_kernel(const TransposeRec* __restrict__ recs, in
   const int bx = l % R.tx;
   l /= R.tx;
   transpose_tile<float>(R.in, R.out, R.ny, nullptr, 0, R.nx, R.ny, bx, l % R.ty, l / R.ty, tile);
-}
-
-// ------------------------------------------------------------------ slab/TMA
-struct SlabShared {
-  uint64_t bars[kNStage];
-  int mlo, mhi, abort_flag;
-  int emin[kMaxSlabs], emax[kMaxSlabs], zmin[kMaxSlabs], zmax[kMaxSlabs];
-  double red[8];
-};
-
-// 16-bit boxes take half the shared memory, so those instantiations ask for a
-// register budget that lets four CTAs share an SM.
-template <class V>
-constexpr int slab_min_blocks() { return sizeof(V) == 4 ? 3 : 4; }
-
-// One CTA of the slab kernel: ray tile `tile` of the call.  Shared by the
-// one-scan kernel and the work-list kernel over many scans; smem_raw is the
-// 128-byte aligned dynamic shared memory (TMA destinations).
-template <class V, int BX, bool CHECK, int NS>
-__device__ __forceinline__ void fwd_slab_body(const CUtensorMap* map_v, const CUtensorMap* map_t,
-                                              const V* __restrict__ vol, const ViewParams* __restrict__ views,
-                                              const GridConst& gc, int BZ, const FwdOut& o, int* flags,
-                                              const TileId& tile, unsigned char* smem_raw, SlabShared& sh) {
-  constexpr int BXY = BX * kBoxY;
-  const ViewParams vp = views[tile.z];
-  const int dom = vp.dom;
-  const CUtensorMap* map = dom ? map_v : map_t;
-  const int tid = threadIdx.x;
-  const int p = tile.z;
-  const int u0 = tile.x * kTU, v0 = tile.y * kTV;
-  const int u = u0 + (tid % kTU), v = v0 + (tid / kTU);
-  const bool active = (u < gc.W) && (v < gc.H);
-  const Ray r = make_ray(vp, gc, min(u, gc.W - 1), min(v, gc.H - 1));
-  const bool hit = active && (r.a2 > r.a1);
-  // Frame coordinates: e = cross axis, d = slab axis (y for dom = 1, x for dom = 0).
-  const float ce0 = dom ? r.c0x : r.c0y, dce = dom ? r.dcx : r.dcy;
-  const float cd0 = dom ? r.c0y : r.c0x, dcd = dom ? r.dcy : r.dcx;
-  const float idcd = 1.f / dcd;
-  const float ke = dom ? gc.kx : gc.ky, be = dom ? gc.bx : gc.by;
-  const float kd = dom ? gc.ky : gc.kx, bd = dom ? gc.by : gc.bx;
-  const float Se = dom ? vp.Sx : vp.Sy, Sd = dom ? vp.Sy : vp.Sx;
-
-  if (tid == 0) {
-    sh.mlo = INT_MAX;
-    sh.mhi = INT_MIN;
-    sh.abort_flag = 0;
-    for (int s = 0; s < NS; ++s) mbar_init(&sh.bars[s], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  if (hit) {
-    const int f0 = int(floorf(cd0));
-    const int f1 = int(floorf(fmaf(float(gc.N - 1), dcd, cd0)));
-    const int m0 = (max(f0, kSlabBase) - kSlabBase) / kTS;
-    const int m1 = (max(f1, kSlabBase) - kSlabBase) / kTS;
-    atomicMin(&sh.mlo, min(m0, m1));
-    atomicMax(&sh.mhi, max(m0, m1));
-  }
-  __syncthreads();
-  const int mlo = sh.mlo, mhi = sh.mhi;
-  int nslab = (mhi >= mlo) ? (mhi - mlo + 1) : 0;
-  if (nslab > kMaxSlabs) {
-    if (tid == 0) atomicAdd(&flags[0], 1);
-    nslab = 0;
-  }
-
-  // Footprint of every slab: bounding box of the four corner rays of the tile
-  // at the two bounding planes of the slab (the tile's rays form a convex
-  // pyramid, so its cross-section inside the slab lies in that box).
-  for (int i = tid; i < nslab; i += blockDim.x) {
-    sh.emin[i] = INT_MAX; sh.emax[i] = INT_MIN;
-    sh.zmin[i] = INT_MAX; sh.zmax[i] = INT_MIN;
-  }
-  __syncthreads();
-  const int ue = min(u0 + kTU, gc.W) - 1, ve = min(v0 + kTV, gc.H) - 1;
-  const int ne = dom ? gc.nx : gc.ny;  // volume extent along e
-  for (int q = tid; q < nslab * 8; q += blockDim.x) {
-    const int i = q >> 3, c = q & 7;
-    const int m = mlo + i;
-    const float plane = float(kSlabBase + m * kTS + ((c & 4) ? kTS : 0));
-    const int uc = (c & 1) ? ue : u0, vc = (c & 2) ? ve : v0;
-    const float dx = fmaf(float(uc), vp.Eux, vp.D0x);
-    const float dy = fmaf(float(uc), vp.Euy, vp.D0y);
-    const float dz = fmaf(float(vc), vp.Evz, vp.D0z);
-    const float de = dom ? dx : dy, dd = dom ? dy : dx;
-    const float t = ((plane - bd) / kd - Sd) / dd;
-    float ce = fmaf(fmaf(t, de, Se), ke, be);
-    float cz = fmaf(t * dz, gc.kz, gc.bz);
-    // Clamp before the int conversion so that far-away planes stay finite.
-    // Samples lie inside the volume (texel floors in [-1, n-1]; outside it the
-    // border reads 0), so the box only has to cover the footprint's part in it.
-    const int fe = min(max(int(floorf(fminf(fmaxf(ce, -1.0e5f), 1.0e5f))), -1), ne - 1);
-    const int fz = min(max(int(floorf(fminf(fmaxf(cz, -1.0e5f), 1.0e5f))), -1), gc.nz - 1);
-    atomicMin(&sh.emin[i], fe);
-    atomicMax(&sh.emax[i], fe);
-    atomicMin(&sh.zmin[i], fz);
-    atomicMax(&sh.zmax[i], fz);
-  }
-  __syncthreads();
-
-  const uint32_t box_bytes = uint32_t(BX * kBoxY * BZ * sizeof(V));
-  const uint32_t stage_stride = (box_bytes + 127u) & ~127u;
-  const unsigned maxidx = unsigned(BXY * (BZ - 1) - BX - 2);
-  // Box origin of slab i (visiting order), frame/memory order (e, d, z).
-  auto origin = [&](int i, int& oe, int& od, int& oz, int& m) {
-    m = (vp.dsgn > 0) ? mlo + i : mhi - i;
-    const int ii = m - mlo;
-    oe = (sh.emin[ii] - 1) & ~(int(16 / sizeof(V)) - 1);   // 16-byte aligned x start
-    od = kSlabBase + m * kTS;
-    oz = sh.zmin[ii] - 1;
-  };
-  auto issue = [&](int i) {
-    int oe, od, oz, m;
-    origin(i, oe, od, oz, m);
-    uint64_t* bar = &sh.bars[i % NS];
-    mbar_arrive_expect_tx(bar, box_bytes);
-    tma_load_3d(smem_raw + (i % NS) * stage_stride, map, oe, od, oz, bar);
-  };
-  if (tid == 0) {
-    for (int i = 0; i < min(NS, nslab); ++i) issue(i);
-  }
-
-  float acc = 0.f;
-  float kf = 0.f;
-  const float Nf = float(gc.N);
-  int bad = 0;
-  int done = 0;
-  for (int i = 0; i < nslab; ++i) {
-    const int slot = i % NS;
-    const bool ok = mbar_wait_bounded(&sh.bars[slot], (i / NS) & 1, gc.wait_limit);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) { atomicAdd(&flags[1], 1); sh.abort_flag = 1; }
-      break;
-    }
-    done = i + 1;
-    int oe, od, oz, m;
-    origin(i, oe, od, oz, m);
-    if (CHECK && tid == 0) {
-      // The footprint (max + 1) plus a one-voxel margin must fit in the box.
-      const int ii = m - mlo;
-      if (sh.emax[ii] + 2 - oe >= BX || sh.zmax[ii] + 2 - oz >= BZ) atomicAdd(&flags[0], 1);
-    }
-    if (hit) {
-      const V* s = reinterpret_cast<const V*>(smem_raw + slot * stage_stride);
-      const float lo = float(od), hi = lo + float(kTS);
-      const float cmo = kRoundC - float(oe + od * BX + oz * BXY);
-      if (vp.dsgn > 0)
-        slab_samples<V, BX, 1, CHECK>(s, kf, Nf, ce0, cd0, r.c0z, dce, dcd, idcd, r.dcz, lo, hi, cmo, maxidx, acc,
-                                        bad);
-      else
-        slab_samples<V, BX, -1, CHECK>(s, kf, Nf, ce0, cd0, r.c0z, dce, dcd, idcd, r.dcz, lo, hi, cmo, maxidx, acc,
-                                         bad);
-    }
-    __syncthreads();
-    if (tid == 0 && i + NS < nslab) {
-      fence_proxy_async();
-      issue(i + NS);
-    }
-  }
-  if (sh.abort_flag && tid == 0) {
-    // Drain loads still in flight (bounded) before the CTA exits.
-    for (int i = done; i < min(done + NS, nslab); ++i)
-      if (!mbar_wait_bounded(&sh.bars[i % NS], (i / NS) & 1, kWaitLimit)) sh.abort_flag = 2;
-  }
-  if (CHECK) {
-    if (hit && kf != Nf) bad = 1;  // every sample of a hit ray must be consumed
-    if (bad) atomicAdd(&flags[0], 1);
-  }
-
-  const float grown = grown_rays(vol, vp, gc, u, v, active && !hit);
-  const float val = hit ? acc * r.delta : grown;
-  fwd_epilogue(o, gc, vp, p, u, v, active, val, sh.red, tid, tile.bid);
-}
-
-template <class V, int BX, bool CHECK, int NS>
-__global__ void __launch_bounds__(256, slab_min_blocks<V>()) fwd_slab_kernel(const __grid_constant__ CUtensorMap map_v,
-                                                       const __grid_constant__ CUtensorMap map_t,
-                                                       const V* __restrict__ vol,
-                                                       const ViewParams* __restrict__ views, GridConst gc,
-                                                       int BZ, FwdOut o, int* flags) {
-  // TMA destinations are 128-byte aligned (128 extra bytes are requested).
-  extern __shared__ __align__(128) unsigned char smem_dyn[];
-  unsigned char* smem_raw =
-      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
-  __shared__ SlabShared sh;
-  fwd_slab_body<V, BX, CHECK, NS>(&map_v, &map_t, vol, views, gc, BZ, o, flags, launch_tile(), smem_raw, sh);
 }
 
 // ------------------------------------------------------------------ row pairs
@@ -943,29 +756,15 @@ CUtensorMapDataType tma_dtype(cbct_dtype dt) {
 // until the list is empty and run the one-scan kernel's body on them, so every
 // ray gets the arithmetic of its own launch.  A scan's items are numbered in
 // its one-scan launch order (x fastest), which is also its partial-sum slot.
-enum { kVarSlab1 = 0, kVarSlab2 = 1, kVarPair = 2, kVars = 3 };
-
-template <int VAR>
-constexpr int var_threads() { return VAR == kVarPair ? kPairThreads : 256; }
-template <int VAR, class V>
-constexpr int var_min_blocks() {
-#ifdef CBCT_MULTI_PAIR_MINB
-  if (VAR == kVarPair) return CBCT_MULTI_PAIR_MINB;
-#endif
-  return VAR == kVarPair ? pair_min_blocks<V>() : slab_min_blocks<V>();
-}
-
-template <int VAR, class V, int BX>
-__global__ void __launch_bounds__(var_threads<VAR>(), var_min_blocks<VAR, V>())
+template <int BX>
+__global__ void __launch_bounds__(kPairThreads, pair_min_blocks<float>())
     fwd_multi_kernel(const FwdScanRec* __restrict__ recs, int n_recs, int total, int* __restrict__ counter) {
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   unsigned char* smem_raw =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
-  using Shared = typename std::conditional<VAR <= kVarSlab2, SlabShared, PairShared>::type;
-  __shared__ Shared sh;
+  __shared__ PairShared sh;
   __shared__ int item;
   __shared__ int base[kMultiMaxRecs];
-  constexpr int kBars = VAR == kVarSlab1 ? 1 : VAR == kVarSlab2 ? 2 : kPairStages;
   for (int i = threadIdx.x; i < n_recs; i += blockDim.x) base[i] = recs[i].base;
   int last = -1;
   for (;;) {
@@ -988,21 +787,15 @@ __global__ void __launch_bounds__(var_threads<VAR>(), var_min_blocks<VAR, V>())
       tensormap_acquire(&R.map_t);
       last = lo;
     }
-    const V* vol = static_cast<const V*>(R.vol);
-    if constexpr (VAR == kVarSlab1)
-      fwd_slab_body<V, BX, false, 1>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.o, R.flags, tile, smem_raw, sh);
-    else if constexpr (VAR == kVarSlab2)
-      fwd_slab_body<V, BX, false, 2>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.o, R.flags, tile, smem_raw, sh);
-    else
-      fwd_pair_body<V, BX, false>(&R.map_v, &R.map_t, vol, R.views, R.gc, R.BZ, R.nsl_max, R.o, R.flags, tile,
-                                  smem_raw, sh);
+    fwd_pair_body<float, BX, false>(&R.map_v, &R.map_t, static_cast<const float*>(R.vol), R.views, R.gc, R.BZ,
+                                    R.nsl_max, R.o, R.flags, tile, smem_raw, sh);
     __syncthreads();
     // A wait that gave up is counted in the scan's flag word and its loads
     // drained; only a CTA whose drain also gave up (a copy may still land in
     // its shared memory) stops taking items.
     const bool ok = sh.abort_flag != 2;
     if (threadIdx.x == 0) {
-      for (int i = 0; i < kBars; ++i) mbar_inval(&sh.bars[i]);
+      for (int i = 0; i < kPairStages; ++i) mbar_inval(&sh.bars[i]);
     }
     if (!ok) break;
   }
@@ -1029,54 +822,17 @@ CUtensorMap make_volume_map(cbct_dtype dt, const void* vol, int n0, int n1, int 
 
 namespace {
 
-// Dynamic shared memory of a slab or fan launch: kNStage TMA stages of the
+// Dynamic shared memory of a fan launch: kNStage TMA stages of the
 // box (128-byte aligned) + the fan kernel's lines + alignment slack.
 static size_t forward_smem(const SlabBox& b, size_t es, int lz, int nsl = 0) {
   return kNStage * ((b.bx * b.by * b.bz * es + 127) & ~size_t(127)) + (size_t)kFU * kFKC * lz * sizeof(float) +
          4 * sizeof(int) * (size_t)nsl + 128;
 }
 
-// Slabs a ray can cross in the larger in-plane direction.
-static int slabs_max(const cbct_geometry& g) {
-  return (std::max(g.nx, g.ny) + 1 - kSlabBase + kTS - 1) / kTS + 1;
-}
-
 // Dynamic shared memory of a row-pair launch: kPairStages boxes (128-byte
 // aligned), the per-slab footprints, alignment slack.
 static size_t pair_smem(const SlabBox& b, size_t es, int nsl) {
   return kPairStages * ((b.bx * b.by * b.bz * es + 127) & ~size_t(127)) + 4 * sizeof(int) * (size_t)nsl + 128;
-}
-
-template <class V>
-const SlabBox& box_for(const cbct_plan* p) { return sizeof(V) == 4 ? p->slab : p->slab16; }
-
-// Two stages while they leave the register-bound number of CTAs per SM;
-// boxes so large that they would not (small volumes under detectors of about
-// one pixel per voxel) stage one slab at a time, and the other CTAs' samples
-// cover each CTA's wait.  Returns the stages and sets the dynamic shared memory.
-template <class V>
-int slab_stages(const SlabBox& b, size_t& smem) {
-  const size_t stage = (b.bx * b.by * b.bz * sizeof(V) + 127) & ~size_t(127);
-  const size_t per_cta = sizeof(SlabShared) + 1024 + 128;
-  const bool two = (2 * stage + per_cta) * slab_min_blocks<V>() <= size_t(228) * 1024;
-  smem = (two ? 2 : 1) * stage + 128;
-  return two ? 2 : 1;
-}
-
-template <class V, int BX>
-void launch_slab(cbct_plan* p, const V* vol, const V* volP, const V* volT, const FwdOut& o, dim3 grid, int first,
-                 cudaStream_t st, cbct_dtype dt) {
-  const SlabBox& b = box_for<V>(p);
-  const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
-  const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
-  size_t smem = 0;
-  const bool two = slab_stages<V>(b, smem) == 2;
-  auto pick = [&](auto k2, auto k1) { return two ? k2 : k1; };
-  auto k = p->debug_checks ? pick(fwd_slab_kernel<V, BX, true, 2>, fwd_slab_kernel<V, BX, true, 1>)
-                           : pick(fwd_slab_kernel<V, BX, false, 2>, fwd_slab_kernel<V, BX, false, 1>);
-  ensure_smem_attr((const void*)k, smem);
-  k<<<grid, 256, smem, st>>>(mv, mt, vol, p->d_views + first, p->gc, b.bz, o, p->d_flags);
-  check_launch("fwd_slab_kernel");
 }
 
 template <class V>
@@ -1088,7 +844,7 @@ void launch_pair(cbct_plan* p, const V* vol, const V* volP, const V* volT, const
   const SlabBox& b = pair_box_for<V>(p);
   const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
   const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
-  const int nsl = slabs_max(p->g);
+  const int nsl = forward_slabs(p->g, kTS);
   const size_t smem = pair_smem(b, sizeof(V), nsl);
   const dim3 grid((p->g.width + kPU - 1) / kPU, (p->g.height + kPV - 1) / kPV, cnt);
   if (p->debug_checks) {
@@ -1112,7 +868,7 @@ void launch_fan(cbct_plan* p, const V* vol, const V* volP, const V* volT, const 
   const SlabBox& b = fan_box_for<V>(p);
   const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
   const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
-  const int nsl = slabs_max(p->g);
+  const int nsl = forward_slabs(p->g, kTS);
   const size_t smem = forward_smem(b, sizeof(V), p->fan_lz, nsl);
   const dim3 grid((p->g.width + kFU - 1) / kFU, (p->g.height + kFV - 1) / kFV, cnt);
   if (p->debug_checks) {
@@ -1145,11 +901,11 @@ void* padded_rows(cbct_plan* p, size_t es) {
 
 template <class V>
 void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaStream_t st, cbct_dtype dt,
-                  bool use_slab) {
+                  int variant) {
   const V* vol = static_cast<const V*>(vol_v);
   const int first = p->first[s], cnt = p->count[s];
   dim3 grid((p->g.width + kTU - 1) / kTU, (p->g.height + kTV - 1) / kTV, cnt);
-  if (!use_slab) {
+  if (variant == 0) {
     fwd_gather_kernel<V><<<grid, 256, 0, st>>>(vol, p->d_views + first, p->gc, o);
     check_launch("fwd_gather_kernel");
     return;
@@ -1165,11 +921,11 @@ void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaS
     check_launch("volume_copies_kernel");
   }
   const V* const volP = pad ? pad : vol;
-  if (p->fwd_variant == 4) {
+  if (variant == 4) {
     quad_launch(p, dt, vol, volP, volT, o, first, cnt, st);
     return;
   }
-  if (p->fwd_variant == 3) {
+  if (variant == 3) {
     switch (pair_box_for<V>(p).bx) {
       case 40: launch_pair<V, 40>(p, vol, volP, volT, o, first, cnt, st, dt); break;
       case 56: launch_pair<V, 56>(p, vol, volP, volT, o, first, cnt, st, dt); break;
@@ -1180,7 +936,7 @@ void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaS
     }
     return;
   }
-  if (p->fwd_variant == 2) {
+  if (variant == 2) {
     switch (fan_box_for<V>(p).bx) {
       case 24: launch_fan<V, 24>(p, vol, volP, volT, o, first, cnt, st, dt); break;
       case 40: launch_fan<V, 40>(p, vol, volP, volT, o, first, cnt, st, dt); break;
@@ -1190,22 +946,7 @@ void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaS
     }
     return;
   }
-  switch (box_for<V>(p).bx) {
-    case 40: launch_slab<V, 40>(p, vol, volP, volT, o, grid, first, st, dt); break;
-    case 56: launch_slab<V, 56>(p, vol, volP, volT, o, grid, first, st, dt); break;
-    case 72: launch_slab<V, 72>(p, vol, volP, volT, o, grid, first, st, dt); break;
-    case 104: launch_slab<V, 104>(p, vol, volP, volT, o, grid, first, st, dt); break;
-    case 136: launch_slab<V, 136>(p, vol, volP, volT, o, grid, first, st, dt); break;
-    default: throw Error(CBCT_ERR_INTERNAL, "unsupported slab box width");
-  }
-}
-
-template <class V, int BX>
-void prepare_width(size_t smem) {
-  ensure_smem_attr((const void*)fwd_slab_kernel<V, BX, false, 2>, smem);
-  ensure_smem_attr((const void*)fwd_slab_kernel<V, BX, true, 2>, smem);
-  ensure_smem_attr((const void*)fwd_slab_kernel<V, BX, false, 1>, smem);
-  ensure_smem_attr((const void*)fwd_slab_kernel<V, BX, true, 1>, smem);
+  slab_launch(p, dt, vol, volP, volT, o, first, cnt, st);
 }
 
 template <class V, int BX>
@@ -1224,7 +965,7 @@ template <class V>
 void prepare_typed(const cbct_plan* p) {
   if (p->fwd_variant == 3) {
     const SlabBox& b = pair_box_for<V>(p);
-    const size_t ps = pair_smem(b, sizeof(V), slabs_max(p->g));
+    const size_t ps = pair_smem(b, sizeof(V), forward_slabs(p->g, kTS));
     switch (b.bx) {
       case 40: prepare_pair_width<V, 40>(ps); break;
       case 56: prepare_pair_width<V, 56>(ps); break;
@@ -1236,7 +977,7 @@ void prepare_typed(const cbct_plan* p) {
   }
   if (p->fwd_variant == 2) {
     const SlabBox& f = fan_box_for<V>(p);
-    const size_t fs = forward_smem(f, sizeof(V), p->fan_lz, slabs_max(p->g));
+    const size_t fs = forward_smem(f, sizeof(V), p->fan_lz, forward_slabs(p->g, kTS));
     switch (f.bx) {
       case 24: prepare_fan_width<V, 24>(fs); break;
       case 40: prepare_fan_width<V, 40>(fs); break;
@@ -1245,20 +986,13 @@ void prepare_typed(const cbct_plan* p) {
       default: break;
     }
   }
-  if (p->fwd_variant != 1) return;
-  const SlabBox& b = box_for<V>(p);
-  const size_t smem = forward_smem(b, sizeof(V), 0);
-  switch (b.bx) {
-    case 40: prepare_width<V, 40>(smem); break;
-    case 56: prepare_width<V, 56>(smem); break;
-    case 72: prepare_width<V, 72>(smem); break;
-    case 104: prepare_width<V, 104>(smem); break;
-    case 136: prepare_width<V, 136>(smem); break;
-    default: break;
-  }
 }
 
 }  // namespace
+
+int forward_slabs(const cbct_geometry& g, int TS) {
+  return (std::max(g.nx, g.ny) + 1 - kSlabBase + TS - 1) / TS + 1;
+}
 
 // Largest footprint of one slab over every view and tile of a TU x TV tiling
 // (corner-ray bounding box in the view's frame, computed in FP64): e extent
@@ -1282,7 +1016,7 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
       const int dom = vp.dom;
       const int Nd = dom ? g.ny : g.nx;
       const double ke = dom ? kx : ky, be = dom ? bx : by, kd = dom ? ky : kx, bd = dom ? by : bx;
-      const double Se = dom ? vp.Sx : vp.Sy, Sd = dom ? vp.Sy : vp.Sx;
+      const double Se = dom ? vp.Sx : vp.Sy, Sd = dom ? vp.Sy : vp.Sx, ikd = 1.0 / kd;
       const int nsl = (Nd + 1 - kSlabBase + TS - 1) / TS + 1;
       if (nsl * TS > kMaxSlabs * kTS) { a.ok = 0; break; }
       for (int tv = 0; tv < tiles_v; ++tv) {
@@ -1303,15 +1037,25 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
           if (dd[c] * vp.dsgn <= 0 || dd[c] * vp.dsgn < 0.25 * std::fabs(de[c])) a.ok = 0;
         }
         if (!a.ok) break;
-        for (int m = 0; m < nsl; ++m) {
-          double emn = 1e30, emx = -1e30, tmn = 1e30, tmx = -1e30;
-          for (int c = 0; c < 4; ++c) {
-            const double plane = kSlabBase + m * TS + ((c & 2) ? TS : 0);
-            const double t = ((plane - bd) / kd - Sd) / dd[c & 1];
-            const double ce = (Se + t * de[c & 1]) * ke + be;
-            emn = std::min(emn, ce); emx = std::max(emx, ce);
-            tmn = std::min(tmn, t); tmx = std::max(tmx, t);
+        // Ray parameters t and e coordinates of the tile's two edge columns at a
+        // slab's first plane; the last plane is the next slab's first.
+        const double idd[2] = {1.0 / dd[0], 1.0 / dd[1]};
+        double t0[2], e0[2], t1[2], e1[2];
+        auto at_plane = [&](int m, double (&t)[2], double (&e)[2]) {
+          const double pl = (kSlabBase + m * TS - bd) * ikd - Sd;
+          for (int c = 0; c < 2; ++c) {
+            t[c] = pl * idd[c];
+            e[c] = (Se + t[c] * de[c]) * ke + be;
           }
+        };
+        at_plane(0, t1, e1);
+        for (int m = 0; m < nsl; ++m) {
+          for (int c = 0; c < 2; ++c) { t0[c] = t1[c]; e0[c] = e1[c]; }
+          at_plane(m + 1, t1, e1);
+          const double emn = std::min(std::min(e0[0], e0[1]), std::min(e1[0], e1[1]));
+          const double emx = std::max(std::max(e0[0], e0[1]), std::max(e1[0], e1[1]));
+          const double tmn = std::min(std::min(t0[0], t0[1]), std::min(t1[0], t1[1]));
+          const double tmx = std::max(std::max(t0[0], t0[1]), std::max(t1[0], t1[1]));
           // elements from floor(min)-1 to floor(max)+1 inclusive, +2 margin; the
           // kernels clamp footprints to the volume, whose extent bounds the box
           const int Ne = dom ? g.nx : g.ny;
@@ -1322,18 +1066,31 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
           // where none can exceed the extent found so far.
           const double dmax = std::min(dzabs, (g.nz + 1.0 - bz) / (kz * std::max(tmn, 1e-9)));
           if (tmn > 0 && std::ceil(kz * ((tmx - tmn) * dmax + tmx * dzspan)) + 3 + 2 <= a.z) continue;
-          for (int tv = 0; tv < tiles_v; ++tv) {
+          // One tile row; false where the rows towards the centre, whose extent is
+          // smaller, cannot exceed the extent found so far.
+          auto row = [&](int tv) {
             const double z00 = tmn * dz0[tv], z01 = tmn * dz1[tv], z10 = tmx * dz0[tv], z11 = tmx * dz1[tv];
             const double zmn = std::min(std::min(z00, z01), std::min(z10, z11)) * kz + bz;
             const double zmx = std::max(std::max(z00, z01), std::max(z10, z11)) * kz + bz;
-            if (zmx < -1.0 || zmn > g.nz) continue;
+            if (zmx < -1.0 || zmn > g.nz) return true;
+            if (std::ceil(zmx - zmn) + 3 + 2 <= a.z) return false;
             const int ez = (int)(std::floor(zmx) - std::floor(zmn)) + 3 + 2;
             a.z = std::max(a.z, std::min(ez, g.nz + 4));
+            return true;
+          };
+          row(tiles_v - 1);   // may hold fewer rays than the others
+          int lo_v = 0, hi_v = tiles_v - 2;
+          if (tmn > 0) {
+            while (lo_v <= hi_v && dz1[lo_v] <= 0 && row(lo_v)) ++lo_v;
+            while (hi_v >= lo_v && dz0[hi_v] >= 0 && row(hi_v)) --hi_v;
+            while (lo_v <= hi_v && dz1[lo_v] <= 0) ++lo_v;
+            while (hi_v >= lo_v && dz0[hi_v] >= 0) --hi_v;
           }
+          for (int tv = lo_v; tv <= hi_v; ++tv) row(tv);
         }
       }
     }
-  });
+  }, 16000 / std::max(1, tiles_u * forward_slabs(g, TS)));
   ext_e = ext_z = 0;
   bool ok = true;
   for (const Acc& a : acc) {
@@ -1386,29 +1143,21 @@ void forward_choose_variant(cbct_plan* p) {
     return 0;
   };
   const double row_dz = row_dz_max(p);
+  const double height = double(p->g.fov_v) * (p->g.SAD / p->g.SDD) * p->g.nz / p->g.lz;
+  p->fwd_fill_rays = height <= p->g.nz ? 8e5 : row_dz < 0.9 ? 2e6 : 3e6;
   if ((p->fwd_pref == 0 || p->fwd_pref == 5) && quad_choose(p, row_dz, p->fwd_pref == 5)) {
     p->fwd_variant = 4;
+    if (p->fwd_pref == 0) slab_choose(p);
     return;
   }
   int e, z;
-  if (slab_extents(p, kTU, kTV, kTS, e, z)) {
-    const int w32 = width(kBoxWidths, e, 3), w16 = width(kBoxWidths, e, 7);
-    const int boxz = std::max(z, 2);
-    const SlabBox b32{w32, kBoxY, boxz, 1}, b16{w16, kBoxY, boxz, 1};
-    if (w32 && w16 && boxz <= 256 && forward_smem(b32, 4, 0) <= (size_t)kSmemBudget &&
-        forward_smem(b16, 2, 0) <= (size_t)kSmemBudget) {
-      p->slab = b32;
-      p->slab16 = b16;
-      p->slab_smem = forward_smem(b32, 4, 0);
-      p->fwd_variant = 1;
-    }
-  }
+  if (slab_choose(p)) p->fwd_variant = 1;
   if ((p->fwd_pref == 4 || (p->fwd_pref == 0 && p->fwd_variant == 1 && row_dz < 0.99)) &&
       slab_extents(p, kPU, kPV, kTS, e, z)) {
     const int w32 = width(kBoxWidths, e, 3), w16 = width(kBoxWidths, e, 7);
     const int boxz = std::max(z, 3);
     const SlabBox b32{w32, kPairBoxY, boxz, 1}, b16{w16, kPairBoxY, boxz, 1};
-    const int nsl = slabs_max(p->g);
+    const int nsl = forward_slabs(p->g, kTS);
     if (w32 && w16 && boxz <= 256 && pair_smem(b32, 4, nsl) <= (size_t)kSmemBudget &&
         pair_smem(b16, 2, nsl) <= (size_t)kSmemBudget) {
       p->pair = b32;
@@ -1421,7 +1170,7 @@ void forward_choose_variant(cbct_plan* p) {
     const int boxz = std::max(z, 2);
     const int lz = (boxz + 1) | 1;  // odd: consecutive lines start in different banks
     const SlabBox b32{w32, kBoxY, boxz, 1}, b16{w16, kBoxY, boxz, 1};
-    const int nsl = slabs_max(p->g);
+    const int nsl = forward_slabs(p->g, kTS);
     if (w32 && w16 && boxz <= 256 && forward_smem(b32, 4, lz, nsl) <= (size_t)kSmemBudget &&
         forward_smem(b16, 2, lz, nsl) <= (size_t)kSmemBudget) {
       p->fan = b32;
@@ -1432,11 +1181,31 @@ void forward_choose_variant(cbct_plan* p) {
   }
 }
 
+// Variant of a launch of cnt views.  Row pairs and quads need many rays: a thread
+// marches two or four one after another, and rays cut by the volume's top or bottom
+// face are marched by themselves.  Below fwd_fill_rays rays an automatically chosen
+// plan's launches run the per-ray slab kernel, whose results are bitwise the same.
+// Measured in ms, slab against the better of pairs and quads: detectors that the volume's
+// height covers, threshold 0.8 million rays: 2 views of 0.9 mm pixels into 128^3
+// (0.12 M rays) 0.088 to 0.173, 8 views (0.47 M) 0.223 to 0.232, 32 views (1.9 M) 0.829
+// to 0.692; 2 views of 0.75 mm into 256^3 (0.68 M) 0.54 to 0.71, 8 views (2.7 M) 2.07 to
+// 1.48.  Taller detectors, whose outer rays are cut, 2 million: 8 views of 0.9 mm into
+// 128^3 (0.52 M) 0.243 to 0.310, 32 views (2.1 M) 0.895 to 0.914, 40 views of 301x211
+// into 150x141x93 (2.5 M) 1.07 to 0.97; 3 million for rows 0.9 texel or more apart:
+// 2 views of 1.5 mm into 256^3 (0.2 M) 0.25 to 0.55, 64 views of 256x192 into 128^3
+// (3.1 M) 1.06 to 1.01.
+static int launch_variant(const cbct_plan* p, int cnt) {
+  const bool rows = p->fwd_variant == 3 || p->fwd_variant == 4;
+  if (rows && p->fwd_pref == 0 && p->slab.bx && double(p->g.width) * p->g.height * cnt < p->fwd_fill_rays) return 1;
+  return p->fwd_variant;
+}
+
 void forward_prepare(cbct_plan* p) {
   if (p->fwd_variant < 1) return;
   prepare_typed<float>(p);
   prepare_typed<__half>(p);
   prepare_typed<__nv_bfloat16>(p);
+  if (p->slab.bx) slab_prepare(p);
   if (p->fwd_variant == 4) quad_prepare(p);
   bool any_x = false;
   for (size_t s = 0; s < p->subset_has_xdom.size(); ++s) any_x = any_x || p->subset_has_xdom[s];
@@ -1467,23 +1236,24 @@ void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, floa
   if (cnt == 0) return;
   o.wproj = p->d_pweights ? p->d_pweights + (size_t)p->g.width * p->g.height * p->first[s] : nullptr;
   const size_t es = dtype_size(dt);
-  const bool use_slab = p->fwd_variant >= 1 &&
-                        (!needs_padded_rows(vol, p->g.nx, es) || padded_rows(p, es) != nullptr) &&
-                        (!p->subset_has_xdom[s] || p->d_volT != nullptr);
+  const bool tma = (!needs_padded_rows(vol, p->g.nx, es) || padded_rows(p, es) != nullptr) &&
+                   (!p->subset_has_xdom[s] || p->d_volT != nullptr);
+  const int variant = tma ? launch_variant(p, cnt) : 0;
   // One partial sum per block of the kernel that will run.
-  const bool fan = use_slab && p->fwd_variant == 2, pair = use_slab && p->fwd_variant == 3;
-  const bool quad = use_slab && p->fwd_variant == 4;
-  int TU = fan ? kFU : pair ? kPU : kTU, TV = fan ? kFV : pair ? kPV : kTV;
-  if (quad) quad_tile(p->quad_shape, TU, TV);
+  int TU = kTU, TV = kTV;
+  if (variant == 1) slab_tile(TU, TV);
+  else if (variant == 2) { TU = kFU; TV = kFV; }
+  else if (variant == 3) { TU = kPU; TV = kPV; }
+  else if (variant == 4) quad_tile(p->quad_shape, TU, TV);
   const size_t nblocks = (size_t)((p->g.width + TU - 1) / TU) * ((p->g.height + TV - 1) / TV) * cnt;
   if (norm2_out) {
     if (nblocks > p->n_partials) throw Error(CBCT_ERR_INTERNAL, "partials buffer too small");
     o.partials = p->d_partials;
   }
   switch (dt) {
-    case CBCT_F32: launch_typed<float>(p, s, vol, o, st, dt, use_slab); break;
-    case CBCT_F16: launch_typed<__half>(p, s, vol, o, st, dt, use_slab); break;
-    case CBCT_BF16: launch_typed<__nv_bfloat16>(p, s, vol, o, st, dt, use_slab); break;
+    case CBCT_F32: launch_typed<float>(p, s, vol, o, st, dt, variant); break;
+    case CBCT_F16: launch_typed<__half>(p, s, vol, o, st, dt, variant); break;
+    case CBCT_BF16: launch_typed<__nv_bfloat16>(p, s, vol, o, st, dt, variant); break;
     default: throw Error(CBCT_ERR_INVALID_ARGUMENT, "unknown volume dtype");
   }
   if (norm2_out) finalize_partials(p->d_partials, (int)nblocks, norm2_out, st);
@@ -1505,22 +1275,15 @@ void add_fwd_group(WorkArena& A, FwdMultiKernel k, int threads, const std::vecto
   });
 }
 
-template <int VAR>
-FwdMultiKernel fwd_multi_ptr_v(int bx) {
+FwdMultiKernel fwd_multi_ptr(int bx) {
   switch (bx) {
-    case 40: return fwd_multi_kernel<VAR, float, 40>;
-    case 56: return fwd_multi_kernel<VAR, float, 56>;
-    case 72: return fwd_multi_kernel<VAR, float, 72>;
-    case 104: return fwd_multi_kernel<VAR, float, 104>;
-    case 136: return fwd_multi_kernel<VAR, float, 136>;
+    case 40: return fwd_multi_kernel<40>;
+    case 56: return fwd_multi_kernel<56>;
+    case 72: return fwd_multi_kernel<72>;
+    case 104: return fwd_multi_kernel<104>;
+    case 136: return fwd_multi_kernel<136>;
     default: throw Error(CBCT_ERR_INTERNAL, "unsupported forward box width");
   }
-}
-
-FwdMultiKernel fwd_multi_ptr(int var, int bx) {
-  return var == kVarSlab1   ? fwd_multi_ptr_v<kVarSlab1>(bx)
-         : var == kVarSlab2 ? fwd_multi_ptr_v<kVarSlab2>(bx)
-                            : fwd_multi_ptr_v<kVarPair>(bx);
 }
 
 // The scans of one kernel (kind, shape and box width).
@@ -1565,7 +1328,7 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
     if (cnt == 0) continue;
     const bool tma = p->fwd_variant >= 1 && ((size_t)p->g.nx * 4) % 16 == 0 && ((size_t)p->g.ny * 4) % 16 == 0 &&
                      (reinterpret_cast<uintptr_t>(j.vol) % 16 == 0) && (!p->subset_has_xdom[s] || p->d_volT);
-    const int fv = p->fwd_variant;
+    const int fv = launch_variant(p, cnt);
     auto one_scan = [&A](const MultiFwdJob& jj) {
       A.ops.push_back([jj](cudaStream_t st) {
         forward_launch_ex(jj.p, jj.s, CBCT_F32, jj.vol, jj.out, jj.b, nullptr, 1.f, kModeResidual, jj.apply_offset,
@@ -1576,20 +1339,21 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
       one_scan(j);
       continue;
     }
-    int nsl = slabs_max(p->g), TU, TV, threads;
+    int nsl = forward_slabs(p->g, kTS), TU, TV, threads;
     SlabBox b;
     size_t sm = 0;
     FwdMultiKernel kernel;
     if (fv == 4) {
-      const QuadMulti q = quad_multi(p);
+      const ForwardMulti q = quad_multi(p);
       b = p->quad; kernel = q.kernel; nsl = q.nsl; sm = q.smem; threads = q.threads;
       quad_tile(p->quad_shape, TU, TV);
     } else if (fv == 3) {
       b = p->pair; TU = kPU; TV = kPV; sm = pair_smem(b, 4, nsl); threads = kPairThreads;
-      kernel = fwd_multi_ptr(kVarPair, b.bx);
+      kernel = fwd_multi_ptr(b.bx);
     } else {
-      b = p->slab; TU = kTU; TV = kTV; threads = 256;
-      kernel = fwd_multi_ptr(slab_stages<float>(b, sm) == 2 ? kVarSlab2 : kVarSlab1, b.bx);
+      const ForwardMulti q = slab_multi(p);
+      b = p->slab; kernel = q.kernel; nsl = q.nsl; sm = q.smem; threads = q.threads;
+      slab_tile(TU, TV);
     }
     const int tx = (p->g.width + TU - 1) / TU, ty = (p->g.height + TV - 1) / TV;
     const int nblocks = tx * ty * cnt;

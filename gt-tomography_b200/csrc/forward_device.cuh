@@ -245,6 +245,40 @@ __device__ __forceinline__ void slab_samples(const V* __restrict__ s, float& kf,
   kf = ke;
 }
 
+// First sample of a ray past the slab [lo, hi), at least k: an estimate, then
+// the exact test (monotone in k; floor(x) >= hi <=> x >= hi and floor(x) < lo <=>
+// x < lo, lo and hi being integers).
+__device__ __forceinline__ float slab_end(float k, float Nf, float cd0, float dcd, bool up, float lo, float hi) {
+  auto out_at = [&](float q) {
+    const float x = fmaf(q, dcd, cd0);
+    return up ? (x >= hi) : (x < lo);
+  };
+  float ke = ceilf(__fdividef((up ? hi : lo) - cd0, dcd));
+  ke = fminf(fmaxf(ke, k), Nf);
+  while (ke > k && out_at(ke - 1.f)) ke -= 1.f;
+  while (ke < Nf && !out_at(ke)) ke += 1.f;
+  return ke;
+}
+
+__device__ __forceinline__ float2 floor2_small(float2 x) {
+  const float2 c = make_float2(kRoundC, kRoundC);
+  return __fadd2_rn(__fadd2_rd(x, c), make_float2(-kRoundC, -kRoundC));
+}
+
+// a - b (one rounding, as the scalar difference).
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+
+// In-plane interpolation (e, then d) at q0 and q1, two planes packed.
+template <class V, int BX>
+__device__ __forceinline__ float2 planes2(const V* __restrict__ q0, const V* __restrict__ q1, float2 te, float2 nte,
+                                          float2 td, float2 ntd) {
+  const float2 a = make_float2(sm_f(q0[0]), sm_f(q1[0])), b = make_float2(sm_f(q0[1]), sm_f(q1[1]));
+  const float2 c = make_float2(sm_f(q0[BX]), sm_f(q1[BX])), d = make_float2(sm_f(q0[BX + 1]), sm_f(q1[BX + 1]));
+  const float2 x = __ffma2_rn(te, b, __ffma2_rn(nte, a, a));
+  const float2 y = __ffma2_rn(te, d, __ffma2_rn(nte, c, c));
+  return __ffma2_rn(td, y, __ffma2_rn(ntd, x, x));
+}
+
 }  // namespace
 
 }  // namespace cbct

@@ -27,6 +27,25 @@ CUtensorMap make_volume_map(cbct_dtype dt, const void* vol, int n0, int n1, int 
 // tiling, margins included; false when some view cannot use slabs.
 bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& ext_z);
 
+// Slabs of TS voxels a ray can cross in the larger in-plane direction.
+int forward_slabs(const cbct_geometry& g, int TS);
+
+using FwdMultiKernel = void (*)(const FwdScanRec*, int, int, int*);
+struct ForwardMulti {
+  FwdMultiKernel kernel;       // work-list kernel of the plan's shape and box width
+  int nsl, threads;
+  size_t smem;
+};
+
+// Per-ray slab projector (forward_slab.cu).
+void slab_tile(int& TU, int& TV);
+bool slab_choose(cbct_plan* p);
+void slab_prepare(const cbct_plan* p);
+// vol: the caller's volume; volP: the copy TMA reads it from (or vol itself).
+void slab_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volP, const void* volT, const FwdOut& o,
+                 int first, int cnt, cudaStream_t st);
+ForwardMulti slab_multi(const cbct_plan* p);
+
 // Row-quad projector (forward_quad.cu).
 enum QuadShape { kQuadWide = 0, kQuadWarp = 1, kQuadThin = 2, kQuadShapes = 3 };
 void quad_tile(int shape, int& TU, int& TV);
@@ -36,12 +55,6 @@ void quad_prepare(const cbct_plan* p);
 void quad_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volP, const void* volT, const FwdOut& o,
                  int first, int cnt, cudaStream_t st);
 
-using FwdMultiKernel = void (*)(const FwdScanRec*, int, int, int*);
-struct QuadMulti {
-  FwdMultiKernel kernel;       // work-list kernel of the plan's shape and box width
-  int nsl, threads;
-  size_t smem;
-};
-QuadMulti quad_multi(const cbct_plan* p);
+ForwardMulti quad_multi(const cbct_plan* p);
 
 }  // namespace cbct

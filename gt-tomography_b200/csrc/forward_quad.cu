@@ -37,11 +37,6 @@ constexpr QuadDims dims_of() {
 }
 constexpr QuadDims kDims[kQuadShapes] = {dims_of<kQuadWide>(), dims_of<kQuadWarp>(), dims_of<kQuadThin>()};
 
-// Slabs a ray can cross in the larger in-plane direction.
-int quad_slabs(const cbct_geometry& g, int TS) {
-  return (std::max(g.nx, g.ny) + 1 - kSlabBase + TS - 1) / TS + 1;
-}
-
 // One box (128-byte aligned), the slabs' box origins, alignment slack.
 size_t quad_smem(const SlabBox& b, size_t es, int nsl) {
   return ((b.bx * b.by * b.bz * es + 127) & ~size_t(127)) + sizeof(int2) * (size_t)nsl + 128;
@@ -75,7 +70,7 @@ void with_quad(const cbct_plan* p, F&& f) {
 template <class V>
 void prepare_typed(const cbct_plan* p) {
   const SlabBox& b = sizeof(V) == 4 ? p->quad : p->quad16;
-  const size_t smem = quad_smem(b, sizeof(V), quad_slabs(p->g, kDims[p->quad_shape].TS));
+  const size_t smem = quad_smem(b, sizeof(V), forward_slabs(p->g, kDims[p->quad_shape].TS));
   with_quad<V>(p, [&](auto BX, auto SHAPE) {
     ensure_smem_attr((const void*)quad_kernel<V, decltype(BX)::value, decltype(SHAPE)::value>(), smem);
   });
@@ -88,7 +83,7 @@ void launch_typed(cbct_plan* p, const V* vol, const V* volP, const V* volT, cons
   const CUtensorMap mv = make_volume_map(dt, volP, p->g.nx, p->g.ny, p->g.nz, b);
   const CUtensorMap mt = volT ? make_volume_map(dt, volT, p->g.ny, p->g.nx, p->g.nz, b) : mv;
   const QuadDims& d = kDims[p->quad_shape];
-  const int nsl = quad_slabs(p->g, d.TS);
+  const int nsl = forward_slabs(p->g, d.TS);
   const size_t smem = quad_smem(b, sizeof(V), nsl);
   const dim3 grid((p->g.width + d.TU - 1) / d.TU, (p->g.height + d.TV - 1) / d.TV, cnt);
   with_quad<V>(p, [&](auto BX, auto SHAPE) {
@@ -180,7 +175,7 @@ bool quad_choose(cbct_plan* p, double row_dz, bool forced) {
     // The x start of a box is rounded down to a 16-byte boundary.
     auto width = [](const int (&list)[2], int ext) { return list[0] >= ext ? list[0] : list[1] >= ext ? list[1] : 0; };
     const int w32 = width(kQuadWidths32[s], e + 3), w16 = width(kQuadWidths16[s], e + 7);
-    const int boxz = std::max(z, 4), nsl = quad_slabs(p->g, d.TS);
+    const int boxz = std::max(z, 4), nsl = forward_slabs(p->g, d.TS);
     const SlabBox b32{w32, d.BY, boxz, 1}, b16{w16, d.BY, boxz, 1};
     if (!w32 || !w16 || boxz > 256 || quad_smem(b32, 4, nsl) > (size_t)kSmemBudget ||
         quad_smem(b16, 2, nsl) > (size_t)kSmemBudget)
@@ -211,10 +206,10 @@ void quad_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volP,
   else go(__nv_bfloat16{});
 }
 
-QuadMulti quad_multi(const cbct_plan* p) {
-  QuadMulti m{};
+ForwardMulti quad_multi(const cbct_plan* p) {
+  ForwardMulti m{};
   const QuadDims& d = kDims[p->quad_shape];
-  m.nsl = quad_slabs(p->g, d.TS);
+  m.nsl = forward_slabs(p->g, d.TS);
   m.smem = quad_smem(p->quad, 4, m.nsl);
   m.threads = d.threads;
   with_quad<float>(p, [&](auto BX, auto SHAPE) {

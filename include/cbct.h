@@ -157,7 +157,8 @@ CBCT_API cbct_status cbct_plan_autotune(cbct_plan* plan, float* times_ms_out, vo
 /* CBCT_OPT_FORWARD_KERNEL: 0 = automatic (the row-quad kernel where adjacent
  * detector rows stay within 0.66 z texel of each other, and up to 1.4 texels in
  * launches with enough rays; else the row-pair kernel where rows stay within one
- * texel, else the per-ray slab kernel, each where its boxes fit, else gather),
+ * texel, else the per-ray slab kernel, each where its boxes fit, else gather; launches
+ * too small to fill the GPU run the slab kernel in place of pairs or quads),
  * 1 = slab, 2 = gather, 3 = the column-fan kernel (e/d interpolation shared by the
  * rays of a detector column; slower on B200 at the sizes measured so far), 4 = the
  * row-pair kernel (one thread marches two vertically adjacent rays of a column and
