@@ -1222,7 +1222,7 @@ void forward_choose_variant(cbct_plan* p) {
       if (w >= ext + slack) return w;
     return 0;
   };
-  const double row_dz = row_dz_max(p);
+  const double row_dz = p->fwd_row_dz = row_dz_max(p);
   const double height = double(p->g.fov_v) * (p->g.SAD / p->g.SDD) * p->g.nz / p->g.lz;
   p->fwd_fill_rays = height <= p->g.nz ? 8e5 : row_dz < 0.9 ? 2e6 : 3e6;
   if ((p->fwd_pref == 0 || p->fwd_pref == 5) && quad_choose(p, row_dz, p->fwd_pref == 5)) {
@@ -1274,9 +1274,14 @@ void forward_choose_variant(cbct_plan* p) {
 // into 150x141x93 (2.5 M) 1.07 to 0.97; 3 million for rows 0.9 texel or more apart:
 // 2 views of 1.5 mm into 256^3 (0.2 M) 0.25 to 0.55, 64 views of 256x192 into 128^3
 // (3.1 M) 1.06 to 1.01.
-static int launch_variant(const cbct_plan* p, int cnt) {
+// Rows beyond 1.2 texels (16-bit volumes: 1) share too few planes at any size: 40 views of
+// 400x300 into 256^3, 1.34 texels, 3.78 to 3.75, 1.5 texels 3.30 to 3.76; bf16 at 1.1 texels 4.01
+// to 4.19, 1.18 texels 3.73 to 4.38.
+static int launch_variant(const cbct_plan* p, int cnt, size_t es) {
   const bool rows = p->fwd_variant == 3 || p->fwd_variant == 4;
-  if (rows && p->fwd_pref == 0 && p->slab.bx && double(p->g.width) * p->g.height * cnt < p->fwd_fill_rays) return 1;
+  const double rays = double(p->g.width) * p->g.height * cnt;
+  if (rows && p->fwd_pref == 0 && p->slab.bx && (rays < p->fwd_fill_rays || p->fwd_row_dz >= (es == 2 ? 1.0 : 1.2)))
+    return 1;
   return p->fwd_variant;
 }
 
@@ -1318,7 +1323,7 @@ void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, floa
   const size_t es = dtype_size(dt);
   const bool tma = (!needs_padded_rows(vol, p->g.nx, es) || padded_rows(p, es) != nullptr) &&
                    (!p->subset_has_xdom[s] || p->d_volT != nullptr);
-  const int variant = tma ? launch_variant(p, cnt) : 0;
+  const int variant = tma ? launch_variant(p, cnt, es) : 0;
   // One partial sum per block of the kernel that will run.
   int TU = kTU, TV = kTV;
   if (variant == 1) slab_tile(TU, TV);
@@ -1366,6 +1371,12 @@ FwdMultiKernel fwd_multi_ptr(int bx) {
   }
 }
 
+// Small scans that fill the GPU together run quads where their rows share enough planes
+// (up to 0.9 texel, 0.6 under detectors taller than the volume, whose outer rays are cut).
+// Their rays are bitwise the slab kernel's; a norm is summed tile by tile, so scans that
+// want theirs keep the kernel of their own launches.
+constexpr double kMultiQuadRays = 3e5;
+
 // The scans of one kernel (kind, shape and box width).
 struct FwdGroup {
   FwdMultiKernel k;
@@ -1379,6 +1390,8 @@ struct FwdGroup {
 
 void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
   std::vector<FwdGroup> groups;
+  double all_rays = 0;
+  for (const MultiFwdJob& j : jobs) all_rays += double(j.p->g.width) * j.p->g.height * j.p->count[j.s];
   // Transposes of the volumes the next launches read, one launch for all.
   std::vector<TransposeRec> tr;
   int tr_total = 0;
@@ -1408,7 +1421,10 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
     if (cnt == 0) continue;
     const bool tma = p->fwd_variant >= 1 && ((size_t)p->g.nx * 4) % 16 == 0 && ((size_t)p->g.ny * 4) % 16 == 0 &&
                      (reinterpret_cast<uintptr_t>(j.vol) % 16 == 0) && (!p->subset_has_xdom[s] || p->d_volT);
-    const int fv = launch_variant(p, cnt);
+    int fv = launch_variant(p, cnt, sizeof(float));
+    if (fv == 1 && p->fwd_variant == 4 && p->fwd_pref == 0 && !j.norm2_out && all_rays >= kMultiQuadRays &&
+        p->fwd_row_dz < (p->fwd_fill_rays < 1e6 ? 0.9 : 0.6))
+      fv = 4;
     auto one_scan = [&A](const MultiFwdJob& jj) {
       A.ops.push_back([jj](cudaStream_t st) {
         forward_launch_ex(jj.p, jj.s, CBCT_F32, jj.vol, jj.out, jj.b, nullptr, 1.f, kModeResidual, jj.apply_offset,

@@ -47,7 +47,7 @@ void slab_launch(cbct_plan* p, cbct_dtype dt, const void* vol, const void* volP,
 ForwardMulti slab_multi(const cbct_plan* p);
 
 // Row-quad projector (forward_quad.cu).
-enum QuadShape { kQuadWide = 0, kQuadWarp = 1, kQuadThin = 2, kQuadShapes = 3 };
+enum QuadShape { kQuadWide = 0, kQuadWarp = 1, kQuadThin = 2, kQuadSkew = 3, kQuadShapes = 4 };
 void quad_tile(int shape, int& TU, int& TV);
 bool quad_choose(cbct_plan* p, double row_dz, bool forced);
 void quad_prepare(const cbct_plan* p);

@@ -11,23 +11,26 @@ namespace cbct {
 namespace {
 
 // Shapes, in the order of QuadShape.  The minimum CTAs per SM set the register
-// budget (80, 128 and 96 registers, no spills).
+// budget (80, 128, 96 and 96 registers).
 //  wide : 16 x 32 tiles of 128 threads, slabs of 8 voxels.  Fewest instructions per
 //         sample; its boxes fit six CTAs per SM where rows are under 2/3 texel apart.
 //  warp : one warp per CTA (8 x 16 rays), slabs of 6.  Twice the box bytes per ray,
 //         but no warp waits for another and the last wave is short.
 //  thin : 8 x 32 tiles of 64 threads, slabs of 4, for boxes that are large because
 //         a detector pixel is about a voxel.
+//  skew : 16 x 16 tiles of 64 threads, slabs of 4, for rows a texel or more apart
+//         (see QuadCfg).
 template <int SHAPE> struct ShapeOf;
 template <> struct ShapeOf<kQuadWide> { using C = QuadCfg<16, 8, 8, 8, 1>; static constexpr int minb = 6; };
 template <> struct ShapeOf<kQuadWarp> { using C = QuadCfg<8, 4, 8, 6, 1>; static constexpr int minb = 16; };
 template <> struct ShapeOf<kQuadThin> { using C = QuadCfg<8, 8, 8, 4, 1>; static constexpr int minb = 10; };
+template <> struct ShapeOf<kQuadSkew> { using C = QuadCfg<16, 4, 8, 4, 1, true>; static constexpr int minb = 10; };
 
 // Box widths (elements) per shape and storage size.  fp32: BX * BY is 4, 12, 20 or
 // 28 words mod 32, so that the four row groups of a warp, 4p planes apart, fall on
 // different banks for most row distances p.
-constexpr int kQuadWidths32[kQuadShapes][2] = {{36, 52}, {28, 36}, {28, 36}};
-constexpr int kQuadWidths16[kQuadShapes][2] = {{40, 56}, {40, 56}, {40, 56}};
+constexpr int kQuadWidths32[kQuadShapes][2] = {{36, 52}, {28, 36}, {28, 36}, {36, 44}};
+constexpr int kQuadWidths16[kQuadShapes][2] = {{40, 56}, {40, 56}, {40, 56}, {40, 56}};
 
 struct QuadDims { int TU, TV, TS, BY, threads; };
 template <int SHAPE>
@@ -35,7 +38,8 @@ constexpr QuadDims dims_of() {
   using C = typename ShapeOf<SHAPE>::C;
   return QuadDims{C::TU, C::TV, C::TS, C::BY, C::threads};
 }
-constexpr QuadDims kDims[kQuadShapes] = {dims_of<kQuadWide>(), dims_of<kQuadWarp>(), dims_of<kQuadThin>()};
+constexpr QuadDims kDims[kQuadShapes] = {dims_of<kQuadWide>(), dims_of<kQuadWarp>(), dims_of<kQuadThin>(),
+                                          dims_of<kQuadSkew>()};
 
 // One box (128-byte aligned), the slabs' box origins, alignment slack.
 size_t quad_smem(const SlabBox& b, size_t es, int nsl) {
@@ -63,7 +67,8 @@ void with_quad(const cbct_plan* p, F&& f) {
   const int bx = sizeof(V) == 4 ? p->quad.bx : p->quad16.bx;
   const bool ok = p->quad_shape == kQuadWide   ? with_quad_width<V, kQuadWide>(bx, f)
                   : p->quad_shape == kQuadWarp ? with_quad_width<V, kQuadWarp>(bx, f)
-                                               : with_quad_width<V, kQuadThin>(bx, f);
+                  : p->quad_shape == kQuadThin ? with_quad_width<V, kQuadThin>(bx, f)
+                                               : with_quad_width<V, kQuadSkew>(bx, f);
   if (!ok) throw Error(CBCT_ERR_INTERNAL, "unsupported quad box width");
 }
 
@@ -148,25 +153,27 @@ void quad_tile(int shape, int& TU, int& TV) {
 }
 
 // Whether (and in which shape) the row-quad kernel projects this plan; sets its
-// boxes.  row_dz: largest distance of adjacent rows (texels).
-//  row_dz < 0.66: always (4 planes per quad).  Below 1.4 where a launch has the rays
-//  to fill the GPU for long enough, else the row-pair or slab kernel, whose threads
-//  march fewer rays one after another: from 150,000 rays up to 0.9 texel (15 views of
-//  128x96 into 64^3: 82 us against 105 with row pairs, 8 views: 70 against 59 with
-//  the slab kernel), from a million beyond (18 views of 256x192 into 128^3 at 1.09
-//  texel: 0.370 ms against 0.355; 180 views: 2.40 against 2.87).
+// boxes.  row_dz: largest distance of adjacent rows (texels).  Launches with too few
+// rays to fill the GPU run the slab kernel all the same (launch_variant).
+//  row_dz < 0.66: always (4 planes per quad).  Up to 0.9 where the largest subset has
+//  150,000 rays, up to 1.4 where it has a million: others have no launch that quads would
+//  gain on (180 views of 256x192 into 128^3 at 1.02 texel: 2.42 ms, slab kernel 2.47, row
+//  pairs 3.36; 8 views 0.22, 0.14 and 0.22).
 //  Shape: wide where its tiles are three waves and row_dz < 0.66 (20 views of 512x384
 //  into 160^3: 1.10 ms against 1.17 with the warp shape; 10 views of 192x144 into 64^3,
 //  0.3 waves: 0.139 against 0.115); warp up to 0.9 texel (25 views of 320x240 into
-//  160x144x112: 0.86 ms, wide 0.92, row pairs 1.00); thin beyond (180 views of 256x192
-//  into 128^3: 2.40 ms, warp 2.71, wide 3.69).  The next shape where boxes do not fit.
+//  160x144x112: 0.86 ms, wide 0.92, row pairs 1.00); thin to 1 texel (40 views of 360x220
+//  into 200^3 at 0.99 texel: 1.52 ms, skewed 1.66), skewed beyond (180 views of 256x192
+//  into 128^3 at 1.09 texel: 2.31 ms, thin 2.42, warp 2.71, wide 3.69).  The next shape where
+//  boxes do not fit.
 bool quad_choose(cbct_plan* p, double row_dz, bool forced) {
   const double rays = double(p->g.width) * p->g.height * p->max_subset;
   if (!forced && !(row_dz < 0.66 || (row_dz < 0.9 && rays >= 1.5e5) || (row_dz < 1.4 && rays >= 1e6))) return false;
   const QuadDims& w = kDims[kQuadWide];
   const double wide = std::ceil(p->g.width / double(w.TU)) * std::ceil(p->g.height / double(w.TV)) * p->max_subset;
-  int order[kQuadShapes] = {kQuadWide, kQuadWarp, kQuadThin};
-  if (row_dz >= 0.9) std::swap(order[0], order[2]);
+  int order[kQuadShapes] = {kQuadWide, kQuadWarp, kQuadThin, kQuadSkew};
+  if (row_dz >= 1.0) std::swap(order[0], order[3]), std::swap(order[1], order[2]);
+  else if (row_dz >= 0.9) std::swap(order[0], order[2]);
   else if (row_dz >= 0.66 || wide < 3.0 * 148 * ShapeOf<kQuadWide>::minb) std::swap(order[0], order[1]);
   for (int s : order) {
     const QuadDims& d = kDims[s];

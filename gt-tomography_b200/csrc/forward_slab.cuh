@@ -20,7 +20,7 @@
 //  * no index clamp: a slab's samples are checked at their two ends, coordinates being
 //    monotone along a ray.
 // One 256x192 view into 128^3, whole call: 107 us with 16x16 tiles, 95 once silhouette
-// rays were taken by whole warps, 47 now; 8 views of 128x96 into 64^3, the kernel alone:
+// rays were taken by whole warps, 49 now; 8 views of 128x96 into 64^3, the kernel alone:
 // 59 us before, 33 now; 32 views of 1.5 mm pixels into 128^3: 0.59 ms before, 0.43 now.
 #pragma once
 
