@@ -6,7 +6,7 @@
 // trilinear interpolation with border 0, result scaled by the sample spacing.
 // Interpolation here is FP32 in software (not 9-bit texture weights).
 //
-// Variants (all but the gather kernel give bitwise equal results):
+// Variants (all but the gather kernel give bitwise equal results over aligned rows):
 //  * fwd_slab_kernel (forward_slab.cuh): one thread per ray.  A warp marches a tile of
 //    rays of one view through the volume in slabs of a few voxels along the view's
 //    dominant in-plane axis.  Each slab's footprint (the box around the tile's ray
@@ -23,9 +23,11 @@
 //    launches that fill the GPU (quad_choose and launch_variant have the rules).
 //  * fwd_fan_kernel (opt-in): the in-plane sharing across a whole column,
 //    through shared-memory lines.
-//  * fwd_gather_kernel: the same arithmetic with bounds-checked global loads,
-//    used when the geometry does not fit the slab boxes or the volume pitch is
-//    not TMA-aligned.
+//  * fwd_gather_kernel: bounds-checked global loads, used when the geometry does not fit
+//    the slab boxes or the volume's start is not TMA-aligned.  Volumes whose rows are not
+//    a multiple of 16 bytes take the slab and quad kernels on row-padded copies, in the
+//    gather kernel's form of interpolation (LerpForm): it took those launches before, and
+//    an FP64 residual norm shows the difference of the forms.
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -958,7 +960,7 @@ void launch_fan(cbct_plan* p, const V* vol, const V* volP, const V* volT, const 
 // A volume TMA cannot read in place: rows or start off a 16-byte boundary.  The
 // TMA kernels then read a row-padded copy, made with the transposed one in one pass
 // (8 to 12 bytes per voxel, HBM-bound): 40 views of 301x211 from 150x141x93 voxels
-// take 0.97 ms, the gather kernel's bounds-checked global loads 2.36 ms.
+// take 1.03 ms, the gather kernel's bounds-checked global loads 2.36 ms.
 bool needs_padded_rows(const void* vol, int nx, size_t es) {
   return (nx * es) % 16 != 0 || reinterpret_cast<uintptr_t>(vol) % 16 != 0;
 }
@@ -1078,7 +1080,7 @@ int forward_slabs(const cbct_geometry& g, int TS) {
 // (corner-ray bounding box in the view's frame, computed in FP64): e extent
 // and z extent in elements, including margins.  False when some view cannot
 // use slabs (a ray not dominated by its view's slab axis, or too many slabs).
-bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& ext_z) {
+bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& ext_z, bool beside) {
   const cbct_geometry& g = p->g;
   const double kx = g.nx / (double)g.lx, ky = g.ny / (double)g.ly, kz = g.nz / (double)g.lz;
   const double bx = g.nx / 2.0 - 0.5, by = g.ny / 2.0 - 0.5, bz = g.nz / 2.0 - 0.5;
@@ -1140,11 +1142,12 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
           // kernels clamp footprints to the volume, whose extent bounds the box
           const int Ne = dom ? g.nx : g.ny;
           // a slab where the tile's rays are beside the volume holds no samples
-          if (emx < -1.0 || emn > Ne) continue;
+          if (!beside && (emx < -1.0 || emn > Ne)) continue;
           a.e = std::max(a.e, std::min((int)(std::floor(emx) - std::floor(emn)) + 3 + 2, Ne + 4));
           // A tile row inside the volume spans at most this in z: skip the rows
           // where none can exceed the extent found so far.
-          const double dmax = std::min(dzabs, (g.nz + 1.0 - bz) / (kz * std::max(tmn, 1e-9)));
+          const double dmax =
+              beside ? dzabs : std::min(dzabs, (g.nz + 1.0 - bz) / (kz * std::max(tmn, 1e-9)));
           if (tmn > 0 && std::ceil(kz * ((tmx - tmn) * dmax + tmx * dzspan)) + 3 + 2 <= a.z) continue;
           // One tile row; false where the rows towards the centre, whose extent is
           // smaller, cannot exceed the extent found so far.
@@ -1152,7 +1155,7 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
             const double z00 = tmn * dz0[tv], z01 = tmn * dz1[tv], z10 = tmx * dz0[tv], z11 = tmx * dz1[tv];
             const double zmn = std::min(std::min(z00, z01), std::min(z10, z11)) * kz + bz;
             const double zmx = std::max(std::max(z00, z01), std::max(z10, z11)) * kz + bz;
-            if (zmx < -1.0 || zmn > g.nz) return true;
+            if (!beside && (zmx < -1.0 || zmn > g.nz)) return true;
             if (std::ceil(zmx - zmn) + 3 + 2 <= a.z) return false;
             const int ez = (int)(std::floor(zmx) - std::floor(zmn)) + 3 + 2;
             a.z = std::max(a.z, std::min(ez, g.nz + 4));
@@ -1179,6 +1182,51 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
     ok = ok && a.ok;
   }
   return ok;
+}
+
+// Whether the detector's pixels are so wide that a box of 16 x 16 rays and kTS voxels,
+// two of them a CTA, has no room in shared memory anywhere along the rays.  A bound of
+// its extents from each view's outer columns settles it for all but such detectors.
+static bool wide_pixels(const cbct_plan* p) {
+  const cbct_geometry& g = p->g;
+  const double kx = g.nx / (double)g.lx, ky = g.ny / (double)g.ly, kz = g.nz / (double)g.lz;
+  auto fits = [](int e, int z) {
+    int w32 = 0, w16 = 0;
+    for (int w : kBoxWidths) {
+      if (!w32 && w >= e + 3) w32 = w;
+      if (!w16 && w >= e + 7) w16 = w;
+    }
+    auto smem = [&](int w, int es) { return kNStage * (((size_t)w * kBoxY * z * es + 127) & ~size_t(127)) + 128; };
+    return w32 && w16 && z <= 256 && smem(w32, 4) <= (size_t)kSmemBudget && smem(w16, 2) <= (size_t)kSmemBudget;
+  };
+  double be = 0, bz = 0;
+  for (int iv = 0; iv < p->n_views; ++iv) {
+    const ViewParams& vp = p->hviews[iv];
+    const bool dom = vp.dom;
+    const int Nd = dom ? g.ny : g.nx;
+    const double ke = dom ? kx : ky, kd = dom ? ky : kx, Sd = dom ? vp.Sy : vp.Sx;
+    const double Ee = dom ? vp.Eux : vp.Euy, Ed = dom ? vp.Euy : vp.Eux;
+    const double D0e = dom ? vp.D0x : vp.D0y, D0d = dom ? vp.D0y : vp.D0x;
+    // depth of the farthest slab plane from the source, least depth of a ray at t = 1
+    const double depth = std::fabs(Sd) + (0.5 * Nd + 2.0 * kTS + 2.0) / kd;
+    double dd = 1e30, slope = 0;
+    for (double u : {0.0, g.width - 1.0}) {
+      dd = std::min(dd, std::fabs(D0d + u * Ed));
+      slope = std::max(slope, std::fabs((D0e + u * Ee) / (D0d + u * Ed)));
+    }
+    const double dz = std::max(std::fabs((double)vp.D0z), std::fabs(vp.D0z + (g.height - 1.0) * vp.Evz));
+    be = std::max(be, kTS * slope * ke / kd + depth * ke * (kTU - 1) * std::fabs(Ee * D0d - D0e * Ed) / (dd * dd));
+    bz = std::max(bz, kz * ((kTS / kd / dd + depth * (kTU - 1) * std::fabs(Ed) / (dd * dd)) * dz +
+                            depth / dd * (kTV - 1) * std::fabs((double)vp.Evz)));
+  }
+  auto ext = [](double span, int n) { return int(std::min(std::ceil(std::min(span, 1e6)) + 3 + 2, n + 4.0)); };
+  if (fits(ext(be, std::max(g.nx, g.ny)), std::max(ext(bz, g.nz), 2))) return false;
+  int e, z;
+  return slab_extents(p, kTU, kTV, kTS, e, z, true) && !fits(e, std::max(z, 2));
+}
+
+bool forward_lerp_gather(const cbct_plan* p, size_t es) {
+  return p->fwd_wide || ((size_t)p->g.nx * es) % 16 != 0 || ((size_t)p->g.ny * es) % 16 != 0;
 }
 
 // Largest z distance (texels) between the rays of adjacent detector rows at a
@@ -1214,7 +1262,9 @@ void forward_choose_variant(cbct_plan* p) {
   for (size_t s = 0; s < p->first.size(); ++s)
     for (int i = p->first[s]; i < p->first[s] + p->count[s]; ++i)
       if (p->hviews[i].dom == 0) p->subset_has_xdom[s] = 1;
+  p->fwd_wide = 0;
   if (p->force_gather || p->fwd_pref == 2) return;
+  p->fwd_wide = wide_pixels(p);   // off again for a forced kernel of another form
   // The x start of a box is rounded down to a 16-byte boundary (4 fp32 or 8
   // 16-bit elements), which widens the box by up to 3 or 7 elements.
   auto width = [](const auto& list, int ext, int slack) {
@@ -1228,6 +1278,7 @@ void forward_choose_variant(cbct_plan* p) {
   if ((p->fwd_pref == 0 || p->fwd_pref == 5) && quad_choose(p, row_dz, p->fwd_pref == 5)) {
     p->fwd_variant = 4;
     if (p->fwd_pref == 0) slab_choose(p);
+    else p->fwd_wide = 0;
     return;
   }
   int e, z;
@@ -1243,6 +1294,7 @@ void forward_choose_variant(cbct_plan* p) {
       p->pair = b32;
       p->pair16 = b16;
       p->fwd_variant = 3;
+      if (p->fwd_pref == 4) p->fwd_wide = 0;
     }
   }
   if (p->fwd_pref == 3 && slab_extents(p, kFU, kFV, kTS, e, z)) {
@@ -1257,6 +1309,7 @@ void forward_choose_variant(cbct_plan* p) {
       p->fan16 = b16;
       p->fan_lz = lz;
       p->fwd_variant = 2;
+      p->fwd_wide = 0;
     }
   }
 }
@@ -1282,6 +1335,8 @@ static int launch_variant(const cbct_plan* p, int cnt, size_t es) {
   const double rays = double(p->g.width) * p->g.height * cnt;
   if (rows && p->fwd_pref == 0 && p->slab.bx && (rays < p->fwd_fill_rays || p->fwd_row_dz >= (es == 2 ? 1.0 : 1.2)))
     return 1;
+  // The gather form is compiled for the slab and quad kernels.
+  if (forward_lerp_gather(p, es) && (p->fwd_variant == 2 || p->fwd_variant == 3)) return p->slab.bx ? 1 : 0;
   return p->fwd_variant;
 }
 
@@ -1419,7 +1474,7 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
     cbct_plan* p = j.p;
     const int s = j.s, first = p->first[s], cnt = p->count[s];
     if (cnt == 0) continue;
-    const bool tma = p->fwd_variant >= 1 && ((size_t)p->g.nx * 4) % 16 == 0 && ((size_t)p->g.ny * 4) % 16 == 0 &&
+    const bool tma = p->fwd_variant >= 1 && !forward_lerp_gather(p, sizeof(float)) &&
                      (reinterpret_cast<uintptr_t>(j.vol) % 16 == 0) && (!p->subset_has_xdom[s] || p->d_volT);
     int fv = launch_variant(p, cnt, sizeof(float));
     if (fv == 1 && p->fwd_variant == 4 && p->fwd_pref == 0 && !j.norm2_out && all_rays >= kMultiQuadRays &&

@@ -24,8 +24,14 @@ struct alignas(128) FwdScanRec {
 CUtensorMap make_volume_map(cbct_dtype dt, const void* vol, int n0, int n1, int n2, const SlabBox& b);
 
 // Largest footprint of a slab of TS voxels over every view and tile of a TU x TV
-// tiling, margins included; false when some view cannot use slabs.
-bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& ext_z);
+// tiling, margins included; false when some view cannot use slabs.  beside: also over
+// tiles and slabs whose rays pass beside the volume.
+bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& ext_z, bool beside = false);
+
+// Whether launches of element size es interpolate in the gather kernel's form (see
+// LerpForm): the plan's rows or pixels are such that the gather kernel is the one that
+// reads the caller's volume as it lies.
+bool forward_lerp_gather(const cbct_plan* p, size_t es);
 
 // Slabs of TS voxels a ray can cross in the larger in-plane direction.
 int forward_slabs(const cbct_geometry& g, int TS);

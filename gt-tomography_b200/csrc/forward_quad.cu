@@ -10,28 +10,6 @@ namespace cbct {
 
 namespace {
 
-// Shapes, in the order of QuadShape.  The minimum CTAs per SM set the register
-// budget (80, 128, 96 and 96 registers).
-//  wide : 16 x 32 tiles of 128 threads, slabs of 8 voxels.  Fewest instructions per
-//         sample; its boxes fit six CTAs per SM where rows are under 2/3 texel apart.
-//  warp : one warp per CTA (8 x 16 rays), slabs of 6.  Twice the box bytes per ray,
-//         but no warp waits for another and the last wave is short.
-//  thin : 8 x 32 tiles of 64 threads, slabs of 4, for boxes that are large because
-//         a detector pixel is about a voxel.
-//  skew : 16 x 16 tiles of 64 threads, slabs of 4, for rows a texel or more apart
-//         (see QuadCfg).
-template <int SHAPE> struct ShapeOf;
-template <> struct ShapeOf<kQuadWide> { using C = QuadCfg<16, 8, 8, 8, 1>; static constexpr int minb = 6; };
-template <> struct ShapeOf<kQuadWarp> { using C = QuadCfg<8, 4, 8, 6, 1>; static constexpr int minb = 16; };
-template <> struct ShapeOf<kQuadThin> { using C = QuadCfg<8, 8, 8, 4, 1>; static constexpr int minb = 10; };
-template <> struct ShapeOf<kQuadSkew> { using C = QuadCfg<16, 4, 8, 4, 1, true>; static constexpr int minb = 10; };
-
-// Box widths (elements) per shape and storage size.  fp32: BX * BY is 4, 12, 20 or
-// 28 words mod 32, so that the four row groups of a warp, 4p planes apart, fall on
-// different banks for most row distances p.
-constexpr int kQuadWidths32[kQuadShapes][2] = {{36, 52}, {28, 36}, {28, 36}, {36, 44}};
-constexpr int kQuadWidths16[kQuadShapes][2] = {{40, 56}, {40, 56}, {40, 56}, {40, 56}};
-
 struct QuadDims { int TU, TV, TS, BY, threads; };
 template <int SHAPE>
 constexpr QuadDims dims_of() {
@@ -46,39 +24,19 @@ size_t quad_smem(const SlabBox& b, size_t es, int nsl) {
   return ((b.bx * b.by * b.bz * es + 127) & ~size_t(127)) + sizeof(int2) * (size_t)nsl + 128;
 }
 
-template <class V, int BX, int SHAPE>
-auto quad_kernel() {
-  return fwd_quad_kernel<V, BX, typename ShapeOf<SHAPE>::C, ShapeOf<SHAPE>::minb>;
-}
-
-// Calls f(std::integral_constant<int, BX>, std::integral_constant<int, SHAPE>) for
-// the compiled shape and width.
-template <class V, int SHAPE, class F>
-bool with_quad_width(int bx, F&& f) {
-  constexpr const int(&w)[2] = sizeof(V) == 4 ? kQuadWidths32[SHAPE] : kQuadWidths16[SHAPE];
-  if (bx == w[0]) f(std::integral_constant<int, w[0]>{}, std::integral_constant<int, SHAPE>{});
-  else if (bx == w[1]) f(std::integral_constant<int, w[1]>{}, std::integral_constant<int, SHAPE>{});
-  else return false;
-  return true;
-}
-
-template <class V, class F>
-void with_quad(const cbct_plan* p, F&& f) {
-  const int bx = sizeof(V) == 4 ? p->quad.bx : p->quad16.bx;
-  const bool ok = p->quad_shape == kQuadWide   ? with_quad_width<V, kQuadWide>(bx, f)
-                  : p->quad_shape == kQuadWarp ? with_quad_width<V, kQuadWarp>(bx, f)
-                  : p->quad_shape == kQuadThin ? with_quad_width<V, kQuadThin>(bx, f)
-                                               : with_quad_width<V, kQuadSkew>(bx, f);
-  if (!ok) throw Error(CBCT_ERR_INTERNAL, "unsupported quad box width");
+template <class V>
+QuadKernel<V> quad_kernel(const cbct_plan* p) {
+  if (forward_lerp_gather(p, sizeof(V))) return quad_kernel_gather<V>(p);
+  QuadKernel<V> k = nullptr;
+  with_quad<V>(p, [&](auto BX, auto SHAPE) { k = quad_kernel_of<V, decltype(BX)::value, decltype(SHAPE)::value, false>(); });
+  return k;
 }
 
 template <class V>
 void prepare_typed(const cbct_plan* p) {
   const SlabBox& b = sizeof(V) == 4 ? p->quad : p->quad16;
   const size_t smem = quad_smem(b, sizeof(V), forward_slabs(p->g, kDims[p->quad_shape].TS));
-  with_quad<V>(p, [&](auto BX, auto SHAPE) {
-    ensure_smem_attr((const void*)quad_kernel<V, decltype(BX)::value, decltype(SHAPE)::value>(), smem);
-  });
+  ensure_smem_attr((const void*)quad_kernel<V>(p), smem);
 }
 
 template <class V>
@@ -91,11 +49,9 @@ void launch_typed(cbct_plan* p, const V* vol, const V* volP, const V* volT, cons
   const int nsl = forward_slabs(p->g, d.TS);
   const size_t smem = quad_smem(b, sizeof(V), nsl);
   const dim3 grid((p->g.width + d.TU - 1) / d.TU, (p->g.height + d.TV - 1) / d.TV, cnt);
-  with_quad<V>(p, [&](auto BX, auto SHAPE) {
-    auto k = quad_kernel<V, decltype(BX)::value, decltype(SHAPE)::value>();
-    ensure_smem_attr((const void*)k, smem);
-    k<<<grid, d.threads, smem, st>>>(mv, mt, vol, p->d_views + first, p->gc, b.bz, nsl, p->debug_checks, o, p->d_flags);
-  });
+  const QuadKernel<V> k = quad_kernel<V>(p);
+  ensure_smem_attr((const void*)k, smem);
+  k<<<grid, d.threads, smem, st>>>(mv, mt, vol, p->d_views + first, p->gc, b.bz, nsl, p->debug_checks, o, p->d_flags);
   check_launch("fwd_quad_kernel");
 }
 
@@ -132,7 +88,7 @@ __global__ void __launch_bounds__(ShapeOf<SHAPE>::C::threads, ShapeOf<SHAPE>::mi
       tensormap_acquire(&R.map_t);
       last = lo;
     }
-    fwd_quad_body<float, BX, C>(&R.map_v, &R.map_t, static_cast<const float*>(R.vol), R.views, R.gc, R.BZ, R.nsl_max,
+    fwd_quad_body<float, BX, C, false>(&R.map_v, &R.map_t, static_cast<const float*>(R.vol), R.views, R.gc, R.BZ, R.nsl_max,
                                 false, R.o, R.flags, tile, smem_raw, sh);
     __syncthreads();
     // A wait that gave up is counted in the scan's flag word and its loads

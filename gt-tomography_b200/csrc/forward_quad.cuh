@@ -35,7 +35,7 @@
 //    3.13 ms instead of 2.44).
 #pragma once
 
-#include "forward_device.cuh"
+#include "forward_host.h"
 
 namespace cbct {
 
@@ -72,16 +72,24 @@ struct QuadShared {
   double red[8];
 };
 
-// One plane at q: the same operations, the two e interpolations packed.
-template <class V, int BX>
+// One plane at q: the same operations, the first two interpolations packed.
+template <class V, int BX, int FORM>
 __device__ __forceinline__ float plane1(const V* __restrict__ q, float2 te, float2 nte, float2 td, float2 ntd) {
   const float2 a = make_float2(sm_f(q[0]), sm_f(q[BX])), b = make_float2(sm_f(q[1]), sm_f(q[BX + 1]));
+  if (FORM == kLerpXisE) {
+    const float2 x = lerp2_gather(a, b, te);
+    return fmaf(td.x, x.y - x.x, x.x);
+  }
+  if (FORM == kLerpXisD) {
+    const float2 x = lerp2_gather(make_float2(a.x, b.x), make_float2(a.y, b.y), td);
+    return fmaf(te.x, x.y - x.x, x.x);
+  }
   const float2 e = __ffma2_rn(te, b, __ffma2_rn(nte, a, a));
   return fmaf(td.x, e.y, fmaf(ntd.x, e.x, e.x));
 }
 
 // Samples k .. ke-1 of four rows at any distance: two planes per row.
-template <class V, int BX, int BY>
+template <class V, int BX, int BY, int FORM>
 __device__ __forceinline__ void quad_march_any(const V* __restrict__ s, float k, float ke, float2 c0, float2 dc,
                                                const float2 (&z0)[2], const float2 (&dz)[2], float cmo,
                                                float2 (&acc)[2]) {
@@ -101,15 +109,15 @@ __device__ __forceinline__ void quad_march_any(const V* __restrict__ s, float k,
       const float2 ix = __ffma2_rn(fz, make_float2(float(BXY), float(BXY)), make_float2(cb, cb));
       const V* q0 = s + (unsigned)int_of_biased(ix.x);
       const V* q1 = s + (unsigned)int_of_biased(ix.y);
-      const float2 lo = planes2<V, BX>(q0, q1, te, nte, td, ntd);
-      const float2 hi = planes2<V, BX>(q0 + BXY, q1 + BXY, te, nte, td, ntd);
+      const float2 lo = planes2<V, BX, FORM>(q0, q1, te, nte, td, ntd);
+      const float2 hi = planes2<V, BX, FORM>(q0 + BXY, q1 + BXY, te, nte, td, ntd);
       acc[j] = __fadd2_rn(acc[j], __ffma2_rn(sub2(cz, fz), sub2(hi, lo), lo));
     }
   }
 }
 
 // Samples k .. ke-1 of one ray.
-template <class V, int BX, int BY>
+template <class V, int BX, int BY, int FORM>
 __device__ __forceinline__ void ray_march(const V* __restrict__ s, float k, float ke, float2 c0, float2 dc, float z0,
                                           float dz, float cmo, float& acc) {
   constexpr int BXY = BX * BY;
@@ -118,7 +126,7 @@ __device__ __forceinline__ void ray_march(const V* __restrict__ s, float k, floa
     const float fe = floor_small(ce), fd = floor_small(cd), fz = floor_small(cz);
     const float te = ce - fe, td = cd - fd;
     const V* b = s + (unsigned)int_of_biased(fmaf(fz, float(BXY), fmaf(fd, float(BX), fe)) + cmo);
-    const float2 l = planes2<V, BX>(b, b + BXY, make_float2(te, te), make_float2(-te, -te), make_float2(td, td),
+    const float2 l = planes2<V, BX, FORM>(b, b + BXY, make_float2(te, te), make_float2(-te, -te), make_float2(td, td),
                                     make_float2(-td, -td));
     return fmaf(cz - fz, l.y - l.x, l.x);
   };
@@ -134,7 +142,7 @@ __device__ __forceinline__ void ray_march(const V* __restrict__ s, float k, floa
 // to the lowest row's plane f0, row i's lower plane is Ci or Ci + 1 at every
 // sample (the caller checked the row distance at both ends, and z >= 0).  s is the
 // box's address minus its origin's element index.
-template <class V, int BX, int BY, int C1, int C2, int C3>
+template <class V, int BX, int BY, int FORM, int C1, int C2, int C3>
 __device__ __forceinline__ void quad_march(const V* __restrict__ s, float k, float ke, float2 c0, float2 dc,
                                            const float2 (&z0)[2], const float2 (&dz)[2], float2 (&acc)[2]) {
   constexpr int BXY = BX * BY, NP = C3 + 3;
@@ -167,11 +175,11 @@ __device__ __forceinline__ void quad_march(const V* __restrict__ s, float k, flo
     const float2 te2 = make_float2(te, te), nte2 = make_float2(-te, -te), td2 = make_float2(td, td), ntd2 = make_float2(-td, -td);
 #pragma unroll
     for (int j = 0; j + 1 < NP; j += 2) {
-      const float2 l = planes2<V, BX>(q + j * BXY, q + (j + 1) * BXY, te2, nte2, td2, ntd2);
+      const float2 l = planes2<V, BX, FORM>(q + j * BXY, q + (j + 1) * BXY, te2, nte2, td2, ntd2);
       L[j] = l.x;
       L[j + 1] = l.y;
     }
-    if (NP & 1) L[NP - 1] = plane1<V, BX>(q + (NP - 1) * BXY, te2, nte2, td2, ntd2);
+    if (NP & 1) L[NP - 1] = plane1<V, BX, FORM>(q + (NP - 1) * BXY, te2, nte2, td2, ntd2);
 #pragma unroll
     for (int j = 0; j + 1 < NP; ++j) g[j] = L[j + 1] - L[j];
     const float2 a0 = __fadd2_rn(zz0, make_float2(nf0, nf0 - float(C1)));
@@ -205,8 +213,9 @@ struct OwnRay {
   float z0, dz;
 };
 
-// One CTA: ray tile `tile` of the call.
-template <class V, int BX, class C>
+// One CTA: ray tile `tile` of the call.  GATHER: the gather kernel's
+// interpolation (see LerpForm).
+template <class V, int BX, class C, bool GATHER>
 __device__ __forceinline__ void fwd_quad_body(const CUtensorMap* map_v, const CUtensorMap* map_t,
                                               const V* __restrict__ vol, const ViewParams* __restrict__ views,
                                               const GridConst& gc, int BZ, int nsl_max, bool check, const FwdOut& o,
@@ -389,14 +398,18 @@ __device__ __forceinline__ void fwd_quad_body(const CUtensorMap* map_v, const CU
         if (!inside(fmaf(k, dc.x, c0.x), fmaf(kl, dc.x, c0.x), zmin, zmax + 1.f)) {
           bad = 1;
         } else {
-          switch (zmin >= 0.f ? quad_class(smin, smax) : -1) {
-            case 0: quad_march<V, BX, BY, 0, 0, 0>(so, k, ke, c0, dc, z0, dz, acc); break;
-            case 1: quad_march<V, BX, BY, 0, 0, 1>(so, k, ke, c0, dc, z0, dz, acc); break;
-            case 2: quad_march<V, BX, BY, 0, 1, 1>(so, k, ke, c0, dc, z0, dz, acc); break;
-            case 3: quad_march<V, BX, BY, 0, 1, 2>(so, k, ke, c0, dc, z0, dz, acc); break;
-            case 4: quad_march<V, BX, BY, 1, 2, 3>(so, k, ke, c0, dc, z0, dz, acc); break;
-            default: quad_march_any<V, BX, BY>(s, k, ke, c0, dc, z0, dz, cmo, acc); break;
-          }
+          const int cls = zmin >= 0.f ? quad_class(smin, smax) : -1;
+          with_form<GATHER>(dom, [&](auto form) {
+            constexpr int F = decltype(form)::value;
+            switch (cls) {
+              case 0: quad_march<V, BX, BY, F, 0, 0, 0>(so, k, ke, c0, dc, z0, dz, acc); break;
+              case 1: quad_march<V, BX, BY, F, 0, 0, 1>(so, k, ke, c0, dc, z0, dz, acc); break;
+              case 2: quad_march<V, BX, BY, F, 0, 1, 1>(so, k, ke, c0, dc, z0, dz, acc); break;
+              case 3: quad_march<V, BX, BY, F, 0, 1, 2>(so, k, ke, c0, dc, z0, dz, acc); break;
+              case 4: quad_march<V, BX, BY, F, 1, 2, 3>(so, k, ke, c0, dc, z0, dz, acc); break;
+              default: quad_march_any<V, BX, BY, F>(s, k, ke, c0, dc, z0, dz, cmo, acc); break;
+            }
+          });
         }
       }
       kf = ke;
@@ -407,8 +420,12 @@ __device__ __forceinline__ void fwd_quad_body(const CUtensorMap* map_v, const CU
       const float k = r.k, ke = slab_end(k, Nf, r.c.y, r.d.y, up, lo, hi);
       if (ke > k) {
         const float kl = ke - 1.f, za = fmaf(k, r.dz, r.z0), zb = fmaf(kl, r.dz, r.z0);
-        if (!inside(fmaf(k, r.d.x, r.c.x), fmaf(kl, r.d.x, r.c.x), fminf(za, zb), fmaxf(za, zb))) bad = 1;
-        else ray_march<V, BX, BY>(s, k, ke, r.c, r.d, r.z0, r.dz, cmo, r.acc);
+        if (!inside(fmaf(k, r.d.x, r.c.x), fmaf(kl, r.d.x, r.c.x), fminf(za, zb), fmaxf(za, zb)))
+          bad = 1;
+        else
+          with_form<GATHER>(dom, [&](auto form) {
+            ray_march<V, BX, BY, decltype(form)::value>(s, k, ke, r.c, r.d, r.z0, r.dz, cmo, r.acc);
+          });
         r.k = ke;
       }
     }
@@ -456,7 +473,7 @@ __device__ __forceinline__ void fwd_quad_body(const CUtensorMap* map_v, const CU
   fwd_block_partial(o, sq, sh.red, tid, tile.bid);
 }
 
-template <class V, int BX, class C, int MINB>
+template <class V, int BX, class C, int MINB, bool GATHER>
 __global__ void __launch_bounds__(C::threads, MINB)
     fwd_quad_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_t,
                     const V* __restrict__ vol, const ViewParams* __restrict__ views, GridConst gc, int BZ,
@@ -465,10 +482,70 @@ __global__ void __launch_bounds__(C::threads, MINB)
   unsigned char* smem_raw =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
   __shared__ QuadShared<C::NS> sh;
-  fwd_quad_body<V, BX, C>(&map_v, &map_t, vol, views, gc, BZ, nsl_max, check != 0, o, flags, launch_tile(), smem_raw,
+  fwd_quad_body<V, BX, C, GATHER>(&map_v, &map_t, vol, views, gc, BZ, nsl_max, check != 0, o, flags, launch_tile(), smem_raw,
                           sh);
 }
 
+// ------------------------------------------------------------------ shapes
+template <class V>
+using QuadKernel = void (*)(const CUtensorMap, const CUtensorMap, const V*, const ViewParams*, GridConst, int, int, int,
+                            FwdOut, int*);
+
+// Shapes, in the order of QuadShape.  The minimum CTAs per SM set the register
+// budget (80, 128, 96 and 96 registers).
+//  wide : 16 x 32 tiles of 128 threads, slabs of 8 voxels.  Fewest instructions per
+//         sample; its boxes fit six CTAs per SM where rows are under 2/3 texel apart.
+//  warp : one warp per CTA (8 x 16 rays), slabs of 6.  Twice the box bytes per ray,
+//         but no warp waits for another and the last wave is short.
+//  thin : 8 x 32 tiles of 64 threads, slabs of 4, for boxes that are large because
+//         a detector pixel is about a voxel.
+//  skew : 16 x 16 tiles of 64 threads, slabs of 4, for rows a texel or more apart
+//         (see QuadCfg).
+template <int SHAPE> struct ShapeOf;
+template <> struct ShapeOf<kQuadWide> { using C = QuadCfg<16, 8, 8, 8, 1>; static constexpr int minb = 6; };
+template <> struct ShapeOf<kQuadWarp> { using C = QuadCfg<8, 4, 8, 6, 1>; static constexpr int minb = 16; };
+template <> struct ShapeOf<kQuadThin> { using C = QuadCfg<8, 8, 8, 4, 1>; static constexpr int minb = 10; };
+template <> struct ShapeOf<kQuadSkew> { using C = QuadCfg<16, 4, 8, 4, 1, true>; static constexpr int minb = 10; };
+
+// Box widths (elements) per shape and storage size.  fp32: BX * BY is 4, 12, 20 or
+// 28 words mod 32, so that the four row groups of a warp, 4p planes apart, fall on
+// different banks for most row distances p.
+constexpr int kQuadWidths32[kQuadShapes][2] = {{36, 52}, {28, 36}, {28, 36}, {36, 44}};
+constexpr int kQuadWidths16[kQuadShapes][2] = {{40, 56}, {40, 56}, {40, 56}, {40, 56}};
+
+template <class V, int BX, int SHAPE, bool GATHER>
+QuadKernel<V> quad_kernel_of() {
+  return fwd_quad_kernel<V, BX, typename ShapeOf<SHAPE>::C, ShapeOf<SHAPE>::minb, GATHER>;
+}
+
+// Calls f(std::integral_constant<int, BX>, std::integral_constant<int, SHAPE>) for
+// the compiled shape and width.
+template <class V, int SHAPE, class F>
+bool with_quad_width(int bx, F&& f) {
+  constexpr const int(&w)[2] = sizeof(V) == 4 ? kQuadWidths32[SHAPE] : kQuadWidths16[SHAPE];
+  if (bx == w[0]) f(std::integral_constant<int, w[0]>{}, std::integral_constant<int, SHAPE>{});
+  else if (bx == w[1]) f(std::integral_constant<int, w[1]>{}, std::integral_constant<int, SHAPE>{});
+  else return false;
+  return true;
+}
+
+// Calls f(std::integral_constant<int, BX>, std::integral_constant<int, SHAPE>) for
+// the plan's shape and box width.
+template <class V, class F>
+void with_quad(const cbct_plan* p, F&& f) {
+  const int bx = sizeof(V) == 4 ? p->quad.bx : p->quad16.bx;
+  const bool ok = p->quad_shape == kQuadWide   ? with_quad_width<V, kQuadWide>(bx, f)
+                  : p->quad_shape == kQuadWarp ? with_quad_width<V, kQuadWarp>(bx, f)
+                  : p->quad_shape == kQuadThin ? with_quad_width<V, kQuadThin>(bx, f)
+                                               : with_quad_width<V, kQuadSkew>(bx, f);
+  if (!ok) throw Error(CBCT_ERR_INTERNAL, "unsupported quad box width");
+}
+
 }  // namespace
+
+// The plan's kernel in the gather form (forward_quad_gather.cu, a file of its own to
+// compile beside this one).
+template <class V>
+QuadKernel<V> quad_kernel_gather(const cbct_plan* p);
 
 }  // namespace cbct

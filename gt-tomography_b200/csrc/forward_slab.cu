@@ -39,7 +39,11 @@ template <class V>
 void prepare_typed(const cbct_plan* p) {
   const SlabBox& b = box_of<V>(p);
   const size_t smem = slab_smem(b, sizeof(V), forward_slabs(p->g, kSlabTS));
-  with_slab<V>(b.bx, [&](auto BX) { ensure_smem_attr((const void*)fwd_slab_kernel<V, decltype(BX)::value>, smem); });
+  with_slab<V>(b.bx, [&](auto BX) {
+    ensure_smem_attr(forward_lerp_gather(p, sizeof(V)) ? (const void*)fwd_slab_kernel<V, decltype(BX)::value, true>
+                                                       : (const void*)fwd_slab_kernel<V, decltype(BX)::value, false>,
+                     smem);
+  });
 }
 
 template <class V>
@@ -52,7 +56,8 @@ void launch_typed(cbct_plan* p, const V* vol, const V* volP, const V* volT, cons
   const size_t smem = slab_smem(b, sizeof(V), nsl);
   const dim3 grid((p->g.width + kSlabU - 1) / kSlabU, (p->g.height + kSlabV - 1) / kSlabV, cnt);
   with_slab<V>(b.bx, [&](auto BX) {
-    auto k = fwd_slab_kernel<V, decltype(BX)::value>;
+    auto k = forward_lerp_gather(p, sizeof(V)) ? fwd_slab_kernel<V, decltype(BX)::value, true>
+                                               : fwd_slab_kernel<V, decltype(BX)::value, false>;
     ensure_smem_attr((const void*)k, smem);
     k<<<grid, kSlabThreads, smem, st>>>(mv, mt, vol, p->d_views + first, p->gc, b.bz, nsl, p->debug_checks, o,
                                         p->d_flags);
@@ -92,7 +97,7 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabMinb)
       tensormap_acquire(&R.map_t);
       last = lo;
     }
-    fwd_slab_body<float, BX>(&R.map_v, &R.map_t, static_cast<const float*>(R.vol), R.views, R.gc, R.BZ, R.nsl_max,
+    fwd_slab_body<float, BX, false>(&R.map_v, &R.map_t, static_cast<const float*>(R.vol), R.views, R.gc, R.BZ, R.nsl_max,
                              false, R.o, R.flags, tile, smem_raw, sh);
     __syncthreads();
     // A wait that gave up is counted in the scan's flag word and its loads

@@ -165,7 +165,7 @@ __device__ __forceinline__ void deal_long_runs(float& k, float ke, float2 c0, fl
 }
 
 // Samples k .. ke-1 of one ray (all lanes of the warp call it; k == ke: none).
-template <class V, int BX, int BY>
+template <class V, int BX, int BY, int FORM>
 __device__ __forceinline__ void slab_march(const V* __restrict__ s, float k, float ke, float2 c0, float2 dc, float z0,
                                            float dz, float cmo, float& acc) {
   constexpr int BXY = BX * BY, U = kSlabUnroll;
@@ -176,7 +176,7 @@ __device__ __forceinline__ void slab_march(const V* __restrict__ s, float k, flo
     const float fz = floor_small(cz);
     const float2 t = sub2(pq, f);
     const V* b = s + (unsigned)int_of_biased(fmaf(fz, float(BXY), fmaf(f.y, float(BX), f.x)) + cmo);
-    const float2 l = planes2<V, BX>(b, b + BXY, make_float2(t.x, t.x), make_float2(-t.x, -t.x),
+    const float2 l = planes2<V, BX, FORM>(b, b + BXY, make_float2(t.x, t.x), make_float2(-t.x, -t.x),
                                     make_float2(t.y, t.y), make_float2(-t.y, -t.y));
     return fmaf(cz - fz, l.y - l.x, l.x);
   };
@@ -192,8 +192,9 @@ __device__ __forceinline__ void slab_march(const V* __restrict__ s, float k, flo
 }
 
 // One CTA: ray tile `tile` of the call.  smem_raw is the 128-byte aligned dynamic
-// shared memory: per warp a box and the slabs' box origins.
-template <class V, int BX>
+// shared memory: per warp a box and the slabs' box origins.  GATHER: the
+// gather kernel's interpolation (see LerpForm).
+template <class V, int BX, bool GATHER>
 __device__ __forceinline__ void fwd_slab_body(const CUtensorMap* map_v, const CUtensorMap* map_t,
                                               const V* __restrict__ vol, const ViewParams* __restrict__ views,
                                               const GridConst& gc, int BZ, int nsl_max, bool check,
@@ -313,7 +314,10 @@ __device__ __forceinline__ void fwd_slab_body(const CUtensorMap* map_v, const CU
             fmaxf(za, zb) < float(oz + BZ - 1);
       bad |= !run;
     }
-    slab_march<V, BX, BY>(s, run ? kf : ke, ke, c0, dc, r.c0z, r.dcz, kRoundC - float(oe + od * BX + oz * BXY), acc);
+    const float cmo = kRoundC - float(oe + od * BX + oz * BXY);
+    with_form<GATHER>(dom, [&](auto form) {
+      slab_march<V, BX, BY, decltype(form)::value>(s, run ? kf : ke, ke, c0, dc, r.c0z, r.dcz, cmo, acc);
+    });
     kf = ke;
     __syncwarp();
     if (lane == 0 && i + 1 < nslab) {
@@ -329,7 +333,7 @@ __device__ __forceinline__ void fwd_slab_body(const CUtensorMap* map_v, const CU
   fwd_epilogue(o, gc, vp, tile.z, u, v, active, val, sh.red, tid, tile.bid);
 }
 
-template <class V, int BX>
+template <class V, int BX, bool GATHER>
 __global__ void __launch_bounds__(kSlabThreads, kSlabMinb)
     fwd_slab_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_t,
                     const V* __restrict__ vol, const ViewParams* __restrict__ views, GridConst gc, int BZ,
@@ -338,7 +342,7 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabMinb)
   unsigned char* smem_raw =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
   __shared__ SlabShared sh;
-  fwd_slab_body<V, BX>(&map_v, &map_t, vol, views, gc, BZ, nsl_max, check != 0, o, flags, launch_tile(),
+  fwd_slab_body<V, BX, GATHER>(&map_v, &map_t, vol, views, gc, BZ, nsl_max, check != 0, o, flags, launch_tile(),
                        smem_raw, sh);
 }
 

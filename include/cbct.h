@@ -163,7 +163,10 @@ CBCT_API cbct_status cbct_plan_autotune(cbct_plan* plan, float* times_ms_out, vo
  * rays of a detector column; slower on B200 at the sizes measured so far), 4 = the
  * row-pair kernel (one thread marches two vertically adjacent rays of a column and
  * shares their in-plane interpolation), 5 = the row-quad kernel (four rows per
- * thread).  Slab, fan, row-pair and row-quad results are bitwise equal. */
+ * thread).  Slab, fan, row-pair and row-quad results are bitwise equal.  Volumes with
+ * rows of no multiple of 16 bytes (nx or ny), and pixels of several voxels, are projected
+ * by the slab or quad kernel in the gather kernel's form: bitwise its results for rays
+ * through the volume; a forced pair or fan kernel becomes the slab kernel there. */
 #define CBCT_OPT_FORWARD_KERNEL 3
 /* CBCT_OPT_WAIT_LIMIT: polls (>= 0) a TMA-staged projector kernel spends
  * waiting for its next shared-memory stage before it gives up (default
