@@ -2,6 +2,8 @@
 // translation units.
 #pragma once
 
+#include <algorithm>
+
 #include "forward_device.cuh"
 
 namespace cbct {
@@ -32,6 +34,13 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
 // LerpForm): the plan's rows or pixels are such that the gather kernel is the one that
 // reads the caller's volume as it lies.
 bool forward_lerp_gather(const cbct_plan* p, size_t es);
+
+// Bound of a sample's element index counted from the volume's corner with box b's strides.
+// Kernels form it as an exact FP32 sum: below 2^24, or below 2^22 in the mantissa of a
+// sum biased by 1.5 * 2^23 whose box origin is taken off afterwards.
+inline size_t box_index_bound(const cbct_geometry& g, const SlabBox& b) {
+  return ((size_t)g.nz + 1) * b.bx * b.by + ((size_t)std::max(g.nx, g.ny) + 1) * (b.bx + 1);
+}
 
 // Slabs of TS voxels a ray can cross in the larger in-plane direction.
 int forward_slabs(const cbct_geometry& g, int TS);

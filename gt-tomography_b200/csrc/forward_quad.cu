@@ -121,7 +121,7 @@ void quad_tile(int shape, int& TU, int& TV) {
 //  160x144x112: 0.86 ms, wide 0.92, row pairs 1.00); thin to 1 texel (40 views of 360x220
 //  into 200^3 at 0.99 texel: 1.52 ms, skewed 1.66), skewed beyond (180 views of 256x192
 //  into 128^3 at 1.09 texel: 2.31 ms, thin 2.42, warp 2.71, wide 3.69).  The next shape where
-//  boxes do not fit.
+//  boxes do not fit or its index would leave its range.
 bool quad_choose(cbct_plan* p, double row_dz, bool forced) {
   const double rays = double(p->g.width) * p->g.height * p->max_subset;
   if (!forced && !(row_dz < 0.66 || (row_dz < 0.9 && rays >= 1.5e5) || (row_dz < 1.4 && rays >= 1e6))) return false;
@@ -141,8 +141,9 @@ bool quad_choose(cbct_plan* p, double row_dz, bool forced) {
     const int boxz = std::max(z, 4), nsl = forward_slabs(p->g, d.TS);
     const SlabBox b32{w32, d.BY, boxz, 1}, b16{w16, d.BY, boxz, 1};
     if (!w32 || !w16 || boxz > 256 || quad_smem(b32, 4, nsl) > (size_t)kSmemBudget ||
-        quad_smem(b16, 2, nsl) > (size_t)kSmemBudget)
-      continue;
+        quad_smem(b16, 2, nsl) > (size_t)kSmemBudget || box_index_bound(p->g, b32) >= size_t(1) << 22 ||
+        box_index_bound(p->g, b16) >= size_t(1) << 22)
+      continue;   // (the index bound: volumes of more than 8,000 to 20,000 planes)
     p->quad = b32;
     p->quad16 = b16;
     p->quad_shape = s;

@@ -169,7 +169,8 @@ __device__ __forceinline__ void quad_march(const V* __restrict__ s, float k, flo
     const float2 t = __fadd2_rn(pq, nf);
     const float te = t.x, td = t.y, be = bp.x, nfd = nf.y;
     const float nf0 = kRoundC - __fadd_rd(zz0.x, kRoundC);
-    // the biased sum's mantissa holds the element index (plus the box origin, taken off s)
+    // the biased sum's mantissa holds the element index (plus the box origin, taken off s):
+    // less than 2^22, see box_index_bound
     const V* q = s + int_of_biased(fmaf(nf0, -float(BXY), fmaf(nfd, -float(BX), be)));
     float L[NP], g[NP];
     const float2 te2 = make_float2(te, te), nte2 = make_float2(-te, -te), td2 = make_float2(td, td), ntd2 = make_float2(-td, -td);

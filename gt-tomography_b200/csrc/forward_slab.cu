@@ -132,7 +132,8 @@ bool slab_choose(cbct_plan* p) {
   const SlabBox b32{width(kSlabWidths32, e + 3), kSlabBoxY, std::max(z, 2), 1};
   const SlabBox b16{width(kSlabWidths16, e + 7), kSlabBoxY, std::max(z, 2), 1};
   if (!b32.bx || !b16.bx || b32.bz > 256 || slab_smem(b32, 4, nsl) > (size_t)kSmemBudget ||
-      slab_smem(b16, 2, nsl) > (size_t)kSmemBudget)
+      slab_smem(b16, 2, nsl) > (size_t)kSmemBudget || box_index_bound(p->g, b32) >= size_t(1) << 24 ||
+      box_index_bound(p->g, b16) >= size_t(1) << 24)
     return false;
   p->slab = b32;
   p->slab16 = b16;
