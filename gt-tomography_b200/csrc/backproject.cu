@@ -188,10 +188,13 @@ __global__ void __launch_bounds__(kBX * kBY) bp_kernel(const float* __restrict__
 // FMA pipe together.  The loop has no index clamp (a run's ends are checked per
 // view), takes the byte address of a tap from one multiply-add on the bits of its
 // biased row, and packs pairs of voxels.  36 views of 512x384 into 256^3, the kernel
-// alone: 517 us with clamps, runs of 16 and boxes 56 wide; 447 us now (1.35e12
-// voxel-views/s).
+// alone: 517 us with clamps, runs of 16 and boxes 56 wide; 435 us now (1.39e12
+// voxel-views/s).  A row takes one rounding from the run's start at every eighth voxel
+// and one per two voxels between, four at most (FDK of 256^3 from 360 views against FP64:
+// 1.09e-6; one per voxel along the run 1.18e-6, 1.10e-6 with runs of 16; and a serial
+// chain that made the call 4.66 instead of 4.52 ms).
 // Runs of 32 voxels along z halve the per-view geometry, barriers and staging per
-// voxel against runs of 16 (FDK of 256^3 from 360 views: 4.65 against 5.14 ms); runs
+// voxel against runs of 16 (FDK of 256^3 from 360 views, before the rows above: 4.65 against 5.14 ms); runs
 // of 16 keep more CTAs where the volume is small.
 constexpr int kZRuns[] = {16, 32};
 // Least CTAs of a launch with long runs, four per SM: 20 views into 128^3 (512 CTAs)
@@ -319,7 +322,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
     const float inv = __frcp_rn(yr + gc.SAD);
     const float cu = fmaf(fmaf(gc.SDD * xr, inv, -w.ox), gc.ku, gc.bu) - float(o.x);
     const float A = gc.SDD * inv * gc.kv;
-    float cv = fmaf(fmaf(A, z0, -w.oy * gc.kv), 1.f, gc.bv) - float(o.y);
+    const float cv = fmaf(fmaf(A, z0, -w.oy * gc.kv), 1.f, gc.bv) - float(o.y);
     const float dz = A * gc.vz;
     float wt = 1.f;
     if (FDK) {
@@ -338,10 +341,12 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
                         fmaf(float(ZT - 1), dz, cv) <= float(BV - 1) - 0.01f;
     if (inside) {
       const uint32_t base = smem_u32(sp) + 4u * (unsigned)int(fu) - unsigned(kRoundBits) * (4u * BU);
-      const float2 wt2 = make_float2(wt, wt);
+      const float2 wt2 = make_float2(wt, wt), dz2 = make_float2(2.f * dz, 2.f * dz);
+      float2 c;
 #pragma unroll
       for (int q = 0; q < ZT / 2; ++q) {   // two voxels, packed
-        const float2 c = make_float2(cv, cv + dz);
+        if (q % 4 == 0) c = make_float2(fmaf(float(2 * q), dz, cv), fmaf(float(2 * q + 1), dz, cv));
+        else c = __fadd2_rn(c, dz2);
         const float2 bv = __fadd2_rd(c, make_float2(kRoundC, kRoundC));
         const float2 nf = __ffma2_rn(bv, make_float2(-1.f, -1.f), make_float2(kRoundC, kRoundC));   // -floor
         const float2 av = __fadd2_rn(c, nf);
@@ -353,7 +358,6 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
         const float2 hi = __ffma2_rn(tu, p11, __ffma2_rn(ntu, p01, p01));
         const float2 smp = __ffma2_rn(av, __ffma2_rn(lo, make_float2(-1.f, -1.f), hi), lo);
         acc[q] = FDK ? __ffma2_rn(wt2, smp, acc[q]) : __fadd2_rn(acc[q], smp);
-        cv = c.y + dz;
       }
     }
     // One barrier per view: every thread is done with the stage before it is
