@@ -201,6 +201,14 @@ constexpr int kZRuns[] = {16, 32};
 // take 45.1 us with them and 43.1 without, 25 views into 160x144x128 (720) 65.6
 // and 67.6, 20 views into 64^3 (64) 22.5 and 16.4.
 constexpr int kLongRunCtas = 592;
+// Most shared memory of a CTA with long runs, whose boxes are twice as high: five CTAs
+// per SM, three in launches of four times as many CTAs.  12 views of 0.7, 0.5, 0.45, 0.35
+// and 0.3 mm pixels into 128x128x160 (640 CTAs; 31, 64, 70, 129 and 150 KB): 35.1, 39.2,
+// 40.3, 68.9 and 70.7 us with long runs, 34.6, 37.0, 37.2, 46.4 and 58.6 with short ones;
+// of 0.7, 0.6, 0.5 and 0.4 mm into 256^3 (4096 CTAs; 41, 61, 72 and 129 KB): 167, 191, 202
+// and 383 against 182, 191, 206 and 254.  At 0.25 mm long runs' boxes fit nowhere and short
+// runs' (121 and 142 KB) do: 89 and 602 us.
+constexpr size_t kLongRunSmem[2] = {44 * 1024, 75 * 1024};
 constexpr int kTX = 16, kTY = 8;     // columns per CTA of the TMA back-projector
 
 struct BpView {
@@ -584,26 +592,15 @@ void launch_bp(cbct_plan* p, int s, const float* proj, const BpEpi& e, cudaStrea
 
 }  // namespace
 
-// Chooses the TMA-staged back-projector and its detector box: the largest
-// footprint of any kTX x kTY x zrun block in any view (FP64, corner projections),
-// plus margins.
-void backproject_choose_variant(cbct_plan* p) {
+// Largest footprint (columns, rows; margins included) of any kTX x kTY x zrun block in any
+// view: FP64, corner projections.
+static void bp_extents(const cbct_plan* p, int zrun, int& eu, int& ev) {
   const cbct_geometry& g = p->g;
-  p->bp_variant = 0;
-  p->bp_box = SlabBox{0, 0, 0, 0};
-  p->bp_max_views = 0;
-  if (p->force_gather || p->bp_pref == 1) return;
   const double vx = double(g.lx) / g.nx, vy = double(g.ly) / g.ny, vz = double(g.lz) / g.nz;
   const double ku = g.width / double(g.fov_u), kv = g.height / double(g.fov_v);
   const double bu = g.width / 2.0 - 0.5, bv = g.height / 2.0 - 0.5;
   const int bxn = (g.nx + kTX - 1) / kTX, byn = (g.ny + kTY - 1) / kTY;
-  // Long runs where they leave kLongRunCtas CTAs and pad the volume's height by at
-  // most an eighth more than short ones.
-  auto layers = [&](int r) { return (g.nz + r - 1) / r; };
-  const bool tall = bxn * byn * layers(kZRuns[1]) >= kLongRunCtas &&
-                    layers(kZRuns[1]) * kZRuns[1] * 8 <= layers(kZRuns[0]) * kZRuns[0] * 9;
-  const int zrun = kZRuns[tall], bzn = layers(zrun);
-  p->bp_zrun = zrun;
+  const int bzn = (g.nz + zrun - 1) / zrun;
   std::vector<std::pair<int, int>> acc(host_threads(), {0, 0});
   parallel_for(p->n_views, [&](int lo, int hi, int tid) {
     int& eu = acc[tid].first;
@@ -645,20 +642,41 @@ void backproject_choose_variant(cbct_plan* p) {
         }
     }
   });
-  int eu = 0, ev = 0;
+  eu = ev = 0;
   for (auto& a : acc) {
     eu = std::max(eu, a.first);
     ev = std::max(ev, a.second);
   }
-  int w = 0;
-  for (int c : kBpWidths)
-    if (c >= eu + 3 && (c != kBpWidths[0] || eu + 3 <= kBpNarrow)) { w = c; break; }
-  if (w == 0 || ev > 256) return;
-  p->bp_box = SlabBox{w, std::max(ev, 2), 1, 1};
-  const int maxv = std::min(p->n_views, 1024);
-  if (bp_tma_smem(p, maxv) > (size_t)kSmemBudget) return;
-  p->bp_max_views = maxv;
-  p->bp_variant = 1;
+}
+
+// Chooses the TMA-staged back-projector, its runs along z and its detector box.
+void backproject_choose_variant(cbct_plan* p) {
+  const cbct_geometry& g = p->g;
+  p->bp_variant = 0;
+  p->bp_box = SlabBox{0, 0, 0, 0};
+  p->bp_max_views = 0;
+  if (p->force_gather || p->bp_pref == 1) return;
+  const int bxn = (g.nx + kTX - 1) / kTX, byn = (g.ny + kTY - 1) / kTY, maxv = std::min(p->n_views, 1024);
+  // Long runs where they leave kLongRunCtas CTAs, pad the volume's height by at most an
+  // eighth more than short ones, and their boxes, twice as high, leave an SM enough CTAs
+  // (kLongRunSmem); else short runs.
+  auto layers = [&](int r) { return (g.nz + r - 1) / r; };
+  const int ctas = bxn * byn * layers(kZRuns[1]);
+  const bool tall = ctas >= kLongRunCtas &&
+                    layers(kZRuns[1]) * kZRuns[1] * 8 <= layers(kZRuns[0]) * kZRuns[0] * 9;
+  for (int z = tall; z >= 0; --z) {
+    int eu, ev, w = 0;
+    bp_extents(p, kZRuns[z], eu, ev);
+    for (int c : kBpWidths)
+      if (c >= eu + 3 && (c != kBpWidths[0] || eu + 3 <= kBpNarrow)) { w = c; break; }
+    if (w == 0 || ev > 256) continue;
+    p->bp_box = SlabBox{w, std::max(ev, 2), 1, 1};
+    if (bp_tma_smem(p, maxv) > (z ? kLongRunSmem[ctas >= 4 * kLongRunCtas] : (size_t)kSmemBudget)) continue;
+    p->bp_zrun = kZRuns[z];
+    p->bp_max_views = maxv;
+    p->bp_variant = 1;
+    return;
+  }
 }
 
 void backproject_prepare(cbct_plan* p) {
