@@ -188,13 +188,10 @@ __global__ void __launch_bounds__(kBX * kBY) bp_kernel(const float* __restrict__
 // FMA pipe together.  The loop has no index clamp (a run's ends are checked per
 // view), takes the byte address of a tap from one multiply-add on the bits of its
 // biased row, and packs pairs of voxels.  36 views of 512x384 into 256^3, the kernel
-// alone: 517 us with clamps, runs of 16 and boxes 56 wide; 435 us now (1.39e12
-// voxel-views/s).  A row takes one rounding from the run's start at every eighth voxel
-// and one per two voxels between, four at most (FDK of 256^3 from 360 views against FP64:
-// 1.09e-6; one per voxel along the run 1.18e-6, 1.10e-6 with runs of 16; and a serial
-// chain that made the call 4.66 instead of 4.52 ms).
+// alone: 517 us with clamps, runs of 16 and boxes 56 wide; 420 us now (1.44e12
+// voxel-views/s).
 // Runs of 32 voxels along z halve the per-view geometry, barriers and staging per
-// voxel against runs of 16 (FDK of 256^3 from 360 views, before the rows above: 4.65 against 5.14 ms); runs
+// voxel against runs of 16 (FDK of 256^3 from 360 views: 4.43 against 5.14 ms); runs
 // of 16 keep more CTAs where the volume is small.
 constexpr int kZRuns[] = {16, 32};
 // Least CTAs of a launch with long runs, four per SM: 20 views into 128^3 (512 CTAs)
@@ -246,7 +243,15 @@ bool with_bp(int w, int zrun, F&& f) {
 // of the call.  Shared by the one-scan kernel (block = blockIdx) and the
 // work-list kernel over many scans (block = the item's); base_ptr is the
 // 128-byte aligned dynamic shared memory, bars/abort_flag the CTA's statics.
-template <int EPI, bool FDK, int BU, int ZT>
+//
+// GLOBAL: the rounding of the global-load kernel (detector coordinates counted from the
+// detector's corner, rows stepped voxel by voxel over 8 voxels, lerps as a + t (b - a)),
+// for projections whose rows TMA cannot read in place, which that kernel could take as
+// well.  Otherwise rows are counted from the box of 16 voxels that a row starts in and
+// stepped over these: the second half of a run of 32 takes its own start, as if it were a
+// run.  So results do not depend on the run's length or on the padded copy.
+// (Steps over 32 voxels were 1.9 times as far from FP64 at the run's end.)
+template <int EPI, bool FDK, int BU, int ZT, bool GLOBAL>
 __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewParams* __restrict__ views,
                                             int n_views, const GridConst& gc, const BpEpi& e, int BV, int* flags,
                                             int bi, int bj, int bk, unsigned char* base_ptr, uint64_t* bars,
@@ -300,8 +305,23 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
     o.y = o.y - 1;
     if (ext[q].x + 2 - o.x >= BU || ext[q].y + 2 - o.y >= BV) atomicAdd(&flags[0], 1);
     org[q] = o;
+    ext[q].x = INT_MAX;
   }
   __syncthreads();
+  constexpr int SUB = GLOBAL ? 8 : 16;   // voxels that a row is stepped over
+  if (SUB < ZT && !GLOBAL) {             // the row origin of the second half's box, above org's
+    for (int q = tid; q < n_views * 4; q += nthr) {
+      const int pv = q >> 2, c = q & 3;
+      const BpView w = tv[pv];
+      const float x = fmaf(float((c & 1) ? ie : i0) + 0.5f, gc.vx, -gc.hx);
+      const float y = fmaf(float((c & 2) ? je : j0) + 0.5f, gc.vy, -gc.hy);
+      const float z = fmaf(float(k0 + SUB) + 0.5f, gc.vz, -gc.hz);
+      const float inv = __frcp_rn(fmaf(-w.sn, x, w.cs * y) + gc.SAD);
+      const float cv = fmaf(fmaf(gc.SDD * z, inv, -w.oy), gc.kv, gc.bv);
+      atomicMin(&ext[pv].x, int(floorf(fminf(fmaxf(cv, -1.0e5f), 1.0e5f))) - 1 - org[pv].y);
+    }
+    __syncthreads();
+  }
   auto issue = [&](int pv) {
     uint64_t* bar = &bars[pv & 1];
     mbar_arrive_expect_tx(bar, box_bytes);
@@ -315,7 +335,9 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   const int i = i0 + (warp & 1) * 8 + (lane & 7), j = j0 + (warp >> 1) * 4 + (lane >> 3);
   const float x = fmaf(float(min(i, gc.nx - 1)) + 0.5f, gc.vx, -gc.hx);
   const float y = fmaf(float(min(j, gc.ny - 1)) + 0.5f, gc.vy, -gc.hy);
-  const float z0 = fmaf(float(k0) + 0.5f, gc.vz, -gc.hz);
+  float z0[ZT / SUB];
+#pragma unroll
+  for (int h = 0; h < ZT / SUB; ++h) z0[h] = fmaf(float(k0 + SUB * h) + 0.5f, gc.vz, -gc.hz);
   float2 acc[ZT / 2];
 #pragma unroll
   for (int q = 0; q < ZT / 2; ++q) acc[q] = make_float2(0.f, 0.f);
@@ -328,10 +350,16 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
     const float xr = fmaf(w.cs, x, w.sn * y);
     const float yr = fmaf(-w.sn, x, w.cs * y);
     const float inv = __frcp_rn(yr + gc.SAD);
-    const float cu = fmaf(fmaf(gc.SDD * xr, inv, -w.ox), gc.ku, gc.bu) - float(o.x);
+    const float ca = fmaf(fmaf(gc.SDD * xr, inv, -w.ox), gc.ku, gc.bu), cu = GLOBAL ? ca : ca - float(o.x);
     const float A = gc.SDD * inv * gc.kv;
-    const float cv = fmaf(fmaf(A, z0, -w.oy * gc.kv), 1.f, gc.bv) - float(o.y);
     const float dz = A * gc.vz;
+    // Row of the first voxel of part h of the run: from the detector's corner, or from
+    // the part's box.
+    auto row0 = [&](int h) {
+      if (GLOBAL) return fmaf(A, z0[h], fmaf(-w.oy, gc.kv, gc.bv));
+      return fmaf(fmaf(A, z0[h], -w.oy * gc.kv), 1.f, gc.bv) - float(h == 0 ? o.y : o.y + ext[pv].x);
+    };
+    const float first = row0(0), cv0 = GLOBAL ? first - float(o.y) : first;
     float wt = 1.f;
     if (FDK) {
       const float U = 1.f - yr / gc.SAD;
@@ -342,30 +370,35 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
     // address comes out of one multiply-add on the biased row's bits.  A run outside
     // its box lies beyond the detector (taps of 0); a footprint that did not fit its
     // box was reported above.
-    const float fu = floor_small(cu);
-    const float au = cu - fu;
+    const float fa = floor_small(cu), fu = GLOBAL ? fa - float(o.x) : fa;
+    const float au = cu - fa;
     const float2 tu = make_float2(au, au), ntu = make_float2(-au, -au);
-    const bool inside = fu >= 0.f && fu <= float(BU - 2) && cv >= 0.f &&
-                        fmaf(float(ZT - 1), dz, cv) <= float(BV - 1) - 0.01f;
+    const bool inside = fu >= 0.f && fu <= float(BU - 2) && cv0 >= 0.f && dz >= 0.f &&
+                        fmaf(float(ZT - 1), dz, cv0) <= float(BV - 1) - 0.01f;
     if (inside) {
-      const uint32_t base = smem_u32(sp) + 4u * (unsigned)int(fu) - unsigned(kRoundBits) * (4u * BU);
-      const float2 wt2 = make_float2(wt, wt), dz2 = make_float2(2.f * dz, 2.f * dz);
-      float2 c;
+      const uint32_t base = smem_u32(sp) + 4u * (unsigned)int(fu) - unsigned(kRoundBits + (GLOBAL ? o.y : 0)) * (4u * BU);
+      const float2 wt2 = make_float2(wt, wt);
 #pragma unroll
-      for (int q = 0; q < ZT / 2; ++q) {   // two voxels, packed
-        if (q % 4 == 0) c = make_float2(fmaf(float(2 * q), dz, cv), fmaf(float(2 * q + 1), dz, cv));
-        else c = __fadd2_rn(c, dz2);
-        const float2 bv = __fadd2_rd(c, make_float2(kRoundC, kRoundC));
-        const float2 nf = __ffma2_rn(bv, make_float2(-1.f, -1.f), make_float2(kRoundC, kRoundC));   // -floor
-        const float2 av = __fadd2_rn(c, nf);
-        const uint32_t ta = __float_as_uint(bv.x) * (4u * BU) + base, tb = __float_as_uint(bv.y) * (4u * BU) + base;
-        const float2 p00 = make_float2(lds_f32<0>(ta), lds_f32<0>(tb)), p10 = make_float2(lds_f32<4>(ta), lds_f32<4>(tb));
-        const float2 p01 = make_float2(lds_f32<4 * BU>(ta), lds_f32<4 * BU>(tb));
-        const float2 p11 = make_float2(lds_f32<4 * BU + 4>(ta), lds_f32<4 * BU + 4>(tb));
-        const float2 lo = __ffma2_rn(tu, p10, __ffma2_rn(ntu, p00, p00));
-        const float2 hi = __ffma2_rn(tu, p11, __ffma2_rn(ntu, p01, p01));
-        const float2 smp = __ffma2_rn(av, __ffma2_rn(lo, make_float2(-1.f, -1.f), hi), lo);
-        acc[q] = FDK ? __ffma2_rn(wt2, smp, acc[q]) : __fadd2_rn(acc[q], smp);
+      for (int h = 0; h < ZT / SUB; ++h) {
+        float cv = h == 0 ? first : row0(h);
+        const uint32_t part = GLOBAL || h == 0 ? base : base + unsigned(ext[pv].x) * (4u * BU);
+#pragma unroll
+        for (int q = h * SUB / 2; q < (h + 1) * SUB / 2; ++q) {   // two voxels, packed
+          const float2 c = make_float2(cv, cv + dz);
+          const float2 bv = __fadd2_rd(c, make_float2(kRoundC, kRoundC));
+          const float2 nf = __ffma2_rn(bv, make_float2(-1.f, -1.f), make_float2(kRoundC, kRoundC));   // -floor
+          const float2 av = __fadd2_rn(c, nf);
+          const uint32_t ta = __float_as_uint(bv.x) * (4u * BU) + part, tb = __float_as_uint(bv.y) * (4u * BU) + part;
+          const float2 p00 = make_float2(lds_f32<0>(ta), lds_f32<0>(tb)), p10 = make_float2(lds_f32<4>(ta), lds_f32<4>(tb));
+          const float2 p01 = make_float2(lds_f32<4 * BU>(ta), lds_f32<4 * BU>(tb));
+          const float2 p11 = make_float2(lds_f32<4 * BU + 4>(ta), lds_f32<4 * BU + 4>(tb));
+          const float2 none = make_float2(-1.f, -1.f);
+          const float2 lo = GLOBAL ? __ffma2_rn(tu, __ffma2_rn(p00, none, p10), p00) : __ffma2_rn(tu, p10, __ffma2_rn(ntu, p00, p00));
+          const float2 hi = GLOBAL ? __ffma2_rn(tu, __ffma2_rn(p01, none, p11), p01) : __ffma2_rn(tu, p11, __ffma2_rn(ntu, p01, p01));
+          const float2 smp = __ffma2_rn(av, __ffma2_rn(lo, none, hi), lo);
+          acc[q] = FDK ? __ffma2_rn(wt2, smp, acc[q]) : __fadd2_rn(acc[q], smp);
+          cv = c.y + dz;
+        }
       }
     }
     // One barrier per view: every thread is done with the stage before it is
@@ -405,7 +438,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   }
 }
 
-template <int EPI, bool FDK, int BU, int ZT>
+template <int EPI, bool FDK, int BU, int ZT, bool GLOBAL>
 __global__ void __launch_bounds__(kTX * kTY) bp_tma_kernel(const __grid_constant__ CUtensorMap map,
                                                            const ViewParams* __restrict__ views, int n_views,
                                                            GridConst gc, BpEpi e, int BV, int* flags) {
@@ -414,7 +447,7 @@ __global__ void __launch_bounds__(kTX * kTY) bp_tma_kernel(const __grid_constant
   __shared__ int abort_flag;
   unsigned char* base_ptr =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
-  bp_tma_body<EPI, FDK, BU, ZT>(&map, views, n_views, gc, e, BV, flags, blockIdx.x, blockIdx.y, blockIdx.z, base_ptr,
+  bp_tma_body<EPI, FDK, BU, ZT, GLOBAL>(&map, views, n_views, gc, e, BV, flags, blockIdx.x, blockIdx.y, blockIdx.z, base_ptr,
                             bars, abort_flag);
 }
 
@@ -464,7 +497,7 @@ __global__ void __launch_bounds__(kTX * kTY) bp_tma_multi_kernel(const BpScanRec
       tensormap_acquire(&R.map);
       last = lo;
     }
-    bp_tma_body<EPI, FDK, BU, ZT>(&R.map, R.views, R.n_views, R.gc, R.e, R.BV, R.flags, bi, bj, bk, base_ptr, bars,
+    bp_tma_body<EPI, FDK, BU, ZT, false>(&R.map, R.views, R.n_views, R.gc, R.e, R.BV, R.flags, bi, bj, bk, base_ptr, bars,
                               abort_flag);
     __syncthreads();
     // A wait that gave up is counted in the scan's flag word and its loads
@@ -500,13 +533,13 @@ CUtensorMap make_bp_map(const cbct_plan* p, const float* proj, int cnt) {
   return m;
 }
 
-template <int EPI, bool FDK, int BU, int ZT>
+template <int EPI, bool FDK, int BU, int ZT, bool GLOBAL>
 void launch_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi& e, cudaStream_t st) {
   const CUtensorMap m = make_bp_map(p, proj, cnt);
   dim3 block(kTX * kTY);
   dim3 grid((p->g.nx + kTX - 1) / kTX, (p->g.ny + kTY - 1) / kTY, (p->g.nz + ZT - 1) / ZT);
   const size_t smem = bp_tma_smem(p, cnt);
-  auto k = bp_tma_kernel<EPI, FDK, BU, ZT>;
+  auto k = bp_tma_kernel<EPI, FDK, BU, ZT, GLOBAL>;
   ensure_smem_attr((const void*)k, smem);
   k<<<grid, block, smem, st>>>(m, p->d_views + first, cnt, p->gc, e, p->bp_box.by, p->d_flags);
   check_launch("bp_tma_kernel");
@@ -526,12 +559,13 @@ bool needs_padded_rows(const cbct_plan* p, const float* proj) {
 // The TMA-staged back-projection of a view range, from a row-padded copy of its
 // projections where TMA cannot read them in place; false where neither is possible.
 // The copy costs 8 bytes per pixel against some hundred bilinear taps per pixel: 40
-// views of 301x211 into 150x141x93 voxels take 98 us with it, 260 us with the
+// views of 301x211 into 150x141x93 voxels take 93 us with it, 260 us with the
 // global-load kernel.
 template <int EPI, bool FDK>
 bool try_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi& e, cudaStream_t st) {
   if (p->bp_variant != 1 || cnt > p->bp_max_views) return false;
-  if (needs_padded_rows(p, proj)) {
+  const bool pad = needs_padded_rows(p, proj);
+  if (pad) {
     if (cnt > p->bp_pad_views) return false;
     const int rows = p->g.height * cnt;
     pad_rows_kernel<<<std::min((rows + 7) / 8, 148 * 16), 256, 0, st>>>(proj, p->d_bp_pad, p->g.width,
@@ -540,23 +574,27 @@ bool try_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi
     proj = p->d_bp_pad;
   }
   return with_bp(p->bp_box.bx, p->bp_zrun, [&](auto W, auto Z) {
-    launch_bp_tma<EPI, FDK, decltype(W)::value, decltype(Z)::value>(p, first, cnt, proj, e, st);
+    if (pad) launch_bp_tma<EPI, FDK, decltype(W)::value, decltype(Z)::value, true>(p, first, cnt, proj, e, st);
+    else launch_bp_tma<EPI, FDK, decltype(W)::value, decltype(Z)::value, false>(p, first, cnt, proj, e, st);
   });
 }
 
+// global: the kernels of padded copies (detectors of odd rows), else the others.
 template <int EPI, bool FDK, int BU, int ZT>
-void prepare_bp_width(size_t smem) {
-  ensure_smem_attr((const void*)bp_tma_kernel<EPI, FDK, BU, ZT>, smem);
+void prepare_bp_width(size_t smem, bool global) {
+  ensure_smem_attr(global ? (const void*)bp_tma_kernel<EPI, FDK, BU, ZT, true>
+                          : (const void*)bp_tma_kernel<EPI, FDK, BU, ZT, false>,
+                   smem);
 }
 
 template <int BU, int ZT>
-void prepare_bp_all(size_t smem) {
-  prepare_bp_width<kStore, false, BU, ZT>(smem);
-  prepare_bp_width<kStore, true, BU, ZT>(smem);
-  prepare_bp_width<kRecip, false, BU, ZT>(smem);
-  prepare_bp_width<kMom, false, BU, ZT>(smem);
-  prepare_bp_width<kSart, false, BU, ZT>(smem);
-  prepare_bp_width<kStep, false, BU, ZT>(smem);
+void prepare_bp_all(size_t smem, bool global) {
+  prepare_bp_width<kStore, false, BU, ZT>(smem, global);
+  prepare_bp_width<kStore, true, BU, ZT>(smem, global);
+  prepare_bp_width<kRecip, false, BU, ZT>(smem, global);
+  prepare_bp_width<kMom, false, BU, ZT>(smem, global);
+  prepare_bp_width<kSart, false, BU, ZT>(smem, global);
+  prepare_bp_width<kStep, false, BU, ZT>(smem, global);
 }
 
 template <int EPI, bool FDK>
@@ -682,7 +720,9 @@ void backproject_choose_variant(cbct_plan* p) {
 void backproject_prepare(cbct_plan* p) {
   if (p->bp_variant == 1) {
     const size_t sm = bp_tma_smem(p, p->bp_max_views);
-    with_bp(p->bp_box.bx, p->bp_zrun, [&](auto W, auto Z) { prepare_bp_all<decltype(W)::value, decltype(Z)::value>(sm); });
+    with_bp(p->bp_box.bx, p->bp_zrun, [&](auto W, auto Z) {
+      prepare_bp_all<decltype(W)::value, decltype(Z)::value>(sm, p->g.width % 4 != 0);
+    });
     if (bp_pad_bytes(p->g, p->max_subset) && !p->d_bp_pad) {
       p->d_bp_pad = static_cast<float*>(plan_alloc(p, bp_pad_bytes(p->g, p->max_subset)));
       p->bp_pad_views = std::min(p->max_subset, kBpPadViews);

@@ -8,8 +8,8 @@ pytestmark = pytest.mark.gpu
 
 # Detectors of 200 rows: coordinates below 256 and, counted from a box's corner, below 128.
 # The kernel's rows differ from FP64 by three roundings of A z (at most 100 rows: 3 x
-# 2^-24 x 100), two at detector coordinates (2^-17 each at most), five at box coordinates
-# (2^-18 each) and the tap's own three (values below 256, 2^-17 each): below 1e-4 at most.
+# 2^-24 x 100), two at detector coordinates (2^-17 each at most), fifteen at box coordinates
+# (2^-19 each) and the tap's own three (values below 256, 2^-17 each): below 1e-4.
 BOUND = 1e-4
 
 
