@@ -193,7 +193,14 @@ __global__ void __launch_bounds__(kBX * kBY) bp_kernel(const float* __restrict__
 // Runs of 32 voxels along z halve the per-view geometry, barriers and staging per
 // voxel against runs of 16 (FDK of 256^3 from 360 views: 4.43 against 5.14 ms); runs
 // of 16 keep more CTAs where the volume is small.
-constexpr int kZRuns[] = {16, 32};
+// Volumes of fewer planes than a short run take kernels of their own (kFlatRun), whose boxes
+// hold the volume's planes only, rounded up to what is taken between two looks at them:
+// thick planes need that (24 views of 0.8 mm pixels into 256x256x12 voxels of 1x1x8 mm: 46
+// us, 79 us with the global-load kernel, which boxes of 16 planes left).  A check of the
+// planes in the other kernels cost them 2 %.
+constexpr int kZRuns[] = {16, 32, 16};
+constexpr int kFlatRun = 2, kNZRuns = 3;
+constexpr int bp_box_planes(int run, int nz) { return run == kFlatRun ? (nz + 3) / 4 * 4 : kZRuns[run]; }
 // Least CTAs of a launch with long runs, four per SM: 20 views into 128^3 (512 CTAs)
 // take 45.1 us with them and 43.1 without, 25 views into 160x144x128 (720) 65.6
 // and 67.6, 20 views into 64^3 (64) 22.5 and 16.4.
@@ -206,6 +213,11 @@ constexpr int kLongRunCtas = 592;
 // and 383 against 182, 191, 206 and 254.  At 0.25 mm long runs' boxes fit nowhere and short
 // runs' (121 and 142 KB) do: 89 and 602 us.
 constexpr size_t kLongRunSmem[2] = {44 * 1024, 75 * 1024};
+// The same for flat volumes, whose boxes serve few voxels: three CTAs, or 9 KB per plane;
+// else global loads.  24 views into 256x256 voxels, staged and global, us: 3 planes of 10 mm
+// at 65 and 116 KB 45, 44 and 60, 44; 8 of 5 mm at 75 and 135 KB 39, 55 and 67, 56; 12 of 8
+// mm at 78 KB 46, 79; 15 of 3 mm at 96 and 172 KB 50, 86 and 83, 85.
+constexpr size_t flat_smem(int nz) { return size_t(nz <= 8 ? 76 : 9 * nz) * 1024; }
 constexpr int kTX = 16, kTY = 8;     // columns per CTA of the TMA back-projector
 
 struct BpView {
@@ -223,17 +235,18 @@ constexpr int kBpWidths[] = {40, 48, 56, 72, 104, 136};
 constexpr int kBpNarrow = 32;
 constexpr int kNBpWidths = int(sizeof(kBpWidths) / sizeof(int));
 
-// Calls f(std::integral_constant<int, W>, std::integral_constant<int, Z>) for the
-// compiled width W == w and run Z == zrun; false when there is none.
+// Calls f(std::integral_constant<int, W>, std::integral_constant<int, R>) for the
+// compiled width W == w and run kZRuns[R], R == run; false when there is none.
 template <int I = 0, class F>
-bool with_bp(int w, int zrun, F&& f) {
+bool with_bp(int w, int run, F&& f) {
   if constexpr (I < kNBpWidths) {
     if (w == kBpWidths[I]) {
-      if (zrun == kZRuns[0]) f(std::integral_constant<int, kBpWidths[I]>{}, std::integral_constant<int, kZRuns[0]>{});
-      else f(std::integral_constant<int, kBpWidths[I]>{}, std::integral_constant<int, kZRuns[1]>{});
+      if (run == 0) f(std::integral_constant<int, kBpWidths[I]>{}, std::integral_constant<int, 0>{});
+      else if (run == 1) f(std::integral_constant<int, kBpWidths[I]>{}, std::integral_constant<int, 1>{});
+      else f(std::integral_constant<int, kBpWidths[I]>{}, std::integral_constant<int, kFlatRun>{});
       return true;
     }
-    return with_bp<I + 1>(w, zrun, std::forward<F>(f));
+    return with_bp<I + 1>(w, run, std::forward<F>(f));
   } else {
     return false;
   }
@@ -251,11 +264,13 @@ bool with_bp(int w, int zrun, F&& f) {
 // stepped over these: the second half of a run of 32 takes its own start, as if it were a
 // run.  So results do not depend on the run's length or on the padded copy.
 // (Steps over 32 voxels were 1.9 times as far from FP64 at the run's end.)
-template <int EPI, bool FDK, int BU, int ZT, bool GLOBAL>
+template <int EPI, bool FDK, int BU, int RUN, bool GLOBAL>
 __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewParams* __restrict__ views,
                                             int n_views, const GridConst& gc, const BpEpi& e, int BV, int* flags,
                                             int bi, int bj, int bk, unsigned char* base_ptr, uint64_t* bars,
                                             int& abort_flag) {
+  constexpr int ZT = kZRuns[RUN];
+  const int planes = RUN == kFlatRun ? bp_box_planes(RUN, gc.nz) : ZT;   // of the box
   const uint32_t box_bytes = uint32_t(BU * BV * 4);
   const uint32_t stage_stride = (box_bytes + 127u) & ~127u;
   BpView* tv = reinterpret_cast<BpView*>(base_ptr + 2 * stage_stride);
@@ -279,7 +294,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   }
   __syncthreads();
   // Footprints: 8 corners of the block (voxel centres) per view.
-  const int ie = min(i0 + kTX, gc.nx) - 1, je = min(j0 + kTY, gc.ny) - 1, ke = k0 + ZT - 1;
+  const int ie = min(i0 + kTX, gc.nx) - 1, je = min(j0 + kTY, gc.ny) - 1, ke = k0 + planes - 1;
   for (int q = tid; q < n_views * 8; q += nthr) {
     const int pv = q >> 3, c = q & 7;
     const BpView w = tv[pv];
@@ -374,7 +389,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
     const float au = cu - fa;
     const float2 tu = make_float2(au, au), ntu = make_float2(-au, -au);
     const bool inside = fu >= 0.f && fu <= float(BU - 2) && cv0 >= 0.f && dz >= 0.f &&
-                        fmaf(float(ZT - 1), dz, cv0) <= float(BV - 1) - 0.01f;
+                        fmaf(float(planes - 1), dz, cv0) <= float(BV - 1) - 0.01f;
     if (inside) {
       const uint32_t base = smem_u32(sp) + 4u * (unsigned)int(fu) - unsigned(kRoundBits + (GLOBAL ? o.y : 0)) * (4u * BU);
       const float2 wt2 = make_float2(wt, wt);
@@ -384,6 +399,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
         const uint32_t part = GLOBAL || h == 0 ? base : base + unsigned(ext[pv].x) * (4u * BU);
 #pragma unroll
         for (int q = h * SUB / 2; q < (h + 1) * SUB / 2; ++q) {   // two voxels, packed
+          if (RUN == kFlatRun && q > 0 && q % 2 == 0 && 2 * q >= planes) break;
           const float2 c = make_float2(cv, cv + dz);
           const float2 bv = __fadd2_rd(c, make_float2(kRoundC, kRoundC));
           const float2 nf = __ffma2_rn(bv, make_float2(-1.f, -1.f), make_float2(kRoundC, kRoundC));   // -floor
@@ -438,7 +454,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
   }
 }
 
-template <int EPI, bool FDK, int BU, int ZT, bool GLOBAL>
+template <int EPI, bool FDK, int BU, int RUN, bool GLOBAL>
 __global__ void __launch_bounds__(kTX * kTY) bp_tma_kernel(const __grid_constant__ CUtensorMap map,
                                                            const ViewParams* __restrict__ views, int n_views,
                                                            GridConst gc, BpEpi e, int BV, int* flags) {
@@ -447,7 +463,7 @@ __global__ void __launch_bounds__(kTX * kTY) bp_tma_kernel(const __grid_constant
   __shared__ int abort_flag;
   unsigned char* base_ptr =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
-  bp_tma_body<EPI, FDK, BU, ZT, GLOBAL>(&map, views, n_views, gc, e, BV, flags, blockIdx.x, blockIdx.y, blockIdx.z, base_ptr,
+  bp_tma_body<EPI, FDK, BU, RUN, GLOBAL>(&map, views, n_views, gc, e, BV, flags, blockIdx.x, blockIdx.y, blockIdx.z, base_ptr,
                             bars, abort_flag);
 }
 
@@ -469,7 +485,7 @@ struct alignas(128) BpScanRec {
 // atomic counter until the list is empty; the item runs the one-scan kernel's
 // body, so every voxel gets the same arithmetic as in a launch of its own.
 // Items are numbered scan by scan, CTA-grid order (x fastest) inside a scan.
-template <int EPI, bool FDK, int BU, int ZT>
+template <int EPI, bool FDK, int BU, int RUN>
 __global__ void __launch_bounds__(kTX * kTY) bp_tma_multi_kernel(const BpScanRec* __restrict__ recs, int n_recs,
                                                                  int total, int* __restrict__ counter) {
   extern __shared__ __align__(128) unsigned char smem_dyn[];
@@ -497,7 +513,7 @@ __global__ void __launch_bounds__(kTX * kTY) bp_tma_multi_kernel(const BpScanRec
       tensormap_acquire(&R.map);
       last = lo;
     }
-    bp_tma_body<EPI, FDK, BU, ZT, false>(&R.map, R.views, R.n_views, R.gc, R.e, R.BV, R.flags, bi, bj, bk, base_ptr, bars,
+    bp_tma_body<EPI, FDK, BU, RUN, false>(&R.map, R.views, R.n_views, R.gc, R.e, R.BV, R.flags, bi, bj, bk, base_ptr, bars,
                               abort_flag);
     __syncthreads();
     // A wait that gave up is counted in the scan's flag word and its loads
@@ -533,13 +549,13 @@ CUtensorMap make_bp_map(const cbct_plan* p, const float* proj, int cnt) {
   return m;
 }
 
-template <int EPI, bool FDK, int BU, int ZT, bool GLOBAL>
+template <int EPI, bool FDK, int BU, int RUN, bool GLOBAL>
 void launch_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi& e, cudaStream_t st) {
   const CUtensorMap m = make_bp_map(p, proj, cnt);
   dim3 block(kTX * kTY);
-  dim3 grid((p->g.nx + kTX - 1) / kTX, (p->g.ny + kTY - 1) / kTY, (p->g.nz + ZT - 1) / ZT);
+  dim3 grid((p->g.nx + kTX - 1) / kTX, (p->g.ny + kTY - 1) / kTY, (p->g.nz + kZRuns[RUN] - 1) / kZRuns[RUN]);
   const size_t smem = bp_tma_smem(p, cnt);
-  auto k = bp_tma_kernel<EPI, FDK, BU, ZT, GLOBAL>;
+  auto k = bp_tma_kernel<EPI, FDK, BU, RUN, GLOBAL>;
   ensure_smem_attr((const void*)k, smem);
   k<<<grid, block, smem, st>>>(m, p->d_views + first, cnt, p->gc, e, p->bp_box.by, p->d_flags);
   check_launch("bp_tma_kernel");
@@ -573,28 +589,28 @@ bool try_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi
     check_launch("pad_rows_kernel");
     proj = p->d_bp_pad;
   }
-  return with_bp(p->bp_box.bx, p->bp_zrun, [&](auto W, auto Z) {
+  return with_bp(p->bp_box.bx, p->bp_run, [&](auto W, auto Z) {
     if (pad) launch_bp_tma<EPI, FDK, decltype(W)::value, decltype(Z)::value, true>(p, first, cnt, proj, e, st);
     else launch_bp_tma<EPI, FDK, decltype(W)::value, decltype(Z)::value, false>(p, first, cnt, proj, e, st);
   });
 }
 
 // global: the kernels of padded copies (detectors of odd rows), else the others.
-template <int EPI, bool FDK, int BU, int ZT>
+template <int EPI, bool FDK, int BU, int RUN>
 void prepare_bp_width(size_t smem, bool global) {
-  ensure_smem_attr(global ? (const void*)bp_tma_kernel<EPI, FDK, BU, ZT, true>
-                          : (const void*)bp_tma_kernel<EPI, FDK, BU, ZT, false>,
+  ensure_smem_attr(global ? (const void*)bp_tma_kernel<EPI, FDK, BU, RUN, true>
+                          : (const void*)bp_tma_kernel<EPI, FDK, BU, RUN, false>,
                    smem);
 }
 
-template <int BU, int ZT>
+template <int BU, int RUN>
 void prepare_bp_all(size_t smem, bool global) {
-  prepare_bp_width<kStore, false, BU, ZT>(smem, global);
-  prepare_bp_width<kStore, true, BU, ZT>(smem, global);
-  prepare_bp_width<kRecip, false, BU, ZT>(smem, global);
-  prepare_bp_width<kMom, false, BU, ZT>(smem, global);
-  prepare_bp_width<kSart, false, BU, ZT>(smem, global);
-  prepare_bp_width<kStep, false, BU, ZT>(smem, global);
+  prepare_bp_width<kStore, false, BU, RUN>(smem, global);
+  prepare_bp_width<kStore, true, BU, RUN>(smem, global);
+  prepare_bp_width<kRecip, false, BU, RUN>(smem, global);
+  prepare_bp_width<kMom, false, BU, RUN>(smem, global);
+  prepare_bp_width<kSart, false, BU, RUN>(smem, global);
+  prepare_bp_width<kStep, false, BU, RUN>(smem, global);
 }
 
 template <int EPI, bool FDK>
@@ -630,15 +646,15 @@ void launch_bp(cbct_plan* p, int s, const float* proj, const BpEpi& e, cudaStrea
 
 }  // namespace
 
-// Largest footprint (columns, rows; margins included) of any kTX x kTY x zrun block in any
-// view: FP64, corner projections.
-static void bp_extents(const cbct_plan* p, int zrun, int& eu, int& ev) {
+// Largest footprint (columns, rows; margins included) of any block of a run in any view:
+// FP64, corner projections.
+static void bp_extents(const cbct_plan* p, int run, int& eu, int& ev) {
   const cbct_geometry& g = p->g;
   const double vx = double(g.lx) / g.nx, vy = double(g.ly) / g.ny, vz = double(g.lz) / g.nz;
   const double ku = g.width / double(g.fov_u), kv = g.height / double(g.fov_v);
   const double bu = g.width / 2.0 - 0.5, bv = g.height / 2.0 - 0.5;
   const int bxn = (g.nx + kTX - 1) / kTX, byn = (g.ny + kTY - 1) / kTY;
-  const int bzn = (g.nz + zrun - 1) / zrun;
+  const int zrun = kZRuns[run], bzn = (g.nz + zrun - 1) / zrun, planes = bp_box_planes(run, g.nz);
   std::vector<std::pair<int, int>> acc(host_threads(), {0, 0});
   parallel_for(p->n_views, [&](int lo, int hi, int tid) {
     int& eu = acc[tid].first;
@@ -667,7 +683,7 @@ static void bp_extents(const cbct_plan* p, int zrun, int& eu, int& ev) {
           const double bound = g.SDD * kv * ((imx - imn) * (0.5 * g.lz + zrun * vz) + imx * (zrun - 1) * vz);
           if (imn > 0 && std::ceil(bound) + 3 + 2 <= ev) continue;
           for (int bk = 0; bk < bzn; ++bk) {
-            const int k0 = bk * zrun, ke = k0 + zrun - 1;   // whole runs, also past the volume's top
+            const int k0 = bk * zrun, ke = k0 + planes - 1;   // whole runs, also past the volume's top
             const double z0 = (k0 + 0.5) * vz - g.lz / 2.0, z1 = (ke + 0.5) * vz - g.lz / 2.0;
             double vmn = 1e30, vmx = -1e30;
             for (double inv : {imn, imx})
@@ -702,15 +718,17 @@ void backproject_choose_variant(cbct_plan* p) {
   const int ctas = bxn * byn * layers(kZRuns[1]);
   const bool tall = ctas >= kLongRunCtas &&
                     layers(kZRuns[1]) * kZRuns[1] * 8 <= layers(kZRuns[0]) * kZRuns[0] * 9;
-  for (int z = tall; z >= 0; --z) {
+  const bool flat = g.nz < kZRuns[0];
+  for (int z = flat ? kFlatRun : tall; z >= 0; z = z == 1 ? 0 : -1) {
     int eu, ev, w = 0;
-    bp_extents(p, kZRuns[z], eu, ev);
+    bp_extents(p, z, eu, ev);
     for (int c : kBpWidths)
       if (c >= eu + 3 && (c != kBpWidths[0] || eu + 3 <= kBpNarrow)) { w = c; break; }
     if (w == 0 || ev > 256) continue;
     p->bp_box = SlabBox{w, std::max(ev, 2), 1, 1};
-    if (bp_tma_smem(p, maxv) > (z ? kLongRunSmem[ctas >= 4 * kLongRunCtas] : (size_t)kSmemBudget)) continue;
-    p->bp_zrun = kZRuns[z];
+    const size_t most = flat ? flat_smem(g.nz) : z ? kLongRunSmem[ctas >= 4 * kLongRunCtas] : (size_t)kSmemBudget;
+    if (bp_tma_smem(p, maxv) > most) continue;
+    p->bp_run = z;
     p->bp_max_views = maxv;
     p->bp_variant = 1;
     return;
@@ -720,7 +738,7 @@ void backproject_choose_variant(cbct_plan* p) {
 void backproject_prepare(cbct_plan* p) {
   if (p->bp_variant == 1) {
     const size_t sm = bp_tma_smem(p, p->bp_max_views);
-    with_bp(p->bp_box.bx, p->bp_zrun, [&](auto W, auto Z) {
+    with_bp(p->bp_box.bx, p->bp_run, [&](auto W, auto Z) {
       prepare_bp_all<decltype(W)::value, decltype(Z)::value>(sm, p->g.width % 4 != 0);
     });
     if (bp_pad_bytes(p->g, p->max_subset) && !p->d_bp_pad) {
@@ -801,9 +819,9 @@ void backproject_step_launch(cbct_plan* p, int s, const float* proj, const float
 namespace {
 
 // Work-list launch of one box width: records at A.dev + off.
-template <int EPI, int BU, int ZT>
+template <int EPI, int BU, int RUN>
 void add_bp_group(WorkArena& A, const std::vector<BpScanRec>& recs, int total, size_t smem) {
-  auto k = bp_tma_multi_kernel<EPI, false, BU, ZT>;
+  auto k = bp_tma_multi_kernel<EPI, false, BU, RUN>;
   ensure_smem_attr((const void*)k, smem);
   const size_t off = A.add(recs.data(), recs.size() * sizeof(BpScanRec));
   const int ci = A.n_counters++;
@@ -818,7 +836,7 @@ void add_bp_group(WorkArena& A, const std::vector<BpScanRec>& recs, int total, s
 template <int EPI>
 const void* bp_multi_ptr(int c, int z) {
   const void* k = nullptr;
-  with_bp(kBpWidths[c], kZRuns[z], [&](auto W, auto Z) {
+  with_bp(kBpWidths[c], z, [&](auto W, auto Z) {
     k = (const void*)bp_tma_multi_kernel<EPI, false, decltype(W)::value, decltype(Z)::value>;
   });
   return k;
@@ -826,12 +844,12 @@ const void* bp_multi_ptr(int c, int z) {
 
 template <int EPI>
 void backproject_multi_t(WorkArena& A, const std::vector<MultiBpJob>& jobs) {
-  std::vector<BpScanRec> groups[2][kNBpWidths];
-  int totals[2][kNBpWidths] = {};
-  size_t smem[2][kNBpWidths] = {};
+  std::vector<BpScanRec> groups[kNZRuns][kNBpWidths];
+  int totals[kNZRuns][kNBpWidths] = {};
+  size_t smem[kNZRuns][kNBpWidths] = {};
   auto flush = [&](int z, int c) {
     if (groups[z][c].empty()) return;
-    with_bp(kBpWidths[c], kZRuns[z], [&](auto W, auto Z) {
+    with_bp(kBpWidths[c], z, [&](auto W, auto Z) {
       add_bp_group<EPI, decltype(W)::value, decltype(Z)::value>(A, groups[z][c], totals[z][c], smem[z][c]);
     });
     groups[z][c].clear();
@@ -854,8 +872,8 @@ void backproject_multi_t(WorkArena& A, const std::vector<MultiBpJob>& jobs) {
     for (int c = 0; c < kNBpWidths; ++c)
       if (kBpWidths[c] == p->bp_box.bx) w = c;
     const bool tma = p->bp_variant == 1 && cnt <= p->bp_max_views && !needs_padded_rows(p, j.proj) && w >= 0;
-    const int tx = (p->g.nx + kTX - 1) / kTX, ty = (p->g.ny + kTY - 1) / kTY, tz = (p->g.nz + p->bp_zrun - 1) / p->bp_zrun;
-    const int z = p->bp_zrun == kZRuns[1];
+    const int tx = (p->g.nx + kTX - 1) / kTX, ty = (p->g.ny + kTY - 1) / kTY, z = p->bp_run;
+    const int tz = (p->g.nz + kZRuns[z] - 1) / kZRuns[z];
     bool own = !tma;
     if (tma) {
       const void* kfn = bp_multi_ptr<EPI>(w, z);
@@ -886,7 +904,7 @@ void backproject_multi_t(WorkArena& A, const std::vector<MultiBpJob>& jobs) {
     smem[z][w] = std::max(smem[z][w], bp_tma_smem(p, cnt));
     groups[z][w].push_back(r);
   }
-  for (int z = 0; z < 2; ++z)
+  for (int z = 0; z < kNZRuns; ++z)
     for (int c = 0; c < kNBpWidths; ++c) flush(z, c);
 }
 

@@ -226,7 +226,7 @@ struct cbct_plan {
   int bp_variant = 0;       // 0 = global loads, 1 = TMA-staged detector boxes
   int bp_pref = 0;          // 0: TMA-staged where it fits, 1: global loads (autotuner)
   cbct::SlabBox bp_box{};   // detector box (bx = u width, by = v rows)
-  int bp_zrun = 16;         // voxels of a thread's run along z
+  int bp_run = 0;           // its runs along z (index into backproject.cu's kZRuns)
   int bp_max_views = 0;     // views per launch the TMA back-projector holds
   float* d_bp_pad = nullptr;  // row-padded projections where W is not a multiple of 4 (bp_pad_bytes)
   int bp_pad_views = 0;     // views it holds

@@ -44,7 +44,7 @@ def test_runs_of_32_are_runs_of_16(gtb, cuda, fdk, nz, pitch):
 
 @pytest.mark.parametrize("n,W,H,pitch,P", [((30, 27, 21), 45, 34, 1.2, 7), ((48, 40, 33), 61, 50, 1.2, 128),
                                            ((44, 35, 16), 47, 40, 1.4, 5), ((256, 250, 70), 271, 100, 1.7, 6),
-                                           ((256, 256, 64), 401, 220, 0.8, 6)])
+                                           ((256, 256, 64), 401, 220, 0.8, 6), ((64, 48, 5), 90, 30, 1.1, 5)])
 def test_padded_detectors_are_the_global_loads(gtb, cuda, n, W, H, pitch, P):
     import torch
     L = gtb._lib
