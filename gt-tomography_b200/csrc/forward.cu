@@ -1096,7 +1096,7 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
     for (int iv = lo; iv < hi && a.ok; ++iv) {
       const ViewParams& vp = p->hviews[iv];
       const int dom = vp.dom;
-      const int Nd = dom ? g.ny : g.nx;
+      const int Nd = dom ? g.ny : g.nx, Ne = dom ? g.nx : g.ny;
       const double ke = dom ? kx : ky, be = dom ? bx : by, kd = dom ? ky : kx, bd = dom ? by : bx;
       const double Se = dom ? vp.Sx : vp.Sy, Sd = dom ? vp.Sy : vp.Sx, ikd = 1.0 / kd;
       const int nsl = (Nd + 1 - kSlabBase + TS - 1) / TS + 1;
@@ -1108,6 +1108,11 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
       }
       const double dzabs = std::max(std::fabs(dz0[0]), std::fabs(dz1[tiles_v - 1]));
       const double dzspan = (TV - 1) * (double)vp.Evz;
+      // Distances of the first and last slab plane from the source along the slab axis,
+      // and the largest |dz| of a row that meets the volume.
+      const double near = (kSlabBase - bd) * ikd - Sd, far = (kSlabBase + nsl * TS - bd) * ikd - Sd;
+      const double pmax = std::max(std::fabs(near), std::fabs(far)), pmin = std::min(std::fabs(near), std::fabs(far));
+      const bool ahead = near * vp.dsgn > 0 && far * vp.dsgn > 0;
       for (int tu = 0; tu < tiles_u && a.ok; ++tu) {
         const int uc[2] = {tu * TU, std::min(tu * TU + TU, g.width) - 1};
         double de[2], dd[2];
@@ -1122,6 +1127,16 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
         // Ray parameters t and e coordinates of the tile's two edge columns at a
         // slab's first plane; the last plane is the next slab's first.
         const double idd[2] = {1.0 / dd[0], 1.0 / dd[1]};
+        // No slab of this tile spans more than these: skip the tile where neither can
+        // exceed what was found so far (most tiles: two thirds of the time over random plans).
+        const double s0 = de[0] * idd[0], s1 = de[1] * idd[1], ai = std::max(std::fabs(idd[0]), std::fabs(idd[1]));
+        const double dmost = beside || !ahead
+                                 ? dzabs
+                                 : std::min(dzabs, (g.nz + 1.0 - bz) / (kz * pmin * std::min(std::fabs(idd[0]), std::fabs(idd[1]))));
+        const double se = ke * (TS * ikd * std::max(std::fabs(s0), std::fabs(s1)) + pmax * std::fabs(s0 - s1));
+        const double sz = kz * ((TS * ikd * ai + pmax * std::fabs(idd[0] - idd[1])) * dmost + pmax * ai * dzspan);
+        if (std::min(std::ceil(se + 1e-9) + 3 + 2, Ne + 4.0) <= a.e && std::min(std::ceil(sz + 1e-9) + 3 + 2, g.nz + 4.0) <= a.z)
+          continue;
         double t0[2], e0[2], t1[2], e1[2];
         auto at_plane = [&](int m, double (&t)[2], double (&e)[2]) {
           const double pl = (kSlabBase + m * TS - bd) * ikd - Sd;
@@ -1140,7 +1155,6 @@ bool slab_extents(const cbct_plan* p, int TU, int TV, int TS, int& ext_e, int& e
           const double tmx = std::max(std::max(t0[0], t0[1]), std::max(t1[0], t1[1]));
           // elements from floor(min)-1 to floor(max)+1 inclusive, +2 margin; the
           // kernels clamp footprints to the volume, whose extent bounds the box
-          const int Ne = dom ? g.nx : g.ny;
           // a slab where the tile's rays are beside the volume holds no samples
           if (!beside && (emx < -1.0 || emn > Ne)) continue;
           a.e = std::max(a.e, std::min((int)(std::floor(emx) - std::floor(emn)) + 3 + 2, Ne + 4));
@@ -1245,6 +1259,10 @@ static double row_dz_max(const cbct_plan* p) {
   return m;
 }
 
+// Row distances (texels) from which launches take the slab kernel at any size (see
+// launch_variant), fp32 and 16-bit volumes.
+constexpr double kRowsApart = 1.2, kRowsApart16 = 1.0;
+
 // Chooses the forward variant and its TMA boxes from the plan geometry: the
 // row-quad kernel by quad_choose's rule, else the row-pair kernel where adjacent
 // detector rows are less than one z texel apart over the whole volume (so pairs
@@ -1277,8 +1295,11 @@ void forward_choose_variant(cbct_plan* p) {
   p->fwd_fill_rays = height <= p->g.nz ? 8e5 : row_dz < 0.9 ? 2e6 : 3e6;
   if ((p->fwd_pref == 0 || p->fwd_pref == 5) && quad_choose(p, row_dz, p->fwd_pref == 5)) {
     p->fwd_variant = 4;
-    if (p->fwd_pref == 0) slab_choose(p);
-    else p->fwd_wide = 0;
+    // The slab kernel's boxes, where launch_variant may take it for some view range.
+    bool slab = row_dz >= kRowsApart16;
+    for (int c : p->count) slab = slab || (c > 0 && double(p->g.width) * p->g.height * c < p->fwd_fill_rays);
+    if (p->fwd_pref == 5) p->fwd_wide = 0;
+    else if (slab) slab_choose(p);
     return;
   }
   int e, z;
@@ -1333,7 +1354,7 @@ void forward_choose_variant(cbct_plan* p) {
 static int launch_variant(const cbct_plan* p, int cnt, size_t es) {
   const bool rows = p->fwd_variant == 3 || p->fwd_variant == 4;
   const double rays = double(p->g.width) * p->g.height * cnt;
-  if (rows && p->fwd_pref == 0 && p->slab.bx && (rays < p->fwd_fill_rays || p->fwd_row_dz >= (es == 2 ? 1.0 : 1.2)))
+  if (rows && p->fwd_pref == 0 && p->slab.bx && (rays < p->fwd_fill_rays || p->fwd_row_dz >= (es == 2 ? kRowsApart16 : kRowsApart)))
     return 1;
   // The gather form is compiled for the slab and quad kernels.
   if (forward_lerp_gather(p, es) && (p->fwd_variant == 2 || p->fwd_variant == 3)) return p->slab.bx ? 1 : 0;
