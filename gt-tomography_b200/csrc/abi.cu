@@ -56,9 +56,19 @@ void ensure_smem_attr(const void* func, size_t bytes) {
 
 void* plan_alloc(cbct_plan* p, size_t bytes) {
   if (bytes == 0) return nullptr;
+  void* ptr = plan_try_alloc(p, bytes);
+  if (!ptr) throw Error(CBCT_ERR_OUT_OF_MEMORY, "plan buffer of " + std::to_string(bytes) + " bytes: out of memory");
+  return ptr;
+}
+
+void* plan_try_alloc(cbct_plan* p, size_t bytes) {
   void* ptr = nullptr;
-  if (p->pool) CBCT_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, p->pool, p->pool_stream));
-  else CBCT_CUDA(cudaMalloc(&ptr, bytes));
+  const cudaError_t e = p->pool ? cudaMallocFromPoolAsync(&ptr, bytes, p->pool, p->pool_stream) : cudaMalloc(&ptr, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  CBCT_CUDA(e);
   p->allocs.emplace_back(ptr, bytes);
   p->dev_bytes += bytes;
   p->dev_bytes_peak = std::max(p->dev_bytes_peak, p->dev_bytes);
@@ -231,7 +241,7 @@ void plan_free(cbct_plan* p) {
 
 cbct_plan* plan_create(const cbct_geometry* g, const float* angles, const float* offsets, int n_views,
                        const int* subset_sizes, int n_subsets, const int* offcorr, cudaMemPool_t pool,
-                       cudaStream_t pool_stream, bool forward_buffers) {
+                       cudaStream_t pool_stream, bool forward_buffers, bool pads) {
   validate_geometry(g);
   CBCT_REQUIRE(n_views > 0, "n_views must be positive");
   CBCT_REQUIRE(angles && offsets, "angles/offsets are NULL");
@@ -270,6 +280,7 @@ cbct_plan* plan_create(const cbct_geometry* g, const float* angles, const float*
     p->hviews.push_back(make_view(*g, angles[i], offsets[2 * i], offsets[2 * i + 1]));
   }
   CBCT_CUDA(cudaGetDevice(&p->device));
+  p->pads = pads;
   p->pool = pool;
   p->pool_stream = pool_stream;
   p->d_views = plan_alloc_n<ViewParams>(p.get(), n_views);

@@ -632,6 +632,7 @@ void launch_bp(cbct_plan* p, int s, const float* proj, const BpEpi& e, cudaStrea
   const int first = p->first[s], cnt = p->count[s];
   if (cnt == 0) return;
   if (EPI == kStore && p->bp_variant == 1 && p->bp_pad_views > 0 && cnt > p->bp_pad_views) {
+    if (cnt > kMaxViewsSmem) throw Error(CBCT_ERR_UNSUPPORTED, "more than 1024 views in one back-projection");
     const size_t plane = (size_t)p->g.width * p->g.height;
     for (int i = 0; i < cnt; i += p->bp_pad_views) {
       BpEpi c = e;
@@ -741,9 +742,11 @@ void backproject_prepare(cbct_plan* p) {
     with_bp(p->bp_box.bx, p->bp_run, [&](auto W, auto Z) {
       prepare_bp_all<decltype(W)::value, decltype(Z)::value>(sm, p->g.width % 4 != 0);
     });
-    if (bp_pad_bytes(p->g, p->max_subset) && !p->d_bp_pad) {
-      p->d_bp_pad = static_cast<float*>(plan_alloc(p, bp_pad_bytes(p->g, p->max_subset)));
-      p->bp_pad_views = std::min(p->max_subset, kBpPadViews);
+    // Where the device has no room for the padded copy, the global-load kernel runs, whose
+    // results are the same.
+    if (bp_pad_bytes(p->g, p->max_subset) && !p->d_bp_pad && p->pads) {
+      p->d_bp_pad = static_cast<float*>(plan_try_alloc(p, bp_pad_bytes(p->g, p->max_subset)));
+      if (p->d_bp_pad) p->bp_pad_views = std::min(p->max_subset, kBpPadViews);
     }
   }
   const size_t smem = sizeof(ViewParams) * (size_t)std::min(p->n_views, kMaxViewsSmem);

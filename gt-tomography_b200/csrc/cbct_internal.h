@@ -228,6 +228,8 @@ struct cbct_plan {
   cbct::SlabBox bp_box{};   // detector box (bx = u width, by = v rows)
   int bp_run = 0;           // its runs along z (index into backproject.cu's kZRuns)
   int bp_max_views = 0;     // views per launch the TMA back-projector holds
+  int pads = 1;             // row-padded copies wanted (0: a request whose budget has no room for them)
+  int volT_plain = 0;       // d_volT has room for the unpadded transpose only
   float* d_bp_pad = nullptr;  // row-padded projections where W is not a multiple of 4 (bp_pad_bytes)
   int bp_pad_views = 0;     // views it holds
 
@@ -288,6 +290,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 // stream order (see cbct_plan::pool).  plan_upload copies host data that may
 // be released as soon as the call returns.
 void* plan_alloc(cbct_plan* p, size_t bytes);
+void* plan_try_alloc(cbct_plan* p, size_t bytes);   // NULL where the device has no room
 void plan_dealloc(cbct_plan* p, void* ptr);
 void plan_upload(cbct_plan* p, void* dst, const void* src, size_t bytes);
 void plan_memset(cbct_plan* p, void* dst, int value, size_t bytes);
@@ -398,9 +401,10 @@ void plan_check_flags(cbct_plan* p, cudaStream_t st);
 bool stream_capturing(cudaStream_t st);
 // forward_buffers = false leaves out the forward projector's transposed-volume
 // buffer (plans that only back-project; their forward calls take the gather path).
+// pads = false leaves out the row-padded copies (see forward_prepare).
 cbct_plan* plan_create(const cbct_geometry* g, const float* angles, const float* offsets, int n_views,
                        const int* subset_sizes, int n_subsets, const int* offcorr, cudaMemPool_t pool,
-                       cudaStream_t pool_stream, bool forward_buffers);
+                       cudaStream_t pool_stream, bool forward_buffers, bool pads = true);
 void plan_free(cbct_plan* p);
 bool short_scan_rule(const cbct_geometry& g, const float* angles, int n);
 bool offset_override_rule(const cbct_geometry& g, const float* offsets, int n);

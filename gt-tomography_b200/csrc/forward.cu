@@ -969,7 +969,7 @@ bool needs_padded_rows(const void* vol, int nx, size_t es) {
 // 16-bit volumes keep theirs behind the transposed copy (d_volT has fp32 room).
 void* padded_rows(cbct_plan* p, size_t es) {
   if (p->g.nx % 4 != 0) return p->d_volP;
-  if (es == 2 && p->g.nx % 8 != 0 && p->d_volT) return static_cast<char*>(p->d_volT) + volT16_bytes(p->g);
+  if (es == 2 && p->g.nx % 8 != 0 && p->d_volT && !p->volT_plain) return static_cast<char*>(p->d_volT) + volT16_bytes(p->g);
   return nullptr;
 }
 
@@ -1370,8 +1370,20 @@ void forward_prepare(cbct_plan* p) {
   if (p->fwd_variant == 4) quad_prepare(p);
   bool any_x = false;
   for (size_t s = 0; s < p->subset_has_xdom.size(); ++s) any_x = any_x || p->subset_has_xdom[s];
-  if (any_x && !p->d_volT) p->d_volT = plan_alloc(p, volT_bytes(p->g));
-  if (volP_bytes(p->g) && !p->d_volP) p->d_volP = plan_alloc(p, volP_bytes(p->g));
+  // Row-padded copies are made where the device has room for them: without, launches over
+  // rows that TMA cannot read run the gather kernel, whose rays through the volume they
+  // are anyway.
+  const size_t plain = (size_t)p->g.nx * p->g.ny * p->g.nz * 4;
+  const bool padded = volT_bytes(p->g) > plain || volP_bytes(p->g);
+  if (any_x && !p->d_volT) {
+    if (!padded) p->d_volT = plan_alloc(p, plain);
+    else if (p->pads) p->d_volT = plan_try_alloc(p, volT_bytes(p->g));
+    if (!p->d_volT && p->g.nx % 4 == 0 && p->g.ny % 4 == 0) {   // aligned fp32 launches need theirs
+      p->d_volT = plan_alloc(p, plain);
+      p->volT_plain = 1;
+    }
+  }
+  if (volP_bytes(p->g) && !p->d_volP && p->pads && (!any_x || p->d_volT)) p->d_volP = plan_try_alloc(p, volP_bytes(p->g));
 }
 
 void forward_launch(cbct_plan* p, int s, cbct_dtype dt, const void* vol, float* out, const float* b,
@@ -1398,7 +1410,7 @@ void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, floa
   o.wproj = p->d_pweights ? p->d_pweights + (size_t)p->g.width * p->g.height * p->first[s] : nullptr;
   const size_t es = dtype_size(dt);
   const bool tma = (!needs_padded_rows(vol, p->g.nx, es) || padded_rows(p, es) != nullptr) &&
-                   (!p->subset_has_xdom[s] || p->d_volT != nullptr);
+                   (!p->subset_has_xdom[s] || (p->d_volT != nullptr && !(p->volT_plain && forward_lerp_gather(p, es))));
   const int variant = tma ? launch_variant(p, cnt, es) : 0;
   // One partial sum per block of the kernel that will run.
   int TU = kTU, TV = kTV;

@@ -42,6 +42,7 @@ struct Request {
   cbct_request r{};
   std::vector<float> angles, offsets, filter;
   size_t bytes = 0;
+  bool pads = true;      // row-padded copies in the reservation
   double t_submit = 0, t_admit = 0, t_done = 0;
   int bypassed = 0;
   int slot = -1;
@@ -68,7 +69,9 @@ void validate_request(const cbct_request& r) {
 // Device footprint: every buffer plan_alloc will hand out for this request,
 // each with a rounding allowance.  Mirrors plan_create, forward_prepare,
 // fdk_state, fdk_run, osmom_solve's workspace and the request's own buffers.
-size_t request_bytes(const cbct_request& r) {
+// pads: the row-padded copies of the projectors too, which a plan does without where the
+// budget has no room for them.
+size_t request_bytes(const cbct_request& r, bool pads = true) {
   const cbct_geometry& g = r.geometry;
   const size_t P = (size_t)r.n_views, pl = plane(g), nv = (size_t)g.nx * g.ny * g.nz;
   const size_t tiles = forward_tiles(g.width, g.height);
@@ -81,7 +84,7 @@ size_t request_bytes(const cbct_request& r) {
   add(pl * P * dtype_size(r.storage));  // projections
   add(nv * sizeof(float));              // volume
   const int sub = r.kind == CBCT_REQ_FDK ? r.n_views : (r.n_views + r.n_subsets - 1) / r.n_subsets;
-  if (bp_pad_bytes(g, sub)) add(bp_pad_bytes(g, sub));  // row-padded projections of the back-projector
+  if (pads && bp_pad_bytes(g, sub)) add(bp_pad_bytes(g, sub));  // row-padded projections of the back-projector
   if (r.kind == CBCT_REQ_FDK) {
     size_t L = 2;
     while (L < 2 * (size_t)g.width - 1) L <<= 1;
@@ -92,8 +95,8 @@ size_t request_bytes(const cbct_request& r) {
     add(sizeof(float) * g.width * P);
     if (r.storage != CBCT_F32) add(sizeof(float) * pl * P);  // FP32 filtered copy
   } else {
-    add(volT_bytes(g));       // volume copies of the forward projector (upper bound)
-    if (volP_bytes(g)) add(volP_bytes(g));
+    add(pads ? volT_bytes(g) : nv * sizeof(float));   // volume copies of the forward projector (upper bound)
+    if (pads && volP_bytes(g)) add(volP_bytes(g));
     add((2 * nv + pl * P) * sizeof(float));  // solver workspace (FP32 volume input)
   }
   return b + n * kAllocSlack;
@@ -187,7 +190,7 @@ void run_request(cbct_server* sv, Request& q, cudaStream_t st) {
   }
   std::unique_ptr<cbct_plan, void (*)(cbct_plan*)> plan(
       plan_create(&g, ang.data(), off.data(), P, sizes.data(), S, offcorr.data(), sv->pool, st,
-                  r.kind == CBCT_REQ_OSMOM),
+                  r.kind == CBCT_REQ_OSMOM, q.pads),
       plan_free);
   cbct_plan* p = plan.get();
   const float* filter = q.filter.empty() ? nullptr : q.filter.data();
@@ -335,6 +338,10 @@ cbct_status cbct_server_submit(cbct_server* sv, const cbct_request* req, uint64_
     q->r.offsets_xy = nullptr;
     q->r.filter = nullptr;
     q->bytes = request_bytes(*req);
+    if (q->bytes > sv->cfg.hbm_budget_bytes) {
+      q->pads = false;
+      q->bytes = request_bytes(*req, false);
+    }
     if (q->bytes > sv->cfg.hbm_budget_bytes)
       throw Error(CBCT_ERR_BUDGET, "request needs " + std::to_string(q->bytes) + " device bytes; the budget is " +
                                        std::to_string(sv->cfg.hbm_budget_bytes));

@@ -519,7 +519,8 @@ CBCT_API cbct_status cbct_host_backproject(cbct_plan* plan, int32_t s_first, int
  * with its own CUDA stream, and a stream-ordered device memory pool.  A
  * submitted request waits until a slot is idle and its device footprint
  * (cbct_server_request_bytes) fits into what the admitted requests leave of
- * the budget; the oldest waiting request that fits is admitted first, and a
+ * the budget (without its row-padded copies, where the whole budget has no room for
+ * them); the oldest waiting request that fits is admitted first, and a
  * request passed over 8 times blocks younger ones until it fits.  An admitted
  * request builds its plan (set-up rules of CBSubsetOperator::setup and
  * hoCuConebeamProjectionOperator::setup), copies its projections host ->
@@ -568,7 +569,8 @@ typedef struct {
 
 CBCT_API cbct_status cbct_server_create(const cbct_server_config* cfg, cbct_server** server_out);
 
-/* Device bytes the request will hold while it runs (its admission footprint). */
+/* Device bytes the request will hold while it runs (its admission footprint), the
+ * row-padded copies of odd sizes included, which it can do without. */
 CBCT_API cbct_status cbct_server_request_bytes(const cbct_request* req, size_t* bytes_out);
 
 /* Queues a request; returns at once.  CBCT_ERR_BUDGET when its footprint
