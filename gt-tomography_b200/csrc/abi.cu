@@ -328,6 +328,32 @@ bool stream_capturing(cudaStream_t st) {
   return cs != cudaStreamCaptureStatusNone;
 }
 
+ScratchUse::ScratchUse(ScratchOrder& o, cudaStream_t st, bool on) : o_(o), st_(st), on_(on) {
+  if (!on_) return;
+  lock_ = std::unique_lock<std::mutex>(o_.mu);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamGetCaptureInfo(st_, &cs, &capture_) != cudaSuccess) {
+    (void)cudaGetLastError();   // the legacy stream while another captures: nothing can be ordered
+    on_ = false;
+    return;
+  }
+  k_ = cs != cudaStreamCaptureStatusNone;
+  if (k_) id_ = reinterpret_cast<uintptr_t>(st_);   // ids cannot be asked for under capture
+  else CBCT_CUDA(cudaStreamGetId(st_, &id_));
+  if (!o_.done[k_]) {
+    CBCT_CUDA(cudaEventCreateWithFlags(&o_.done[k_], cudaEventDisableTiming));
+    return;
+  }
+  if (o_.stream[k_] != id_ && (k_ == 0 || o_.capture == capture_)) CBCT_CUDA(cudaStreamWaitEvent(st_, o_.done[k_], 0));
+}
+
+ScratchUse::~ScratchUse() {
+  if (!on_) return;
+  if (cudaEventRecord(o_.done[k_], st_) != cudaSuccess) (void)cudaGetLastError();
+  o_.stream[k_] = id_;
+  if (k_) o_.capture = capture_;
+}
+
 void plan_check_flags(cbct_plan* p, cudaStream_t st) {
   int h[4] = {0, 0, 0, 0};
   CBCT_CUDA(cudaMemcpyAsync(h, p->d_flags, sizeof(h), cudaMemcpyDeviceToHost, st));

@@ -581,8 +581,9 @@ template <int EPI, bool FDK>
 bool try_bp_tma(cbct_plan* p, int first, int cnt, const float* proj, const BpEpi& e, cudaStream_t st) {
   if (p->bp_variant != 1 || cnt > p->bp_max_views) return false;
   const bool pad = needs_padded_rows(p, proj);
+  if (pad && cnt > p->bp_pad_views) return false;
+  ScratchUse use(p->bp_order, st, pad);   // the global-load kernel needs no scratch: any stream may call
   if (pad) {
-    if (cnt > p->bp_pad_views) return false;
     const int rows = p->g.height * cnt;
     pad_rows_kernel<<<std::min((rows + 7) / 8, 148 * 16), 256, 0, st>>>(proj, p->d_bp_pad, p->g.width,
                                                                        tma_pitch(p->g.width, 4), rows);

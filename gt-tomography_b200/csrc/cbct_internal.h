@@ -9,6 +9,7 @@
 #include <functional>
 #include <new>
 #include <stdexcept>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -192,6 +193,41 @@ inline size_t forward_tiles(int W, int H) {
 }  // namespace cbct
 
 // ---------------------------------------------------------------- the plan
+namespace cbct {
+
+// Launches that fill and read one scratch buffer of a plan, from any stream or host thread:
+// each waits for the last one's event unless it is on the same stream.  Under capture it
+// waits for the last one of the same capture; a graph's replays and eager calls are the
+// caller's to order.
+struct ScratchOrder {
+  std::mutex mu;
+  cudaEvent_t done[2] = {nullptr, nullptr};      // of the last eager and the last captured use
+  unsigned long long stream[2] = {0, 0};         // their streams (cudaStreamGetId, handle)
+  unsigned long long capture = 0;                // and the latter's capture
+  ~ScratchOrder() {
+    for (cudaEvent_t e : done)
+      if (e) cudaEventDestroy(e);
+  }
+};
+
+class ScratchUse {
+ public:
+  ScratchUse(ScratchOrder& o, cudaStream_t st, bool on);   // abi.cu; on = false: does nothing
+  ~ScratchUse();
+  ScratchUse(const ScratchUse&) = delete;
+  ScratchUse& operator=(const ScratchUse&) = delete;
+
+ private:
+  ScratchOrder& o_;
+  cudaStream_t st_;
+  bool on_;
+  int k_ = 0;                                    // 1 under capture
+  unsigned long long id_ = 0, capture_ = 0;
+  std::unique_lock<std::mutex> lock_;
+};
+
+}  // namespace cbct
+
 struct cbct_plan {
   cbct_geometry g{};
   cbct::GridConst gc{};
@@ -228,6 +264,7 @@ struct cbct_plan {
   cbct::SlabBox bp_box{};   // detector box (bx = u width, by = v rows)
   int bp_run = 0;           // its runs along z (index into backproject.cu's kZRuns)
   int bp_max_views = 0;     // views per launch the TMA back-projector holds
+  cbct::ScratchOrder fwd_order, bp_order;   // of d_volT and d_volP of odd sizes, and of d_bp_pad
   int pads = 1;             // row-padded copies wanted (0: a request whose budget has no room for them)
   int volT_plain = 0;       // d_volT has room for the unpadded transpose only
   float* d_bp_pad = nullptr;  // row-padded projections where W is not a multiple of 4 (bp_pad_bytes)

@@ -989,6 +989,9 @@ void launch_typed(cbct_plan* p, int s, const void* vol_v, const FwdOut& o, cudaS
   const int pitchT = tma_pitch(p->g.ny, sizeof(V)), pitchP = tma_pitch(p->g.nx, sizeof(V));
   V* const volT = p->subset_has_xdom[s] ? static_cast<V*>(p->d_volT) : nullptr;
   V* const pad = needs_padded_rows(vol, p->g.nx, sizeof(V)) ? static_cast<V*>(padded_rows(p, sizeof(V))) : nullptr;
+  // Odd sizes: calls that the gather kernel would take without scratch may come from
+  // several streams.
+  ScratchUse use(p->fwd_order, st, (volT || pad) && (p->g.nx % 8 || p->g.ny % 8));
   if (volT || pad) {
     const int nx = p->g.nx, ny = p->g.ny, nz = p->g.nz;
     if (sizeof(V) == 2 && nx % 2 == 0 && reinterpret_cast<uintptr_t>(vol) % 4 == 0) {

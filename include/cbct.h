@@ -17,6 +17,12 @@
  * Device pointers are CUDA global-memory pointers of the current device.
  * All device work is enqueued on the caller's stream (0 = legacy default
  * stream); no entry point synchronises the device unless documented.
+ * Calls on one plan share buffers that it owns (transposed volumes, weighted
+ * projections, partial sums, FDK, solver and host-operator workspaces): order
+ * them on one stream or by events.  Two kinds may run on several streams and
+ * host threads at once, as they need no such buffer or the library orders its
+ * use: cbct_backproject without weights, and cbct_forward of volumes whose
+ * rows (nx or ny) are not a multiple of 16 bytes.
  */
 #ifndef CBCT_H_
 #define CBCT_H_
