@@ -234,8 +234,6 @@ void plan_free(cbct_plan* p) {
   fdk_state_free(p);
   graph_cache_free(p);
   while (!p->allocs.empty()) plan_dealloc(p, p->allocs.back().first);
-  for (cudaStream_t s : p->host_streams)
-    if (s) cudaStreamDestroy(s);
   delete p;
 }
 

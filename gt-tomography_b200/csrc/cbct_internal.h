@@ -283,7 +283,6 @@ struct cbct_plan {
   float* d_stream_buf[2] = {nullptr, nullptr};  // batch buffers of the host-array operators
   size_t stream_buf_elems = 0;
   float* d_stream_vol = nullptr;    // bin volume of the host-array operators
-  cudaStream_t host_streams[2] = {nullptr, nullptr};  // their compute and copy streams (made on first use)
 
   // solver workspace (allocated on first solve, reused)
   float* ws = nullptr;

@@ -13,6 +13,8 @@
 // acquisition indices (conebeam_projection.cu:744-761).  Host arrays should be
 // page-locked for the transfers to overlap the kernels; the calls return once
 // the host outputs are written.
+#include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "cbct_internal.h"
@@ -25,24 +27,60 @@ void backproject_launch(cbct_plan* p, int s, const float* proj, float* vol, int 
 
 namespace {
 
-// The plan's two streams and the events between them; both streams are idle and the
-// events released on every exit path.  The streams are made on first use and kept with
-// the plan: making and destroying a pair takes 220 us, a fifth of an FBP call of 180
-// views of 256x192 into 128^3 (1.15 ms; 0.93 with the plan's streams, of which 0.80 are
-// the two transfers).
-struct Pipe {
+// Idle pairs of compute and copy streams, kept for the next call of any plan: making and
+// destroying a pair takes 220 us, a fifth of an FBP call of 180 views of 256x192 into 128^3
+// (1.15 ms; 0.93 with a kept pair, of which 0.80 are the two transfers).  A call takes a
+// pair of its device for itself and gives it back idle; at most kIdlePairs are kept per
+// device, those of more calls at once are destroyed.
+struct StreamPair {
+  int device;
   cudaStream_t compute, copy;
+};
+constexpr int kIdlePairs = 4;
+std::mutex idle_mutex;
+std::vector<StreamPair>& idle_pairs() {
+  static auto* pairs = new std::vector<StreamPair>;   // not destroyed: the driver may be gone by then
+  return *pairs;
+}
+
+// A call's two streams and the events between them; both streams are idle and the events
+// released on every exit path.
+struct Pipe {
+  int device;
+  cudaStream_t compute = nullptr, copy = nullptr;
   std::vector<cudaEvent_t> events;
-  explicit Pipe(cbct_plan* p) {
-    for (cudaStream_t& s : p->host_streams)
-      if (!s) CBCT_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    compute = p->host_streams[0];
-    copy = p->host_streams[1];
+  explicit Pipe(const cbct_plan* p) : device(p->device) {
+    {
+      std::lock_guard<std::mutex> lock(idle_mutex);
+      auto& idle = idle_pairs();
+      const auto it = std::find_if(idle.begin(), idle.end(), [&](const StreamPair& s) { return s.device == device; });
+      if (it != idle.end()) {
+        compute = it->compute;
+        copy = it->copy;
+        idle.erase(it);
+        return;
+      }
+    }
+    CBCT_CUDA(cudaStreamCreateWithFlags(&compute, cudaStreamNonBlocking));
+    if (const cudaError_t e = cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking); e != cudaSuccess) {
+      cudaStreamDestroy(compute);
+      CBCT_CUDA(e);
+    }
   }
+  Pipe(const Pipe&) = delete;
   ~Pipe() {
-    cudaStreamSynchronize(compute);
-    cudaStreamSynchronize(copy);
+    const bool ok = (cudaStreamSynchronize(compute) == cudaSuccess) & (cudaStreamSynchronize(copy) == cudaSuccess);
     for (cudaEvent_t e : events) cudaEventDestroy(e);
+    if (ok) {
+      std::lock_guard<std::mutex> lock(idle_mutex);
+      auto& idle = idle_pairs();
+      if (std::count_if(idle.begin(), idle.end(), [&](const StreamPair& s) { return s.device == device; }) < kIdlePairs) {
+        idle.push_back({device, compute, copy});
+        return;
+      }
+    }
+    cudaStreamDestroy(compute);
+    cudaStreamDestroy(copy);
   }
   cudaEvent_t record(cudaStream_t s) {
     cudaEvent_t e;
