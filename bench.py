@@ -429,7 +429,7 @@ def ours(args, wl: Workload):
     rays0 = wl.W * wl.H * n0
     alg_bytes = 4 * nvox + 4 * rays0 * 3        # volume + b read + r write (+ per-pixel offset weight computed)
     hbm, peak_kind = peaks()
-    variant = plan.forward_variant()
+    variant = plan.launch_variant(s0)
     achieved = alg_bytes / t_fwd / 1e9
     samples_s = rays0 * wl.Nsamp / t_fwd
 
@@ -672,7 +672,7 @@ def kernel_only(args, wl: Workload):
     e1.record(stream)
     e1.synchronize()
     print(json.dumps({"kernel": args.only, "ms_per_launch": e0.elapsed_time(e1) / max(args.steps, 1),
-                      "variant": plan.forward_variant(), "views": n0}), flush=True)
+                      "variant": plan.launch_variant(s0), "views": n0}), flush=True)
 
 
 def batched(args):

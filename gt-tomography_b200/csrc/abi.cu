@@ -488,13 +488,15 @@ cbct_status cbct_plan_subset(const cbct_plan* plan, int32_t s, int32_t* first_ou
   });
 }
 
-const char* cbct_plan_forward_variant(const cbct_plan* plan) {
-  if (!plan) return "";
-  return plan->fwd_variant == 4   ? "tma-quad"
-         : plan->fwd_variant == 3 ? "tma-pair"
-         : plan->fwd_variant == 2 ? "tma-fan"
-         : plan->fwd_variant == 1 ? "tma-slab"
-                                  : "gather";
+static const char* variant_name(int v) {
+  return v == 4 ? "tma-quad" : v == 3 ? "tma-pair" : v == 2 ? "tma-fan" : v == 1 ? "tma-slab" : "gather";
+}
+
+const char* cbct_plan_forward_variant(const cbct_plan* plan) { return plan ? variant_name(plan->fwd_variant) : ""; }
+
+const char* cbct_plan_launch_variant(const cbct_plan* plan, int32_t s, cbct_dtype vol_dtype) {
+  if (!plan || s < -1 || s >= plan->n_subsets || (unsigned)vol_dtype > CBCT_BF16) return "";
+  return variant_name(forward_variant_of(plan, s < 0 ? plan->n_subsets : s, vol_dtype));
 }
 
 cbct_status cbct_plan_set_option(cbct_plan* plan, int32_t option, int32_t value) {

@@ -1,7 +1,7 @@
 // autotune.cu -- choose the projector variants of a plan by timing them.
 //
 // Which forward projector is fastest depends on the geometry: the slab kernel
-// (16x16 ray tiles, per-ray trilinear samples from TMA boxes), the row-pair
+// (a warp per 8x4 rays, per-ray trilinear samples from TMA boxes), the row-pair
 // and row-quad kernels (two or four rays of a column per thread sharing their
 // in-plane interpolation), the fan kernel (8x32 tiles, e/d interpolation shared by a
 // detector column; larger boxes), or the gather kernel (no staging); likewise

@@ -369,6 +369,8 @@ inline size_t bp_pad_bytes(const cbct_geometry& g, int max_subset) {
 
 // forward.cu
 void forward_prepare(cbct_plan* p);
+// Kernel that view range s launches for volumes of type dt (variants as cbct_plan::fwd_variant).
+int forward_variant_of(const cbct_plan* p, int s, cbct_dtype dt);
 // b: measured projections of storage type b_dtype (residual mode).
 void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, float* out, const void* b,
                        const float* pw, float scale, int mode, int apply_offset, int accumulate,

@@ -967,7 +967,7 @@ bool needs_padded_rows(const void* vol, int nx, size_t es) {
 
 // Plan buffer for a row-padded copy of a volume of element size es, or NULL.
 // 16-bit volumes keep theirs behind the transposed copy (d_volT has fp32 room).
-void* padded_rows(cbct_plan* p, size_t es) {
+void* padded_rows(const cbct_plan* p, size_t es) {
   if (p->g.nx % 4 != 0) return p->d_volP;
   if (es == 2 && p->g.nx % 8 != 0 && p->d_volT && !p->volT_plain) return static_cast<char*>(p->d_volT) + volT16_bytes(p->g);
   return nullptr;
@@ -1296,13 +1296,16 @@ void forward_choose_variant(cbct_plan* p) {
   const double row_dz = p->fwd_row_dz = row_dz_max(p);
   const double height = double(p->g.fov_v) * (p->g.SAD / p->g.SDD) * p->g.nz / p->g.lz;
   p->fwd_fill_rays = height <= p->g.nz ? 8e5 : row_dz < 0.9 ? 2e6 : 3e6;
-  if ((p->fwd_pref == 0 || p->fwd_pref == 5) && quad_choose(p, row_dz, p->fwd_pref == 5)) {
+  // Rows so far apart that no launch would take quads (launch_variant), where the slab
+  // kernel's boxes fit.
+  const bool apart = p->fwd_pref == 0 && row_dz >= kRowsApart && slab_choose(p);
+  if (!apart && (p->fwd_pref == 0 || p->fwd_pref == 5) && quad_choose(p, row_dz, p->fwd_pref == 5)) {
     p->fwd_variant = 4;
     // The slab kernel's boxes, where launch_variant may take it for some view range.
     bool slab = row_dz >= kRowsApart16;
     for (int c : p->count) slab = slab || (c > 0 && double(p->g.width) * p->g.height * c < p->fwd_fill_rays);
     if (p->fwd_pref == 5) p->fwd_wide = 0;
-    else if (slab) slab_choose(p);
+    if (p->fwd_pref == 0 && slab) slab_choose(p);
     return;
   }
   int e, z;
@@ -1364,6 +1367,15 @@ static int launch_variant(const cbct_plan* p, int cnt, size_t es) {
   return p->fwd_variant;
 }
 
+static int variant_of(const cbct_plan* p, int s, cbct_dtype dt, const void* vol) {
+  const size_t es = dtype_size(dt);
+  const bool tma = (!needs_padded_rows(vol, p->g.nx, es) || padded_rows(p, es) != nullptr) &&
+                   (!p->subset_has_xdom[s] || (p->d_volT != nullptr && !(p->volT_plain && forward_lerp_gather(p, es))));
+  return tma ? launch_variant(p, p->count[s], es) : 0;
+}
+
+int forward_variant_of(const cbct_plan* p, int s, cbct_dtype dt) { return variant_of(p, s, dt, nullptr); }
+
 void forward_prepare(cbct_plan* p) {
   if (p->fwd_variant < 1) return;
   prepare_typed<float>(p);
@@ -1411,10 +1423,7 @@ void forward_launch_ex(cbct_plan* p, int s, cbct_dtype dt, const void* vol, floa
   const int cnt = p->count[s];
   if (cnt == 0) return;
   o.wproj = p->d_pweights ? p->d_pweights + (size_t)p->g.width * p->g.height * p->first[s] : nullptr;
-  const size_t es = dtype_size(dt);
-  const bool tma = (!needs_padded_rows(vol, p->g.nx, es) || padded_rows(p, es) != nullptr) &&
-                   (!p->subset_has_xdom[s] || (p->d_volT != nullptr && !(p->volT_plain && forward_lerp_gather(p, es))));
-  const int variant = tma ? launch_variant(p, cnt, es) : 0;
+  const int variant = variant_of(p, s, dt, vol);
   // One partial sum per block of the kernel that will run.
   int TU = kTU, TV = kTV;
   if (variant == 1) slab_tile(TU, TV);

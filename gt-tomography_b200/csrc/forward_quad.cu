@@ -112,9 +112,10 @@ void quad_tile(int shape, int& TU, int& TV) {
 // boxes.  row_dz: largest distance of adjacent rows (texels).  Launches with too few
 // rays to fill the GPU run the slab kernel all the same (launch_variant).
 //  row_dz < 0.66: always (4 planes per quad).  Up to 0.9 where the largest subset has
-//  150,000 rays, up to 1.4 where it has a million: others have no launch that quads would
-//  gain on (180 views of 256x192 into 128^3 at 1.02 texel: 2.42 ms, slab kernel 2.47, row
-//  pairs 3.36; 8 views 0.22, 0.14 and 0.22).
+//  150,000 rays, up to 1.4 where it has a million (from 1.2 on the caller prefers the slab
+//  kernel where its boxes fit): others have no launch that quads would gain on (180 views
+//  of 256x192 into 128^3 at 1.09 texel: 2.42 ms, slab kernel 2.47, row pairs 3.36; 8 views
+//  0.22, 0.14 and 0.22).
 //  Shape: wide where its tiles are three waves and row_dz < 0.66 (20 views of 512x384
 //  into 160^3: 1.10 ms against 1.17 with the warp shape; 10 views of 192x144 into 64^3,
 //  0.3 waves: 0.139 against 0.115); warp up to 0.9 texel (25 views of 320x240 into

@@ -295,6 +295,10 @@ class Plan:
     def forward_variant(self) -> str:
         return L.lib().cbct_plan_forward_variant(self._h).decode()
 
+    def launch_variant(self, s=-1, vol_dtype=L.CBCT_F32) -> str:
+        """The projector that forward launches for subset s and this volume type."""
+        return L.lib().cbct_plan_launch_variant(self._h, s, vol_dtype).decode()
+
     def set_option(self, opt: int, value: int):
         L.call("cbct_plan_set_option", self._h, opt, int(value))
 

@@ -145,6 +145,11 @@ CBCT_API cbct_status cbct_plan_subset(const cbct_plan* plan, int32_t s, int32_t*
  * "tma-fan" or "gather"). */
 CBCT_API const char* cbct_plan_forward_variant(const cbct_plan* plan);
 
+/* Name of the variant that cbct_forward launches for subset s (-1: all views) of the plan
+ * and volumes of type vol_dtype that start on a 16-byte boundary: launches of few rays, of
+ * rows far apart or of odd sizes take another than the plan's ("" for bad arguments). */
+CBCT_API const char* cbct_plan_launch_variant(const cbct_plan* plan, int32_t s, cbct_dtype vol_dtype);
+
 /* Autotuner (no reference counterpart): runs every forward projector (slab,
  * column-fan, gather, row-pair, row-quad) and back-projector (TMA-staged,
  * global loads) the plan can use on its largest subset, keeps the fastest of
@@ -161,8 +166,8 @@ CBCT_API cbct_status cbct_plan_autotune(cbct_plan* plan, float* times_ms_out, vo
 #define CBCT_OPT_DEBUG_CHECKS 1
 #define CBCT_OPT_FORCE_GATHER 2
 /* CBCT_OPT_FORWARD_KERNEL: 0 = automatic (the row-quad kernel where adjacent
- * detector rows stay within 0.66 z texel of each other, and up to 1.4 texels in
- * launches with enough rays; else the row-pair kernel where rows stay within one
+ * detector rows stay within 0.66 z texel of each other, and up to 1.2 texels (16-bit
+ * volumes: 1) in launches with enough rays; else the row-pair kernel where rows stay within one
  * texel, else the per-ray slab kernel, each where its boxes fit, else gather; launches
  * too small to fill the GPU run the slab kernel in place of pairs or quads),
  * 1 = slab, 2 = gather, 3 = the column-fan kernel (e/d interpolation shared by the
