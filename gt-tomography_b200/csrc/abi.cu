@@ -511,6 +511,7 @@ cbct_status cbct_plan_set_option(cbct_plan* plan, int32_t option, int32_t value)
     } else if (option == CBCT_OPT_STATUS_CHECK) {
       plan->status_check = value != 0;
     } else if (option == CBCT_OPT_FORCE_GATHER || option == CBCT_OPT_FORWARD_KERNEL) {
+      plan->fwd_tuned_views = 0;
       if (option == CBCT_OPT_FORCE_GATHER) plan->force_gather = value != 0;
       else {
         CBCT_REQUIRE(value >= 0 && value <= 5, "forward kernel must be 0 (automatic), 1 (slab), 2 (gather), 3 (fan), "

@@ -8,8 +8,9 @@
 // the TMA-staged and the plain back-projector.  The autotuner runs every
 // candidate the plan can use on the plan's largest subset (one warm-up and
 // three timed launches each, CUDA events on the caller's stream) and keeps the
-// fastest.  All candidates give
-// results within FP32 rounding of each other (slab, pair, quad and fan bitwise
+// fastest, for launches of that many views: smaller ones keep the automatic plan's
+// rule (row pairs and quads lose launches of few rays to the slab kernel).  All candidates
+// give results within FP32 rounding of each other (slab, pair, quad and fan bitwise
 // equal).
 // No counterpart in the reference.
 #include <vector>
@@ -58,6 +59,7 @@ void plan_autotune(cbct_plan* p, float* times, cudaStream_t st) {
     // must be the one asked for; slot = its entry of times[]
     const int prefs[5] = {1, 3, 2, 4, 5}, want[5] = {1, 2, 0, 3, 4}, slot[5] = {0, 1, 2, 5, 6};
     const int saved_pref = p->fwd_pref;
+    p->fwd_tuned_views = 0;
     int best = -1;
     float best_ms = 0.f;
     for (int c = 0; c < 5; ++c) {
@@ -72,6 +74,7 @@ void plan_autotune(cbct_plan* p, float* times, cudaStream_t st) {
       if (best < 0 || ms < best_ms) { best = c; best_ms = ms; }
     }
     p->fwd_pref = best >= 0 ? prefs[best] : saved_pref;
+    p->fwd_tuned_views = best >= 0 ? p->count[s] : 0;
     forward_choose_variant(p);
     forward_prepare(p);
     // back-projection: TMA-staged boxes (pref 0) or global loads (pref 1)

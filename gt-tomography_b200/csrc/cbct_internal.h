@@ -245,6 +245,7 @@ struct cbct_plan {
   double fwd_fill_rays = 0; // row-pair and row-quad launches of fewer rays run the slab kernel (launch_variant)
   int fwd_wide = 0;         // pixels too wide for a box of 16 x 16 rays (forward_lerp_gather)
   double fwd_row_dz = 0;    // largest z distance of adjacent detector rows in the volume (texels)
+  int fwd_tuned_views = 0;  // autotuned plans: views of the subset fwd_pref was timed on (0: not autotuned)
   int fwd_pref = 0;         // CBCT_OPT_FORWARD_KERNEL: 0 automatic, 1 slab, 2 gather, 3 fan, 4 pair, 5 quad
   cbct::SlabBox pair{};     // row-pair kernel box for fp32 storage
   cbct::SlabBox pair16{};   // row-pair kernel box for 16-bit storage

@@ -1305,7 +1305,7 @@ void forward_choose_variant(cbct_plan* p) {
     bool slab = row_dz >= kRowsApart16;
     for (int c : p->count) slab = slab || (c > 0 && double(p->g.width) * p->g.height * c < p->fwd_fill_rays);
     if (p->fwd_pref == 5) p->fwd_wide = 0;
-    if (p->fwd_pref == 0 && slab) slab_choose(p);
+    if ((p->fwd_pref == 0 && slab) || p->fwd_tuned_views) slab_choose(p);
     return;
   }
   int e, z;
@@ -1360,7 +1360,8 @@ void forward_choose_variant(cbct_plan* p) {
 static int launch_variant(const cbct_plan* p, int cnt, size_t es) {
   const bool rows = p->fwd_variant == 3 || p->fwd_variant == 4;
   const double rays = double(p->g.width) * p->g.height * cnt;
-  if (rows && p->fwd_pref == 0 && p->slab.bx && (rays < p->fwd_fill_rays || p->fwd_row_dz >= (es == 2 ? kRowsApart16 : kRowsApart)))
+  const bool automatic = p->fwd_pref == 0 || cnt < p->fwd_tuned_views;
+  if (rows && automatic && p->slab.bx && (rays < p->fwd_fill_rays || p->fwd_row_dz >= (es == 2 ? kRowsApart16 : kRowsApart)))
     return 1;
   // The gather form is compiled for the slab and quad kernels.
   if (forward_lerp_gather(p, es) && (p->fwd_variant == 2 || p->fwd_variant == 3)) return p->slab.bx ? 1 : 0;
@@ -1522,7 +1523,7 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
     const bool tma = p->fwd_variant >= 1 && !forward_lerp_gather(p, sizeof(float)) &&
                      (reinterpret_cast<uintptr_t>(j.vol) % 16 == 0) && (!p->subset_has_xdom[s] || p->d_volT);
     int fv = launch_variant(p, cnt, sizeof(float));
-    if (fv == 1 && p->fwd_variant == 4 && p->fwd_pref == 0 && !j.norm2_out && all_rays >= kMultiQuadRays &&
+    if (fv == 1 && p->fwd_variant == 4 && (p->fwd_pref == 0 || p->fwd_tuned_views) && !j.norm2_out && all_rays >= kMultiQuadRays &&
         p->fwd_row_dz < (p->fwd_fill_rays < 1e6 ? 0.9 : 0.6))
       fv = 4;
     auto one_scan = [&A](const MultiFwdJob& jj) {

@@ -57,6 +57,22 @@ def test_names(gtb, cuda):
         assert plan.launch_variant() == name
 
 
+def test_autotuned_plans_keep_the_rule_of_small_launches(gtb, cuda):
+    """The autotuner times the largest subset; a launch of one view is not that."""
+    import torch
+    plan = _plan(gtb, (128, 128, 96), 256, 192, 0.7, [60, 1])
+    plan.autotune()
+    assert plan.launch_variant(0) == "tma-quad"     # three million rays
+    assert plan.launch_variant(1) == "tma-slab"
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(3)
+    vol = torch.rand(plan.vol_shape, generator=gen, device=cuda)
+    a = plan.forward(vol, torch.empty(plan.proj_shape(1), device=cuda), 1)
+    plan.set_option(gtb._lib.CBCT_OPT_FORWARD_KERNEL, 5)
+    assert plan.launch_variant(1) == "tma-quad"     # forced again
+    assert torch.equal(a, plan.forward(vol, torch.empty(plan.proj_shape(1), device=cuda), 1))
+
+
 # rows 0.8 texel apart under covered detectors, 0.5 under detectors taller than the volume:
 # scans of some 300,000 rays per subset, which take the slab kernel alone and quads in the
 # work lists of a batch (two groups of three)
