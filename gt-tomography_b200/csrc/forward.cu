@@ -1349,9 +1349,11 @@ void forward_choose_variant(cbct_plan* p) {
 // height covers, threshold 0.8 million rays: 2 views of 0.9 mm pixels into 128^3
 // (0.12 M rays) 0.088 to 0.173, 8 views (0.47 M) 0.223 to 0.232, 32 views (1.9 M) 0.829
 // to 0.692; 2 views of 0.75 mm into 256^3 (0.68 M) 0.54 to 0.71, 8 views (2.7 M) 2.07 to
-// 1.48.  Taller detectors, whose outer rays are cut, 2 million: 8 views of 0.9 mm into
-// 128^3 (0.52 M) 0.243 to 0.310, 32 views (2.1 M) 0.895 to 0.914, 40 views of 301x211
-// into 150x141x93 (2.5 M) 1.07 to 0.97; 3 million for rows 0.9 texel or more apart:
+// 1.48.  Taller detectors, whose outer rays are cut, 2 million, between
+// break-evens of 1 and 3 million by volume and detector: 4 views of 512x512 into 256^3 (1.0
+// M) 0.89 to 0.81, 8 views (2.1 M) 1.71 to 1.52; 304x208 into 152x144x96 20 views (1.3 M)
+// 0.57 to 0.60, 32 views (2.0 M) 0.88 to 0.86; 256x256 into 128^3 32 views (2.1 M) 0.86 to
+// 0.90, 48 views (3.1 M) 1.27 to 1.27; 3 million for rows 0.9 texel or more apart:
 // 2 views of 1.5 mm into 256^3 (0.2 M) 0.25 to 0.55, 64 views of 256x192 into 128^3
 // (3.1 M) 1.06 to 1.01.
 // Rows beyond 1.2 texels (16-bit volumes: 1) share too few planes at any size: 40 views of
@@ -1472,10 +1474,17 @@ FwdMultiKernel fwd_multi_ptr(int bx) {
   }
 }
 
-// Small scans that fill the GPU together run quads where their rows share enough planes
-// (up to 0.9 texel, 0.6 under detectors taller than the volume, whose outer rays are cut).
+// Small scans that fill the GPU together run quads where their rows share enough planes.
 // Their rays are bitwise the slab kernel's; a norm is summed tile by tile, so scans that
-// want theirs keep the kernel of their own launches.
+// want theirs keep the kernel of their own launches.  Whole batches of 2, 4 or 6 scans, us,
+// with quads and with the slab kernel:
+//  detectors that the volume's height covers, rows up to 0.9 texel, 300,000 rays a step: 0.45
+//  texel, 0.06 M rays 765, 720; 0.25 M 1487, 2045; 1.4 M 5493, 9486; 0.66 texel, 0.83 M 4559,
+//  6606; 0.77 texel, 0.9 M 4218, 3979; 0.85 texel, 0.52 M 3855, 4061; 1.2 M 7763, 8903;
+//  taller detectors, whose outer rays are cut, rows up to half a texel, 0.6 from three
+//  million rays a step: 0.42 texel, 0.08 M
+//  1247, 834; 0.31 M 2243, 2423; 1.7 M 11649, 11968; 0.53 texel, 0.81 M 7428, 6561; 0.56
+//  texel, 0.59 M 3923, 3731; 1.8 M 11084, 9221; 4.4 M 21097, 22172.
 constexpr double kMultiQuadRays = 3e5;
 
 // The scans of one kernel (kind, shape and box width).
@@ -1524,7 +1533,7 @@ void forward_multi(WorkArena& A, const std::vector<MultiFwdJob>& jobs) {
                      (reinterpret_cast<uintptr_t>(j.vol) % 16 == 0) && (!p->subset_has_xdom[s] || p->d_volT);
     int fv = launch_variant(p, cnt, sizeof(float));
     if (fv == 1 && p->fwd_variant == 4 && (p->fwd_pref == 0 || p->fwd_tuned_views) && !j.norm2_out && all_rays >= kMultiQuadRays &&
-        p->fwd_row_dz < (p->fwd_fill_rays < 1e6 ? 0.9 : 0.6))
+        p->fwd_row_dz < (p->fwd_fill_rays < 1e6 ? 0.9 : all_rays < 3e6 ? 0.5 : 0.6))
       fv = 4;
     auto one_scan = [&A](const MultiFwdJob& jj) {
       A.ops.push_back([jj](cudaStream_t st) {
