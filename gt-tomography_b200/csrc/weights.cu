@@ -887,10 +887,14 @@ void offset_weight_launch(cbct_plan* p, int s, const float* in, float* out, int 
   if (cnt == 0) return;
   const bool vec = p->g.width % 4 == 0 && (reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
   const int cols = vec ? 128 : 32;
-  const dim3 grid((p->g.width + cols - 1) / cols, (p->g.height + kOffRows - 1) / kOffRows, cnt), block(32, 8);
-  if (vec) offset_weight_kernel<4><<<grid, block, 0, st>>>(in, out, p->d_views + first, p->gc, variant);
-  else offset_weight_kernel<1><<<grid, block, 0, st>>>(in, out, p->d_views + first, p->gc, variant);
-  check_launch("offset_weight_kernel");
+  for (int i = 0; i < cnt; i += 65535) {   // views are the grid's z
+    const size_t o = (size_t)p->g.width * p->g.height * i;
+    const dim3 grid((p->g.width + cols - 1) / cols, (p->g.height + kOffRows - 1) / kOffRows, std::min(cnt - i, 65535));
+    const dim3 block(32, 8);
+    if (vec) offset_weight_kernel<4><<<grid, block, 0, st>>>(in + o, out + o, p->d_views + first + i, p->gc, variant);
+    else offset_weight_kernel<1><<<grid, block, 0, st>>>(in + o, out + o, p->d_views + first + i, p->gc, variant);
+    check_launch("offset_weight_kernel");
+  }
 }
 
 void fdk_prepare(cbct_plan* p, const float* filter) { fdk_state(p, filter); }
