@@ -146,7 +146,6 @@ __global__ void __launch_bounds__(kBX * kBY) bp_kernel(const float* __restrict__
     const bool u0ok = (unsigned)iu < (unsigned)gc.W, u1ok = (unsigned)(iu + 1) < (unsigned)gc.W;
     const int cu0 = min(max(iu, 0), gc.W - 1), cu1 = min(max(iu + 1, 0), gc.W - 1);
     const float* pv = proj + (size_t)p * plane;
-    const float dz = A * gc.vz;
     float cv = fmaf(A, z0, B);
 #pragma unroll
     for (int q = 0; q < kZB; ++q) {
@@ -164,7 +163,7 @@ __global__ void __launch_bounds__(kBX * kBY) bp_kernel(const float* __restrict__
       const float b = fmaf(au, p11 - p01, p01);
       const float s = fmaf(av, b - a, a);
       acc[q] = FDK ? fmaf(w, s, acc[q]) : acc[q] + s;
-      cv += dz;
+      cv = fmaf(A, gc.vz, cv);
     }
   }
 
@@ -400,7 +399,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
 #pragma unroll
         for (int q = h * SUB / 2; q < (h + 1) * SUB / 2; ++q) {   // two voxels, packed
           if (RUN == kFlatRun && q > 0 && q % 2 == 0 && 2 * q >= planes) break;
-          const float2 c = make_float2(cv, cv + dz);
+          const float2 c = make_float2(cv, fmaf(A, gc.vz, cv));   // one rounding a step
           const float2 bv = __fadd2_rd(c, make_float2(kRoundC, kRoundC));
           const float2 nf = __ffma2_rn(bv, make_float2(-1.f, -1.f), make_float2(kRoundC, kRoundC));   // -floor
           const float2 av = __fadd2_rn(c, nf);
@@ -413,7 +412,7 @@ __device__ __forceinline__ void bp_tma_body(const CUtensorMap* map, const ViewPa
           const float2 hi = GLOBAL ? __ffma2_rn(tu, __ffma2_rn(p01, none, p11), p01) : __ffma2_rn(tu, p11, __ffma2_rn(ntu, p01, p01));
           const float2 smp = __ffma2_rn(av, __ffma2_rn(lo, none, hi), lo);
           acc[q] = FDK ? __ffma2_rn(wt2, smp, acc[q]) : __fadd2_rn(acc[q], smp);
-          cv = c.y + dz;
+          cv = fmaf(A, gc.vz, c.y);
         }
       }
     }

@@ -7,10 +7,11 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _plan(gtb, n, W, H, pitch, P, ox=1.0):
+def _plan(gtb, n, W, H, pitch, P, ox=1.0, voxel=1.0):
     L = gtb._lib
-    g = L.CbctGeometry(1000.0, 1500.0, W * pitch, H * pitch, W, H, n[0], n[1], n[2], float(n[0]), float(n[1]),
-                       float(n[2]), 1.5)
+    m = voxel
+    g = L.CbctGeometry(1000.0, 1500.0, W * pitch * m, H * pitch * m, W, H, n[0], n[1], n[2], n[0] * m, n[1] * m,
+                       n[2] * m, 1.5)
     return gtb.Plan(g, (5.0 + np.arange(P) * (360.0 / P)).astype(np.float32),
                     np.tile(np.array([[ox, -0.5]], np.float32), (P, 1)))
 
@@ -24,8 +25,8 @@ def _rand(cuda, shape, seed):
 
 @pytest.mark.parametrize("fdk", [False, True])
 @pytest.mark.parametrize("nz", [64, 63, 96, 50])
-@pytest.mark.parametrize("pitch", [0.6, 1.2])
-def test_runs_of_32_are_runs_of_16(gtb, cuda, fdk, nz, pitch):
+@pytest.mark.parametrize("pitch,voxel", [(0.6, 1.0), (1.2, 1.0), (1.2, 0.75)])
+def test_runs_of_32_are_runs_of_16(gtb, cuda, fdk, nz, pitch, voxel):
     """256 x 256 columns have the CTAs for runs of 32, the 64 x 64 in their middle (the same
     blocks of 16 x 8 columns, exact coordinates) do not."""
     import torch
@@ -34,7 +35,7 @@ def test_runs_of_32_are_runs_of_16(gtb, cuda, fdk, nz, pitch):
     proj = _rand(cuda, (P, H, W), 1)
     outs = []
     for m in (256, 64):
-        plan = _plan(gtb, (m, m, nz), W, H, pitch, P)
+        plan = _plan(gtb, (m, m, nz), W, H, pitch, P, voxel=voxel)
         out = torch.full(plan.vol_shape, 0.25, dtype=torch.float32, device=cuda)
         plan.backproject(proj, out, -1, L.CBCT_BP_FDK_WEIGHT if fdk else 0, True, True)
         assert plan.read_flags() == (0, 0)
@@ -45,7 +46,8 @@ def test_runs_of_32_are_runs_of_16(gtb, cuda, fdk, nz, pitch):
 @pytest.mark.parametrize("n,W,H,pitch,P", [((30, 27, 21), 45, 34, 1.2, 7), ((48, 40, 33), 61, 50, 1.2, 128),
                                            ((44, 35, 16), 47, 40, 1.4, 5), ((256, 250, 70), 271, 100, 1.7, 6),
                                            ((256, 256, 64), 401, 220, 0.8, 6), ((64, 48, 5), 90, 30, 1.1, 5)])
-def test_padded_detectors_are_the_global_loads(gtb, cuda, n, W, H, pitch, P):
+@pytest.mark.parametrize("voxel", [1.0, 0.73])
+def test_padded_detectors_are_the_global_loads(gtb, cuda, n, W, H, pitch, P, voxel):
     import torch
     L = gtb._lib
     proj = _rand(cuda, (P, H, W), 2)
@@ -55,7 +57,7 @@ def test_padded_detectors_are_the_global_loads(gtb, cuda, n, W, H, pitch, P):
         for accumulate in (False, True):
             outs = []
             for gather in (1, 0):
-                plan = _plan(gtb, n, W, H, pitch, P, 2.5)
+                plan = _plan(gtb, n, W, H, pitch, P, 2.5, voxel)
                 plan.set_option(L.CBCT_OPT_FORCE_GATHER, gather)
                 if accumulate:
                     plan.set_mask(mask)
@@ -76,7 +78,7 @@ def test_steps_of_odd_sizes(gtb, cuda):
     vol = _rand(cuda, (n[2], n[1], n[0]), 6)
     got = []
     for gather in (1, 0):
-        plan = _plan(gtb, n, W, H, 1.3, P)
+        plan = _plan(gtb, n, W, H, 1.3, P, voxel=0.73)
         plan.set_option(L.CBCT_OPT_FORCE_GATHER, gather)
         z, xold, pre = vol.clone(), 0.9 * vol, torch.full_like(vol, 1e-4)
         r, n2 = torch.empty_like(b), torch.zeros(1, dtype=torch.float64, device=cuda)
