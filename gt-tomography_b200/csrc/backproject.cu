@@ -99,7 +99,7 @@ __device__ __forceinline__ void bp_store(const BpEpi& e, size_t idx, float g) {
 // Voxels of a thread's z-run whose epilogue operands are loaded together.  Besides
 // the loads in flight, this sets the registers the compiler gives the kernel: at 8 the
 // view loop keeps its register pairs in place (96 registers for runs of 32; FDK of
-// 256^3 from 360 views of 512x384: 4.67 ms, at 4 with 72 registers 4.90).
+// 256^3 from 360 views of 512x384 when it was chosen: 4.67 ms, at 4 with 72 registers 4.90).
 constexpr int kEpiChunk = 8;
 
 template <int EPI, bool FDK>
