@@ -46,10 +46,11 @@ std::vector<StreamPair>& idle_pairs() {
 // A call's two streams and the events between them; both streams are idle and the events
 // released on every exit path.
 struct Pipe {
-  int device;
+  int device = 0;
   cudaStream_t compute = nullptr, copy = nullptr;
   std::vector<cudaEvent_t> events;
-  explicit Pipe(const cbct_plan* p) : device(p->device) {
+  Pipe() {
+    CBCT_CUDA(cudaGetDevice(&device));
     {
       std::lock_guard<std::mutex> lock(idle_mutex);
       auto& idle = idle_pairs();
@@ -145,7 +146,7 @@ void host_forward(cbct_plan* p, int s0, int ns, const float* vol_host, float* pr
   float* buf[2];
   float* vol;
   stream_buffers(p, largest_batch(p, s0, ns), buf, &vol);
-  Pipe pipe(p);
+  Pipe pipe;
   cudaEvent_t start;
   CBCT_CUDA(cudaEventCreateWithFlags(&start, cudaEventDisableTiming));
   pipe.events.push_back(start);
@@ -180,7 +181,7 @@ void host_backproject(cbct_plan* p, int s0, int ns, const float* proj_host, floa
   float* vol;
   stream_buffers(p, std::max<size_t>(largest_batch(p, s0, ns), plane), buf, &vol);
   if (fbp) fdk_prepare(p, filter);
-  Pipe pipe(p);
+  Pipe pipe;
   cudaEvent_t start;
   CBCT_CUDA(cudaEventCreateWithFlags(&start, cudaEventDisableTiming));
   pipe.events.push_back(start);
